@@ -329,14 +329,22 @@ __global__ void k_oct_nchild(int64_t n_int, const uint32_t* __restrict__ slots, 
 }
 
 __global__ void k_oct_childlist(int64_t n_int, const uint32_t* __restrict__ slots,
-                                const uint32_t* __restrict__ first, uint32_t* __restrict__ ids) {
+                                const uint32_t* __restrict__ first, uint32_t* __restrict__ ids,
+                                uint8_t* __restrict__ ninner) {
   int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (id >= n_int) return;
-  uint32_t w = first[id];
+  const uint32_t f = first[id];
+  uint32_t w = f;
+#pragma unroll
+  for (int s = 0; s < 8; ++s) {  // internal children first (EMPTY_SLOT has the leaf bit)
+    const uint32_t c = slots[id * 8 + s];
+    if (!(c & LEAF_BIT)) ids[w++] = c;
+  }
+  ninner[id] = (uint8_t)(w - f);
 #pragma unroll
   for (int s = 0; s < 8; ++s) {
-    uint32_t c = slots[id * 8 + s];
-    if (c != EMPTY_SLOT) ids[w++] = c;
+    const uint32_t c = slots[id * 8 + s];
+    if ((c & LEAF_BIT) && c != EMPTY_SLOT) ids[w++] = c;
   }
 }
 
@@ -543,7 +551,8 @@ __device__ __forceinline__ WalkNode make_record(uint32_t c, const uint32_t* __re
                                                 const float* __restrict__ massf, const uint8_t* __restrict__ leaf_depth,
                                                 const uint4* __restrict__ walk, const uint8_t* __restrict__ o_depth,
                                                 const uint32_t* __restrict__ nchild,
-                                                const uint32_t* __restrict__ child_first, double h0, double thr) {
+                                                const uint32_t* __restrict__ child_first,
+                                                const uint8_t* __restrict__ ninner) {
   WalkNode r;
   r.pad = 0;
   if (c & LEAF_BIT) {
@@ -562,8 +571,7 @@ __device__ __forceinline__ WalkNode make_record(uint32_t c, const uint32_t* __re
     r.cq[2] = w.z;
     r.mass = __uint_as_float(w.w);
     r.first = 1u + child_first[c];
-    const int dep = o_depth[c];
-    r.info = nchild[c] | ((uint32_t)dep << 4) | (ldexp(h0, -dep) < thr ? WN_TERMINAL : 0u);
+    r.info = nchild[c] | ((uint32_t)o_depth[c] << 4) | ((uint32_t)ninner[c] << 12);
     r.ref = c;
   }
   return r;
@@ -574,21 +582,20 @@ __global__ void k_walk_records(int64_t n_int, const uint32_t* __restrict__ qx, c
                                const uint8_t* __restrict__ leaf_depth, const uint4* __restrict__ walk,
                                const uint8_t* __restrict__ o_depth, const uint32_t* __restrict__ nchild,
                                const uint32_t* __restrict__ child_first, const uint32_t* __restrict__ child_ids,
-                               const TreeParams* __restrict__ prm, double thr, WalkNode* __restrict__ recs) {
+                               const uint8_t* __restrict__ ninner, WalkNode* __restrict__ recs) {
   int64_t P = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (P >= n_int) return;
-  const double h0 = prm->half;
-  if (P == 0)
-    recs[0] = make_record(0u, qx, qy, qz, massf, leaf_depth, walk, o_depth, nchild, child_first, h0, thr);
+  if (P == 0) recs[0] = make_record(0u, qx, qy, qz, massf, leaf_depth, walk, o_depth, nchild, child_first, ninner);
   const uint32_t f = child_first[P], nc = nchild[P];
   for (uint32_t r = 0; r < nc; ++r)
     recs[1 + (int64_t)f + r] =
-        make_record(child_ids[f + r], qx, qy, qz, massf, leaf_depth, walk, o_depth, nchild, child_first, h0, thr);
+        make_record(child_ids[f + r], qx, qy, qz, massf, leaf_depth, walk, o_depth, nchild, child_first, ninner);
 }
 
 // ---------------------------------------------------------------------------
 // walk groups: maximal subtrees of <= group_max particles, consecutive small
-// siblings packed together
+// siblings packed together; cells above pack_depth are always split, and
+// their children never packed, so no group is wider than a cell of that depth
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t child_count(uint32_t c, const uint32_t* __restrict__ o_first,
                                                 const uint32_t* __restrict__ o_last) {
@@ -599,21 +606,24 @@ __device__ __forceinline__ uint32_t child_first_particle(uint32_t c, const uint3
 }
 
 template <bool WRITE>
-__global__ void k_groups(int64_t n_int, int group_max, const uint32_t* __restrict__ slots,
-                         const uint32_t* __restrict__ o_first, const uint32_t* __restrict__ o_last,
+__global__ void k_groups(int64_t n_int, int group_max, int pack_depth, const uint8_t* __restrict__ o_depth,
+                         const uint32_t* __restrict__ slots, const uint32_t* __restrict__ o_first,
+                         const uint32_t* __restrict__ o_last,
                          uint32_t* __restrict__ counts, const uint32_t* __restrict__ base,
                          uint32_t* __restrict__ gfirst, uint32_t* __restrict__ gsize) {
   int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (id >= n_int) return;
   const uint32_t mine = o_last[id] - o_first[id] + 1u;
   uint32_t ng = 0, w = WRITE ? base[id] : 0u;
-  if (mine > (uint32_t)group_max) {
+  const int dep = o_depth[id];
+  if (mine > (uint32_t)group_max || dep < pack_depth) {
+    const uint32_t pack_max = dep < pack_depth ? 0u : (uint32_t)group_max;
     uint32_t run_first = 0, run_n = 0;
     for (int s = 0; s < 8; ++s) {
       const uint32_t c = slots[id * 8 + s];
       if (c == EMPTY_SLOT) continue;
       const uint32_t k = child_count(c, o_first, o_last);
-      if (k > (uint32_t)group_max) {
+      if (k > (uint32_t)group_max || (k > 1u && dep + 1 < pack_depth)) {
         if (run_n) {
           if (WRITE) { gfirst[w] = run_first; gsize[w] = run_n; ++w; }
           ++ng;
@@ -621,7 +631,7 @@ __global__ void k_groups(int64_t n_int, int group_max, const uint32_t* __restric
         }
         continue;
       }
-      if (run_n && run_n + k > (uint32_t)group_max) {
+      if (run_n && run_n + k > pack_max) {
         if (WRITE) { gfirst[w] = run_first; gsize[w] = run_n; ++w; }
         ++ng;
         run_n = 0;
@@ -813,7 +823,8 @@ void launch_octree_links(int64_t n, int64_t n_int, TreeBuffers& t, void* scan_sc
   k_oct_nchild<<<grid_for(n_int, 256, 1ll << 30), 256, 0, s>>>(n_int, t.o_slots, t.o_nchild);
   TPM_LAUNCH_CHECK();
   exclusive_scan_u32(t.o_nchild, t.o_child_first, n_int, &t.scalars[3], scan_scratch, s);
-  k_oct_childlist<<<grid_for(n_int, 256, 1ll << 30), 256, 0, s>>>(n_int, t.o_slots, t.o_child_first, t.child_ids);
+  k_oct_childlist<<<grid_for(n_int, 256, 1ll << 30), 256, 0, s>>>(n_int, t.o_slots, t.o_child_first, t.child_ids,
+                                                                  t.o_ninner);
   TPM_LAUNCH_CHECK();
 }
 
@@ -863,22 +874,25 @@ void launch_cell_q(int64_t n_int, double box, TreeBuffers& t, cudaStream_t s) {
   TPM_LAUNCH_CHECK();
 }
 
-void launch_walk_records(const Particles& p, int64_t n, int64_t n_int, double thr, TreeBuffers& t, cudaStream_t s) {
+void launch_walk_records(const Particles& p, int64_t n, int64_t n_int, TreeBuffers& t, cudaStream_t s) {
   (void)n;
   k_walk_records<<<grid_for(n_int, 128, 1ll << 30), 128, 0, s>>>(n_int, p.qx, p.qy, p.qz, p.massf, t.leaf_depth,
                                                                  t.o_walk, t.o_depth, t.o_nchild, t.o_child_first,
-                                                                 t.child_ids, t.params, thr, t.recs);
+                                                                 t.child_ids, t.o_ninner, t.recs);
   TPM_LAUNCH_CHECK();
 }
 
-void launch_groups(int64_t n, int64_t n_int, int group_max, TreeBuffers& t, void* scan_scratch, cudaStream_t s) {
+void launch_groups(int64_t n, int64_t n_int, int group_max, int pack_depth, TreeBuffers& t, void* scan_scratch,
+                   cudaStream_t s) {
   (void)n;
-  k_groups<false><<<grid_for(n_int, 256, 1ll << 30), 256, 0, s>>>(n_int, group_max, t.o_slots, t.o_first, t.o_last,
-                                                                  t.grp_count_per_node, nullptr, nullptr, nullptr);
+  k_groups<false><<<grid_for(n_int, 256, 1ll << 30), 256, 0, s>>>(
+      n_int, group_max, pack_depth, t.o_depth, t.o_slots, t.o_first, t.o_last, t.grp_count_per_node, nullptr, nullptr,
+      nullptr);
   TPM_LAUNCH_CHECK();
   exclusive_scan_u32(t.grp_count_per_node, t.grp_base, n_int, &t.scalars[1], scan_scratch, s);
-  k_groups<true><<<grid_for(n_int, 256, 1ll << 30), 256, 0, s>>>(n_int, group_max, t.o_slots, t.o_first, t.o_last,
-                                                                 nullptr, t.grp_base, t.grp_first, t.grp_size);
+  k_groups<true><<<grid_for(n_int, 256, 1ll << 30), 256, 0, s>>>(
+      n_int, group_max, pack_depth, t.o_depth, t.o_slots, t.o_first, t.o_last, nullptr, t.grp_base, t.grp_first,
+      t.grp_size);
   TPM_LAUNCH_CHECK();
 }
 

@@ -13,18 +13,18 @@ constexpr int KEY_LEVELS = 42;  // 21 octant digits in each of two 64-bit words
 // One node of the walk, 32 bytes.  Records are laid out so that the children
 // of every internal node are contiguous (root at 0, the children of internal
 // node P at 1 + child_first[P] ...), so the walk reads a node's children with
-// one coalesced load.
+// one coalesced load; internal children come before leaves.
 struct __align__(16) WalkNode {
   uint32_t cq[3];    // fixed-point centre of mass (leaf: the particle)
   float mass;
   uint32_t first;    // record index of the first child (internal nodes)
-  uint32_t info;     // nchild [0,4) | depth [4,10) | leaf bit 10 | terminal bit 11
+  uint32_t info;     // nchild [0,4) | depth [4,10) | leaf bit 10 | internal children [12,16)
   uint32_t ref;      // leaf: sorted particle index; internal: octree node id
   uint32_t pad;
 };
 constexpr uint32_t WN_LEAF = 1u << 10;
-constexpr uint32_t WN_TERMINAL = 1u << 11;
 __host__ __device__ inline uint32_t wn_nchild(uint32_t info) { return info & 15u; }
+__host__ __device__ inline uint32_t wn_ninner(uint32_t info) { return (info >> 12) & 15u; }
 __host__ __device__ inline int wn_depth(uint32_t info) { return (int)((info >> 4) & 63u); }
 
 // Geometry of one force evaluation, computed on the device.
@@ -75,7 +75,8 @@ struct TreeBuffers {
   uint32_t* o_nchild;
   uint32_t* o_child_first;
   uint32_t* o_cnt;      // internal node ids bucketed by depth (aggregation order)
-  uint32_t* child_ids;  // compacted, same encoding as o_slots
+  uint8_t* o_ninner;    // internal children
+  uint32_t* child_ids;  // compacted (internal children, then leaves), same encoding as o_slots
   double* o_mass;
   double* o_com;   // 3 per node
   double* o_quad;  // 6 per node
@@ -112,13 +113,16 @@ void launch_octree_links(int64_t n, int64_t n_int, TreeBuffers& t, void* scan_sc
 // with_quad the quadrupole tensors too.
 void launch_aggregate(const Particles& p, int64_t n, int64_t n_int, double box, TreeBuffers& t, cudaStream_t s,
                       bool with_quad = false);
-void launch_walk_records(const Particles& p, int64_t n, int64_t n_int, double thr, TreeBuffers& t, cudaStream_t s);
+void launch_walk_records(const Particles& p, int64_t n, int64_t n_int, TreeBuffers& t, cudaStream_t s);
 // Per internal node: the centre of its octree cell (child_center replayed
 // along the node's octant path, octree.rs:446-465) in fixed point and the
 // Frobenius norm of its six stored quadrupole components (the relative
 // opening criterion's estimate, octree.rs:769-796).  Needs the quadrupoles.
 void launch_cell_q(int64_t n_int, double box, TreeBuffers& t, cudaStream_t s);
-void launch_groups(int64_t n, int64_t n_int, int group_max, TreeBuffers& t, void* scan_scratch, cudaStream_t s);
+// Walk groups of at most group_max particles, each inside one octree cell of
+// depth pack_depth or more.
+void launch_groups(int64_t n, int64_t n_int, int group_max, int pack_depth, TreeBuffers& t, void* scan_scratch,
+                   cudaStream_t s);
 void launch_hilbert_keys(const Particles& p, int64_t n, double box, const TreeParams* prm, uint64_t* keys,
                          uint32_t* vals, cudaStream_t s);
 // Morton keys (particle_morton, sfc.rs:54-81) with the normalisation of prm's

@@ -234,6 +234,7 @@ struct tpm_handle {
   void* scan_scratch = nullptr;
   uint32_t* stack = nullptr;
   int walk_grid = 0;
+  bool poly = false;  // the walk's erfc polynomial covers r_cut
   uint2* deferred = nullptr;
   uint32_t* ndeferred = nullptr;
   unsigned long long* stats_dev = nullptr;
@@ -449,6 +450,7 @@ void ensure_tree_capacity(tpm_handle* h, int64_t n_int) {
   T.o_nchild = h->alloc<uint32_t>(c, 2);
   T.o_child_first = h->alloc<uint32_t>(c, 2);
   T.o_cnt = h->alloc<uint32_t>(c, 2);
+  T.o_ninner = h->alloc<uint8_t>(c, 2);
   T.child_ids = h->alloc<uint32_t>(c + h->cap + 8, 2);
   T.o_mass = h->alloc<double>(c, 2);
   T.o_com = h->alloc<double>(3 * c, 2);
@@ -462,6 +464,28 @@ void ensure_tree_capacity(tpm_handle* h, int64_t n_int) {
   T.grp_size = h->alloc<uint32_t>(h->cap + 1, 2);
   T.cap_int = c;
   T.cap_groups = h->cap + 1;
+}
+
+// The widest walk group.  Sources are taken relative to the group's first
+// target, so their minimum image must serve the whole group out to r_cut (and a
+// monopole's half side, below 0.1 r_cut): an extent of L/2 - 1.12 r_cut at
+// most.  2.8 r_cut bounds the rounding of the relative positions (the pair
+// loop's band grows with extent / r_cut; 2.8 is L/16 on a 256^3 mesh at r_cut =
+// 5.6 cells), but L/16 is always wide enough to hold a group of a large box.
+// The accurate walk opens every node whose images may matter, which depends on
+// the extent: it keeps L/16, and walks targets alone when r_cut > L/5.
+double max_extent(const tpm_handle* h) {
+  const double box = h->cfg.box_size, rc = h->r_cut;
+  if (h->cfg.flags & TPM_FLAG_ACCURATE) return rc > 0.2 * box ? 0.0 : box / 16.0;
+  const double fits = 0.5 * box - 1.12 * rc;
+  return std::max(0.0, std::min(fits, std::max(box / 16.0, std::min(0.25 * box, 2.8 * rc))));
+}
+
+// A float in both halves of a packed pair.
+unsigned long long twice(float v) {
+  uint32_t b;
+  std::memcpy(&b, &v, 4);
+  return (unsigned long long)b << 32 | b;
 }
 
 float ms_between(cudaEvent_t a, cudaEvent_t b) {
@@ -590,8 +614,11 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
       launch_aggregate(h->P[h->cur], n, h->n_int, box, T, s, rel);
       h->quad_valid = rel;
       if (rel) launch_cell_q(h->n_int, box, T, s);
-      launch_walk_records(h->P[h->cur], n, h->n_int, h->thr, T, s);
-      launch_groups(n, h->n_int, walk_targets_per_warp(), T, h->scan_scratch, s);
+      launch_walk_records(h->P[h->cur], n, h->n_int, T, s);
+      int pack_depth = 0;  // the first depth whose cells are no wider than a walk group may be
+      const double extent = max_extent(h);
+      while (pack_depth < DEPTH_BINS && !(std::ldexp(2.0 * h->params_host.half, -pack_depth) <= extent)) ++pack_depth;
+      launch_groups(n, h->n_int, walk_group_size(n), pack_depth, T, h->scan_scratch, s);
       TPM_CUDA(cudaMemcpyAsync(sc, T.scalars, sizeof(sc), cudaMemcpyDeviceToHost, s));
       TPM_CUDA(cudaStreamSynchronize(s));
       h->n_groups = sc[1];
@@ -652,29 +679,36 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
       const double rc2_u = h->rc2 / (u * u);
       a.rc2_lo = (float)(rc2_u * (1.0 - 1e-4));
       a.rc2_hi = (float)(rc2_u * (1.0 + 1e-4));
+      a.rc2_mid = 0.5f * (a.rc2_lo + a.rc2_hi);
+      a.rc2_band = 0.5f * (a.rc2_hi - a.rc2_lo) * 1.01f + 1e-6f * a.rc2_hi;
       // The pair loop's band: near r_cut its FP32 distance carries a relative
-      // error below 2.4e-7 (1 + E / r_cut) + 2e-7, E = the widest group the
-      // walk accepts (1/16 of the box; coordinates are group-relative floats),
+      // error below 2.4e-7 (1 + E / r_cut) + 2e-7, E = the widest group
+      // (coordinates are group-relative floats),
       // since periodic leaves have no half side and monopoles h < 0.1 r_cut;
       // 8 times that (at least 1e-5) leaves every pair the FP32 path could
       // misjudge to the float64 test.  The aperiodic walk's leaves carry their
       // cell's half side (cancellation against it): the node band of 1e-4.
       {
-        const double e_over_rc = (box / 16.0) / h->r_cut;
+        const double e_over_rc = std::max(max_extent(h), box / 16.0) / h->r_cut;
         const double pband = h->periodic ? std::max(1e-5, 8.0 * (2.4e-7 * (1.0 + e_over_rc) + 2e-7)) : 1e-4;
         a.prc2_lo = (float)(rc2_u * (1.0 - pband));
         a.prc2_hi = (float)(rc2_u * (1.0 + pband));
-        uint32_t lo_bits, hi_bits;
-        std::memcpy(&lo_bits, &a.prc2_lo, 4);
-        std::memcpy(&hi_bits, &a.prc2_hi, 4);
-        a.prc2_lo_bits = lo_bits;
-        a.pband_bits = hi_bits - lo_bits;
+        // the pair loop flags |s - mid| <= pband, a little more than (lo, hi]
+        a.prc2_mid = 0.5f * (a.prc2_lo + a.prc2_hi);
+        a.pband = 0.5f * (a.prc2_hi - a.prc2_lo) * 1.01f + 1e-6f * a.prc2_hi;
       }
       a.grc2_lo = (float)(rc2_u * (1.0 - 4e-4));
       a.grc2_hi = (float)(rc2_u * (1.0 + 4e-4));
       a.eps2_u = (float)(eps2 / (u * u));
+      a.eps2_2 = twice(std::max(a.eps2_u, 1e-30f));
       const double cx = u / (std::sqrt(2.0) * h->r_s);
       a.pcx = (float)(0.3275911 * cx);
+      a.poly = h->poly ? 1 : 0;
+      if (h->poly) {
+        float c[POLY_DEGREE + 1];
+        erfc_poly(h->r_cut / (std::sqrt(2.0) * h->r_s), cx, c);
+        for (int k = 0; k <= POLY_DEGREE; ++k) a.poly2[k] = twice(c[k]);
+      }
       a.ex2k = (float)(-(cx * cx) / std::log(2.0));
       const double tq = std::ldexp(4.0, -U);
       a.tiny_u = (float)(tq * tq);
@@ -697,27 +731,35 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
       a.rel_k = (float)(h->cfg.err_tol_force_acc * u * u * u);
       if (a.accurate) {  // no reference decisions to reproduce: no float64 band, no COM-on-target opening
         a.rc2_lo = a.rc2_hi = (float)rc2_u;
-        a.prc2_lo = a.prc2_hi = a.rc2_lo;
-        std::memcpy(&a.prc2_lo_bits, &a.prc2_lo, 4);
-        a.pband_bits = 0u;
+        a.prc2_lo = a.prc2_hi = a.prc2_mid = a.rc2_lo;
         a.tiny_u = -1.f;
       }
       a.ax = h->srx; a.ay = h->sry; a.az = h->srz;
       a.stats = h->stats_dev; a.err = T.err;
       a.deferred = h->deferred; a.ndeferred = h->ndeferred; a.cap_deferred = DEFERRED_CAP;
       a.stack = h->stack; a.stack_cap = STACK_CAP;
-      a.single_target = h->r_cut > 0.2 * box ? 1 : 0;
       a.pcounts = h->pcounts;
       a.only = use_net ? h->fallback : only;
       {
-        // a group spans at most L/16 (wider ones are walked target by target),
-        // so for a node of cull half side hc the +-L images lie at least
-        // 7L/16 - hc away: beyond r_cut once hc < 7L/16 - r_cut (hc <= 2 h)
+        // for a node of cull half side hc (h, or 2 h in accurate mode) the +-L
+        // images lie at least L/2 - extent - hc away: beyond r_cut once hc is
+        // below L/2 - extent - r_cut
         const double box_u = std::ldexp(1.0, 32 - U), rc_u = std::sqrt(rc2_u) * 1.001;
+        const double reach = a.accurate ? 7.0 / 16.0 * box_u : 0.5 * box_u - 1.001 * max_extent(h) / u;
+        const double wide = a.accurate ? 2.0 : 1.0;
         int dimg = 0;
-        while (dimg < 64 && !(7.0 / 16.0 * box_u - 2.0 * std::ldexp(a.h0_u, -dimg) > rc_u)) ++dimg;
+        while (dimg < 64 && !(reach - wide * std::ldexp(a.h0_u, -dimg) > rc_u)) ++dimg;
         a.img_depth = dimg;
       }
+      // the depth at which internal nodes become monopoles
+      double thr_depth = h0;
+      int dstar = 0;
+      while (!(thr_depth < h->thr) && dstar < 200) {
+        thr_depth = std::ldexp(h0, -(++dstar));
+      }
+      h->stats.terminal_depth = dstar;
+      a.h_term = std::ldexp(a.h0_u, -dstar);
+      a.term_depth = dstar;
       TPM_CUDA(cudaMemsetAsync(h->work, 0, sizeof(uint32_t), s));
       TPM_CUDA(cudaMemsetAsync(h->ndeferred, 0, sizeof(uint32_t), s));
       launch_walk(a, h->walk_grid, s);
@@ -725,12 +767,6 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
       TPM_CUDA(cudaMemcpyAsync(&nd, h->ndeferred, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
       TPM_CUDA(cudaStreamSynchronize(s));
       if (nd) launch_deferred(a, std::min(nd, DEFERRED_CAP), s);
-      double thr_depth = h0;
-      int dstar = 0;
-      while (!(thr_depth < h->thr) && dstar < 200) {
-        thr_depth = std::ldexp(h0, -(++dstar));
-      }
-      h->stats.terminal_depth = dstar;
     } else {
       TPM_CUDA(cudaMemsetAsync(h->srx, 0, sizeof(float) * n, s));
       TPM_CUDA(cudaMemsetAsync(h->sry, 0, sizeof(float) * n, s));
@@ -1001,7 +1037,11 @@ int tpm_create(const tpm_config* cfg, tpm_handle** out) {
     h->ndeferred = h->alloc<uint32_t>(1, 0);
     h->deferred = h->alloc<uint2>(DEFERRED_CAP, 0);
     int sms = prop.multiProcessorCount;
-    h->walk_grid = sms * walk_blocks_per_sm((cfg->flags & TPM_FLAG_ACCURATE) != 0);
+    {
+      float unused[POLY_DEGREE + 1];
+      h->poly = erfc_poly(h->r_cut / (std::sqrt(2.0) * h->r_s), 1.0, unused);
+    }
+    h->walk_grid = sms * walk_blocks_per_sm(h->periodic, (cfg->flags & TPM_FLAG_ACCURATE) != 0, h->poly);
     h->stack = h->alloc<uint32_t>(walk_stack_words(h->walk_grid, STACK_CAP), 0);
     TPM_CUDA(cudaMemset(h->T.err, 0, sizeof(uint32_t)));
     pm_plan_init(h->pm, nm, cfg->box_size, h->pm_only ? 0.0 : h->r_s, cfg->flags, cfg->device);

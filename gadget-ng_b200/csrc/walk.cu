@@ -11,26 +11,31 @@
 // target interacts with a node depends on every ancestor on its path.
 //
 // Warp design: the 32 lanes hold up to 32 target particles from one compact
-// subtree.  The warp walks the tree once for all of them: each stack entry
-// carries a 32-bit mask of the targets that still see that node.  Nodes are
-// classified against the group's bounding box in FP32 with a safety margin
+// subtree.  The warp walks the tree once for all of them: each range of nodes
+// on its stack carries a 32-bit mask of the targets that still see it.  Nodes
+// are classified against the group's bounding box in FP32 with a safety margin
 // (certainly culled / certainly kept for every target / undecided); undecided
-// internal nodes get a per-target test when they are popped, which refines the
-// mask, so the hierarchical culls of the reference are reproduced exactly.
-// Terminal nodes (leaves and monopole-depth cells) go to an interaction list
-// in shared memory; the lanes evaluate the list against the group's targets
-// with each target's own final test fused into the pair kernel (a group of c
+// internal nodes get a per-target test before they are pushed, which refines
+// the mask, so the hierarchical culls of the reference are reproduced exactly.
+// Terminal nodes (leaves and monopole-depth cells) go to interaction lists in
+// shared memory; the lanes evaluate a list against the group's targets with
+// each target's own final test fused into the pair kernel (a group of c
 // targets gives every target 32 / c lanes, each on a share of the entries).
 // The running per-target sums, the targets' positions and the group box stay
-// in shared memory (read where a flush, a refinement or a classification
-// needs them), so the traversal keeps its registers: 7 resident blocks per SM
-// at 72 registers.  Any decision
-// that falls inside a narrow band around r_cut is re-evaluated in float64
-// with the reference's exact expression, so the interaction set equals the
-// reference's.  Pair arithmetic is FP32: exact fixed-point differences split
-// into two floats, rsqrt / rcp / ex2 hardware approximations, the A&S 7.1.26
-// erfc, and Kahan-compensated per-target accumulators.
-#include <cstdlib>
+// in shared memory.  Any decision that falls inside a narrow band around r_cut
+// is re-evaluated in float64 with the reference's exact expression, so the
+// interaction set equals the reference's.  Pair arithmetic is FP32: exact
+// fixed-point differences rounded once, rsqrt / ex2 hardware approximations,
+// a polynomial for the A&S 7.1.26 erfc, Kahan-compensated per-target sums.
+//
+// What bounds it (lattice of 128^3, 84 k groups, B200 at 1965 MHz): issue slots.
+// 11.28e9 warp instructions took 11.3 ms at 88 % issue before the pair loop
+// took two entries per iteration in f32x2 arithmetic (63 instructions for
+// two entries, ~106 before) and the traversal was split into open and item
+// steps; 5.93e9 take 7.1 ms at 73 % after (62.7 -> 40.3 ms on the clustered
+// 256^3 box).  About half are the pair loop, its FMA pipe 56 % busy.
+#include <cmath>
+#include <type_traits>
 
 #include "common.cuh"
 #include "tree.cuh"
@@ -44,20 +49,86 @@ constexpr int WALK_THREADS = WALK_WARPS * 32;
 constexpr int CHUNK_L = 64;  // leaf-list capacity (walk 72.9 -> 72.5 ms at 256^3 against 48; 32 is slower)
 // monopole-list capacity: the accurate mode also emits monopoles at pop time
 template <bool ACC> constexpr int chunk_m() { return ACC ? 96 : 64; }
-constexpr int32_t WIDE_GROUP = 1 << 28;  // quanta: 1/16 of the box
 
 
-// One interaction-list entry (32 bytes): the source position relative to
-// the group's first target in walk units (one rounding of the exact int32
-// difference; the group is compact, so the rounding stays far below the
-// softening length and the float64 band settles every borderline cut), mass,
-// cull half side (0 for periodic leaves), the mask of targets that see it and
-// the node (LEAF_BIT | particle for leaves).
-struct __align__(16) Entry {
-  float x, y, z, m;
-  float h;
-  uint32_t mask, node, pad;
+// An interaction list in shared memory, kept in pairs of entries so that the
+// pair loop reads both entries of a packed (f32x2) operand with one load:
+// source positions relative to the group's origin in walk units (one
+// rounding of the exact int32 difference; the group is compact, so the
+// rounding stays far below the softening length and the float64 band settles
+// every borderline cut), masses, the masks of targets that see them, the nodes
+// (LEAF_BIT | particle for leaves) and, where a list needs them, cull half
+// sides.
+template <bool HALF> struct __align__(16) EntryPair {
+  float4 xy;   // x0 x1 y0 y1
+  float4 zm;   // z0 z1 m0 m1
+  uint2 mask;
+  uint2 node;
 };
+template <> struct __align__(16) EntryPair<true> {
+  float4 xy;
+  float4 zm;
+  uint2 mask;
+  uint2 node;
+  float2 h;
+};
+template <int CAP, bool HALF> struct List {
+  static_assert(CAP % 2 == 0, "entries are evaluated two at a time");
+  EntryPair<HALF> pair[CAP / 2];
+  // word w of entry e: members of a pair interleave its two entries
+  __device__ __forceinline__ float* word(int e) { return reinterpret_cast<float*>(&pair[e >> 1]) + (e & 1); }
+  __device__ __forceinline__ const float* word(int e) const {
+    return reinterpret_cast<const float*>(&pair[e >> 1]) + (e & 1);
+  }
+  __device__ __forceinline__ void put(int e, float x, float y, float z, float m, float half, uint32_t see, uint32_t nd) {
+    float* w = word(e);
+    w[0] = x;
+    w[2] = y;
+    w[4] = z;
+    w[6] = m;
+    w[8] = __uint_as_float(see);
+    w[10] = __uint_as_float(nd);
+    if (HALF) w[12] = half;
+  }
+  // nobody sees the second half of an odd list's last pair
+  __device__ __forceinline__ void close(int n) {
+    if (n & 1) word(n)[8] = 0.f;
+  }
+};
+
+// Packed pairs of floats (PTX f32x2, one instruction for both halves).
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// min(|a|, |b|, |c|) in one instruction
+__device__ __forceinline__ float min3_abs(float a, float b, float c) {
+  float r;
+  asm("min.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 
 __device__ __forceinline__ int32_t rel32(uint32_t a, uint32_t b, int periodic) {
   if (periodic) return (int32_t)(a - b);  // minimum image modulo 2^32
@@ -164,19 +235,46 @@ __device__ __forceinline__ void defer(const WalkArgs& a, uint32_t p, uint32_t no
   else atomicOr(a.err, DEV_ERR_DEFERRED);
 }
 
-// FP32 pair term: returns m * erfc(x) / r^3 (walk units), x = r/(sqrt2 r_s);
-// ACC (accurate mode) adds the Gaussian term (2x/sqrt(pi)) exp(-x^2).
-template <bool ACC = false>
+// FP32 pair term: m * erfc(x) / r^3 (walk units), x = r/(sqrt2 r_s), for two
+// entries at once.  K_POLY: erfc as 2^P(r), the fitted polynomial of WalkArgs;
+// K_AS: the A&S 7.1.26 form itself; K_ACC: the A&S form plus the Gaussian term
+// (2x/sqrt(pi)) exp(-x^2) of the accurate mode.
+enum { K_POLY = 0, K_AS = 1, K_ACC = 2 };
+template <int KERNEL>
+__device__ __forceinline__ f32x2 pair_factor2(const WalkArgs& a, f32x2 r2b, f32x2 m) {
+  const f32x2 r2 = add2(r2b, a.eps2_2);
+  const float2 q = unpack2(r2);
+  const f32x2 ri = pack2(rsqrt_approx(q.x), rsqrt_approx(q.y));
+  const f32x2 r = mul2(r2, ri);
+  const f32x2 ri3 = mul2(mul2(ri, ri), ri);
+  f32x2 w;
+  if (KERNEL == K_POLY) {
+    // The coefficients stay in the constant bank: held in registers (over a
+    // list) they slow the walk from 40.3 to 45.0 ms at 256^3, three 64-bit
+    // register operands being more than a packed FMA reads per cycle.
+    f32x2 p = a.poly2[POLY_DEGREE];
+#pragma unroll
+    for (int k = POLY_DEGREE - 1; k >= 0; --k) p = fma2(p, r, a.poly2[k]);
+    const float2 e = unpack2(p);
+    w = pack2(ex2_approx(e.x), ex2_approx(e.y));
+  } else {
+    const float2 d = unpack2(fma2(pack2(a.pcx, a.pcx), r, pack2(1.f, 1.f)));
+    const f32x2 t = pack2(rcp_approx(d.x), rcp_approx(d.y));
+    f32x2 p = pack2(ErfcConst::A5, ErfcConst::A5);
+    p = fma2(p, t, pack2(ErfcConst::A4, ErfcConst::A4));
+    p = fma2(p, t, pack2(ErfcConst::A3, ErfcConst::A3));
+    p = fma2(p, t, pack2(ErfcConst::A2, ErfcConst::A2));
+    p = fma2(p, t, pack2(ErfcConst::A1, ErfcConst::A1));
+    p = mul2(p, t);
+    if (KERNEL == K_ACC) p = fma2(pack2(a.gkc, a.gkc), r, p);
+    const float2 e = unpack2(mul2(r2, pack2(a.ex2k, a.ex2k)));
+    w = mul2(p, pack2(ex2_approx(e.x), ex2_approx(e.y)));
+  }
+  return mul2(mul2(m, w), ri3);
+}
+template <int KERNEL>
 __device__ __forceinline__ float pair_factor(const WalkArgs& a, float r2b, float m) {
-  float r2 = fmaxf(r2b + a.eps2_u, 1e-30f);
-  float ri = rsqrt_approx(r2);
-  float r = r2 * ri;
-  float tt = rcp_approx(fmaf(a.pcx, r, 1.0f));
-  float poly = tt * fmaf(tt, fmaf(tt, fmaf(tt, fmaf(tt, ErfcConst::A5, ErfcConst::A4), ErfcConst::A3), ErfcConst::A2),
-                         ErfcConst::A1);
-  if (ACC) poly = fmaf(a.gkc, r, poly);
-  const float w = poly * ex2_approx(r2 * a.ex2k);
-  return m * w * (ri * ri * ri);
+  return unpack2(pair_factor2<KERNEL>(a, pack2(r2b, r2b), pack2(m, m))).x;
 }
 
 struct Acc {
@@ -191,133 +289,179 @@ struct Acc {
 
 // Lanes of the pair phase.  A group of c targets leaves 32 - c lanes without
 // a target of their own, so R = 32 / c lanes share each target: lane l
-// evaluates target l % c against entries l / c, l / c + R, ... of each list
-// (lanes from R c on evaluate nothing), and the R partial sums of a target
+// evaluates target l % c against the entry pairs l / c, l / c + R, ... of each
+// list (lanes from R c on evaluate nothing), and the R partial sums of a target
 // are folded when its walk ends.  Packed in one register: target | first
-// entry << 8 | R << 16.
+// pair << 8 | R << 16.
 __device__ __forceinline__ uint32_t pair_lanes(int lane, uint32_t c) {
   const uint32_t r = 32u / c, t = (uint32_t)lane % c, off = (uint32_t)lane / c;
   return t | ((off < r ? off : 255u) << 8) | (r << 16);
 }
 
-// Evaluate one interaction list against this lane's pair-phase target.  MONO
-// selects the monopole list (AABB-gap test) or the leaf list (bare-distance
-// test; the aperiodic walk's leaves carry their half side and take the AABB
-// test too).  Borderline pairs are left out here and flagged; resolve_list
-// settles them.
-template <bool MONO, bool ACC>
-__device__ __forceinline__ void flush_list(const WalkArgs& a, const Entry* L, int nl, uint32_t lanes, float tx,
-                                           float ty, float tz, float& fx, float& fy, float& fz, uint32_t& nok,
-                                           bool& amb_any) {
-  const int t = lanes & 0xffu, stride = lanes >> 16;
+// How a list's entries are cut at r_cut: on their bare distance (leaves of the
+// periodic walk), or on the gap to their box of one half side for the whole
+// list (monopoles of the parity walk: all at the terminal depth) or of their
+// own half sides (accurate monopoles, leaves of the aperiodic walk).
+enum { CUT_BARE = 0, CUT_ONE_HALF = 1, CUT_OWN_HALF = 2 };
+
+struct Sums {
+  float x, y, z;
+  uint32_t n;  // entries taken
+};
+
+template <int CUT>
+__device__ __forceinline__ float cut_s(float dx, float dy, float dz, float r2b, float h) {
+  if (CUT == CUT_BARE) return r2b;
+  const float ex = fmaxf(fabsf(dx) - h, 0.f), ey = fmaxf(fabsf(dy) - h, 0.f), ez = fmaxf(fabsf(dz) - h, 0.f);
+  return fmaf(ex, ex, fmaf(ey, ey, ez * ez));
+}
+
+// One lane's share of a list, two entries per iteration in packed arithmetic
+// (issue slots bound the walk, and the f32x2 instructions halve those of the
+// distance, the polynomial and the sums).  Returns true when the lane met a
+// pair that FP32 cannot decide: one inside the band around r_cut^2 or (NEAR) a
+// centre of mass within a few quanta of the target.  Its result is then void,
+// and redo_lane evaluates the lane's share again.  So the loop itself keeps only the
+// sign of s - r_cut^2 and two running minima per pair of entries.
+template <int CUT, bool BAND, bool NEAR, int KERNEL, class L>
+__device__ __forceinline__ bool eval_list(const WalkArgs& a, const L& list, int n, uint32_t lanes, float tx, float ty, float tz, Sums& out) {
+  const uint32_t tbit = 1u << (lanes & 0xffu);
+  const uint32_t stride = lanes >> 16;
+  auto* e = &list.pair[(lanes >> 8) & 0xffu];
+  const auto* end = &list.pair[(n + 1) >> 1];
+  const f32x2 ntx = pack2(-tx, -tx), nty = pack2(-ty, -ty), ntz = pack2(-tz, -tz);
+  const f32x2 nmid = pack2(-a.prc2_mid, -a.prc2_mid);
+  f32x2 fx = 0ull, fy = 0ull, fz = 0ull;
+  uint32_t cnt = 0;
+  float edge = 1e30f, close = 1e30f;
 #pragma unroll 1
-  for (int e = (lanes >> 8) & 0xffu; e < nl; e += stride) {
-    const float4 A = *reinterpret_cast<const float4*>(&L[e].x);
-    const uint4 B = *reinterpret_cast<const uint4*>(&L[e].h);
-    const float h = __uint_as_float(B.x);
-    const uint32_t mask = B.y;
-    const float dx = A.x - tx, dy = A.y - ty, dz = A.z - tz;
-    const float r2b = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-    float s = r2b;
-    if (MONO || !a.periodic) {
-      const float ex = fmaxf(fabsf(dx) - h, 0.f), ey = fmaxf(fabsf(dy) - h, 0.f);
-      const float ez = fmaxf(fabsf(dz) - h, 0.f);
-      s = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
+  for (; e < end; e += stride) {
+    const float4 A = e->xy, B = e->zm;
+    const uint2 M = e->mask;
+    const f32x2 dx = add2(pack2(A.x, A.y), ntx), dy = add2(pack2(A.z, A.w), nty), dz = add2(pack2(B.x, B.y), ntz);
+    const f32x2 r2b = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+    f32x2 s = r2b;
+    if (CUT != CUT_BARE) {
+      float2 h = make_float2(a.h_term, a.h_term);
+      if constexpr (CUT == CUT_OWN_HALF) h = e->h;
+      const float2 x = unpack2(dx), y = unpack2(dy), z = unpack2(dz);
+      const f32x2 ex = pack2(fmaxf(fabsf(x.x) - h.x, 0.f), fmaxf(fabsf(x.y) - h.y, 0.f));
+      const f32x2 ey = pack2(fmaxf(fabsf(y.x) - h.x, 0.f), fmaxf(fabsf(y.y) - h.y, 0.f));
+      const f32x2 ez = pack2(fmaxf(fabsf(z.x) - h.x, 0.f), fmaxf(fabsf(z.y) - h.y, 0.f));
+      s = fma2(ex, ex, fma2(ey, ey, mul2(ez, ez)));
     }
-    const bool in = (mask >> t) & 1u;
-    bool ok = in && s <= a.prc2_lo;
-    if (!ACC) {  // accurate mode reproduces no float64 decisions
-      // s in (prc2_lo, prc2_hi]: positive floats order like their bit patterns
-      bool amb = in && (__float_as_uint(s) - a.prc2_lo_bits - 1u) < a.pband_bits;
-      if (MONO) {
-        // a centre of mass within a few quanta of the target: resolve_list
-        // alone decides it (take it, or open it when it is the target's own
-        // position), so it must not enter the sum here as well
-        const bool near = in && r2b < a.tiny_u;
-        amb = amb || near;
-        ok = ok && !near;
+    const float2 q = unpack2(add2(s, nmid));
+    if (BAND) edge = min3_abs(edge, q.x, q.y);
+    if (NEAR) {
+      const float2 c = unpack2(r2b);
+      close = min3_abs(close, c.x, c.y);
+    }
+    const bool ok0 = (M.x & tbit) && q.x <= 0.f, ok1 = (M.y & tbit) && q.y <= 0.f;
+    const float2 f = unpack2(pair_factor2<KERNEL>(a, r2b, pack2(B.z, B.w)));
+    const f32x2 g = pack2(ok0 ? f.x : 0.f, ok1 ? f.y : 0.f);
+    fx = fma2(dx, g, fx);
+    fy = fma2(dy, g, fy);
+    fz = fma2(dz, g, fz);
+    cnt += ok0 ? 1u : 0u;  // the target's own leaf is masked out at emission
+    cnt += ok1 ? 1u : 0u;
+  }
+  const float2 X = unpack2(fx), Y = unpack2(fy), Z = unpack2(fz);
+  out.x = X.x + X.y;
+  out.y = Y.x + Y.y;
+  out.z = Z.x + Z.y;
+  out.n = cnt;
+  return (BAND && edge <= a.pband) || (NEAR && close < a.tiny_u);
+}
+
+// The share of lane `src` again (rare), all 32 lanes taking entry pairs of it,
+// with the reference's float64 decisions for the undecided entries.  Every
+// lane returns the sums.
+template <int CUT, bool NEAR, int KERNEL, class L>
+__device__ __noinline__ Sums redo_lane(const WalkArgs& a, const L& list, int n, uint32_t lanes, uint32_t p, float tx,
+                                       float ty, float tz, uint32_t* nexact) {
+  const int t = lanes & 0xffu, stride = lanes >> 16, lane = threadIdx.x & 31;
+  Sums o = {0.f, 0.f, 0.f, 0u};
+  for (int e = 2 * (int)(((lanes >> 8) & 0xffu) + (uint32_t)(lane * stride)); e < n; e += 64 * stride) {
+    for (int k = e; k < e + 2 && k < n; ++k) {
+      const float* w = list.word(k);
+      const uint32_t node = __float_as_uint(w[10]);
+      if (!((__float_as_uint(w[8]) >> t) & 1u)) continue;
+      const float dx = w[0] - tx, dy = w[2] - ty, dz = w[4] - tz;
+      const float r2b = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+      const float s = cut_s<CUT>(dx, dy, dz, r2b, CUT == CUT_OWN_HALF ? w[12] : a.h_term);
+      bool take = s <= a.prc2_lo;
+      if ((s > a.prc2_lo && s <= a.prc2_hi) || (NEAR && r2b < a.tiny_u)) {
+        ++*nexact;
+        const int d = exact_terminal(a, p, node);
+        if (d == 2) defer(a, p, node);
+        take = d == 1;
       }
-      amb_any = amb_any || amb;
+      if (!take) continue;
+      const float f = pair_factor<KERNEL>(a, r2b, w[6]);
+      o.x = fmaf(dx, f, o.x);
+      o.y = fmaf(dy, f, o.y);
+      o.z = fmaf(dz, f, o.z);
+      ++o.n;
     }
-    float f = pair_factor<ACC>(a, r2b, A.w);
-    f = ok ? f : 0.f;
-    fx = fmaf(dx, f, fx);
-    fy = fmaf(dy, f, fy);
-    fz = fmaf(dz, f, fz);
-    nok += ok ? 1u : 0u;  // the target's own leaf is masked out at emission
   }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    o.x += __shfl_xor_sync(0xffffffffu, o.x, off);
+    o.y += __shfl_xor_sync(0xffffffffu, o.y, off);
+    o.z += __shfl_xor_sync(0xffffffffu, o.z, off);
+    o.n += __shfl_xor_sync(0xffffffffu, o.n, off);
+  }
+  return o;
 }
 
-// Float64 decisions for this lane's borderline pairs of one list (rare).
-template <bool MONO>
-__device__ __noinline__ void resolve_list(const WalkArgs& a, const Entry* L, int nl, uint32_t lanes, uint32_t p,
-                                          float tx, float ty, float tz, float* f3, uint32_t* nok, uint32_t* nexact) {
-  const int t = lanes & 0xffu, stride = lanes >> 16;
-  for (int e = (lanes >> 8) & 0xffu; e < nl; e += stride) {
-    const float4 A = *reinterpret_cast<const float4*>(&L[e].x);
-    const uint4 B = *reinterpret_cast<const uint4*>(&L[e].h);
-    const float h = __uint_as_float(B.x);
-    const uint32_t mask = B.y, node = B.z;
-    const float dx = A.x - tx, dy = A.y - ty, dz = A.z - tz;
-    const float r2b = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-    float s = r2b;
-    if (MONO || !a.periodic) {
-      const float ex = fmaxf(fabsf(dx) - h, 0.f), ey = fmaxf(fabsf(dy) - h, 0.f);
-      const float ez = fmaxf(fabsf(dz) - h, 0.f);
-      s = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
+// A list against this lane's pair-phase target (its position comes from the
+// lane that holds it, its particle is first + target).
+template <int CUT, bool BAND, bool NEAR, int KERNEL, class L>
+__device__ __forceinline__ Sums eval(const WalkArgs& a, const L& list, int n, uint32_t lanes, uint32_t first,
+                                     const float4* tfs, const float4& T, uint32_t& nexact) {
+  Sums o;
+  const bool flag = eval_list<CUT, BAND, NEAR, KERNEL>(a, list, n, lanes, T.x, T.y, T.z, o);
+  if (BAND || NEAR) {
+    uint32_t again = __ballot_sync(0xffffffffu, flag);
+    while (again) {
+      const int src = __ffs(again) - 1;
+      again &= again - 1;
+      const uint32_t sl = __shfl_sync(0xffffffffu, lanes, src);
+      const float4 S = tfs[sl & 0xffu];
+      const Sums r = redo_lane<CUT, NEAR, KERNEL>(a, list, n, sl, first + (sl & 0xffu), S.x, S.y, S.z, &nexact);
+      if ((threadIdx.x & 31) == src) o = r;
     }
-    const bool in = (mask >> t) & 1u;
-    bool amb = in && s > a.prc2_lo && s <= a.prc2_hi;
-    if (MONO) amb = amb || (in && r2b < a.tiny_u);
-    if (!amb) continue;
-    ++*nexact;
-    const int d = exact_terminal(a, p, node);
-    if (d == 2) defer(a, p, node);
-    if (d != 1) continue;
-    const float f = pair_factor(a, r2b, A.w);
-    f3[0] = fmaf(dx, f, f3[0]);
-    f3[1] = fmaf(dy, f, f3[1]);
-    f3[2] = fmaf(dz, f, f3[2]);
-    ++*nok;
   }
+  return o;
 }
 
-// Evaluate both interaction lists against this lane's pair-phase target
-// (pair_lanes; its position is read from the lane that holds it, its
-// particle is first + target).
+// Evaluate both interaction lists against this lane's pair-phase target.
 // The lane's running sums live in shared memory between flushes (s0 = sx, sy,
 // sz, cx; s1 = cy, cz, leaf count, monopole count bits), so they hold no
 // registers across the traversal.
-template <bool ACC>
-__device__ __forceinline__ void flush(const WalkArgs& a, const Entry* Ll, int nll, const Entry* Lm, int nlm, int lane,
-                                      uint32_t count, uint32_t first, const float4* tfs, float4* s0, float4* s1,
-                                      uint32_t& nexact, uint32_t& neval) {
-  const uint32_t lanes = pair_lanes(lane, count);  // recomputed here: one register less across the traversal
-  uint32_t nleaf = 0, nmono = 0;
-  float fx = 0.f, fy = 0.f, fz = 0.f;
-  bool amb_any = false;
+template <bool PERIODIC, int KERNEL> struct Lists {
+  static constexpr bool ACC = KERNEL == K_ACC;
+  List<CHUNK_L, !PERIODIC> leaf;
+  List<chunk_m<ACC>(), ACC || !PERIODIC> mono;
+};
+template <bool PERIODIC, int KERNEL>
+__device__ __forceinline__ void flush(const WalkArgs& a, const Lists<PERIODIC, KERNEL>& lists, int nll, int nlm,
+                                      int lane, uint32_t lanes, uint32_t first, const float4* tfs, float4* s0,
+                                      float4* s1, uint32_t& nexact, uint32_t& neval) {
+  constexpr bool ACC = KERNEL == K_ACC;
   neval += (uint32_t)(nll + nlm);
-  const int t = lanes & 0xffu;
-  const float4 T = tfs[t];
-  const float tx = T.x, ty = T.y, tz = T.z;
-  flush_list<false, ACC>(a, Ll, nll, lanes, tx, ty, tz, fx, fy, fz, nleaf, amb_any);
-  flush_list<true, ACC>(a, Lm, nlm, lanes, tx, ty, tz, fx, fy, fz, nmono, amb_any);
-  if (!ACC && amb_any) {
-    float f3[3] = {fx, fy, fz};
-    const uint32_t p = first + (uint32_t)t;
-    resolve_list<false>(a, Ll, nll, lanes, p, tx, ty, tz, f3, &nleaf, &nexact);
-    resolve_list<true>(a, Lm, nlm, lanes, p, tx, ty, tz, f3, &nmono, &nexact);
-    fx = f3[0];
-    fy = f3[1];
-    fz = f3[2];
-  }
+  const float4 T = tfs[lanes & 0xffu];
+  const Sums l = eval<PERIODIC ? CUT_BARE : CUT_OWN_HALF, !ACC, false, KERNEL>(a, lists.leaf, nll, lanes, first,
+                                                                               tfs, T, nexact);
+  const Sums m = eval<ACC ? CUT_OWN_HALF : CUT_ONE_HALF, !ACC, !ACC, KERNEL>(a, lists.mono, nlm, lanes, first, tfs,
+                                                                             T, nexact);
   __syncwarp();
   const float4 A = s0[lane], B = s1[lane];
   Acc acc = {A.x, A.y, A.z, A.w, B.x, B.y};
-  acc.add(fx, fy, fz);
+  acc.add(l.x + m.x, l.y + m.y, l.z + m.z);
   s0[lane] = make_float4(acc.sx, acc.sy, acc.sz, acc.cx);
-  s1[lane] = make_float4(acc.cy, acc.cz, __uint_as_float(__float_as_uint(B.z) + nleaf),
-                         __uint_as_float(__float_as_uint(B.w) + nmono));
+  s1[lane] = make_float4(acc.cy, acc.cz, __uint_as_float(__float_as_uint(B.z) + l.n),
+                         __uint_as_float(__float_as_uint(B.w) + m.n));
 }
 
 // Stack entry of an open node: its children's record range, mask of the
@@ -331,13 +475,310 @@ struct __align__(16) StackEntry {
 constexpr int STACK_ENTRIES = 1024;  // global, per warp
 constexpr uint32_t INFO_MAC = 0x40000000u;  // opening angle undecided for the group
 
-// Walk the tree for targets [first, first + count) (count <= TPW) with one warp.
-template <int TPW, bool ACC>
-__device__ void walk_targets(const WalkArgs& a, uint32_t first, uint32_t count, Entry* Ll, Entry* Lm, uint8_t* owner,
-                             StackEntry* stk, float4* rpos, uint4* rmask, float4* s0, float4* s1, float4* tfs,
-                             float4* gbox) {
+// End of a group's walk: fold the pair-phase lanes of each target, write its
+// acceleration and interaction counts, add to the statistics.
+__device__ __forceinline__ void store_sums(const WalkArgs& a, uint32_t p, bool has, uint32_t count, float4 S0,
+                                           float4 S1, uint32_t nexact, uint32_t neval) {
   const int lane = threadIdx.x & 31;
-  const int tgt = lane & (TPW - 1);  // this lane's target within the group
+  Acc acc = {S0.x, S0.y, S0.z, S0.w, S1.x, S1.y};
+  uint32_t nleaf = __float_as_uint(S1.z), nmono = __float_as_uint(S1.w);
+  // fold the R pair-phase lanes of each target (lanes t + j count) into lane t
+  const uint32_t nrep = 32u / count;
+  for (uint32_t j = 1; j < nrep; ++j) {
+    const int src = lane + (int)(j * count);  // in range for the lanes t < count that keep the result
+    const float ox = __shfl_sync(0xffffffffu, acc.sx, src), oy = __shfl_sync(0xffffffffu, acc.sy, src);
+    const float oz = __shfl_sync(0xffffffffu, acc.sz, src);
+    const float cx = __shfl_sync(0xffffffffu, acc.cx, src), cy = __shfl_sync(0xffffffffu, acc.cy, src);
+    const float cz = __shfl_sync(0xffffffffu, acc.cz, src);
+    const uint32_t ol = __shfl_sync(0xffffffffu, nleaf, src), om = __shfl_sync(0xffffffffu, nmono, src);
+    if ((uint32_t)lane < count) {
+      acc.add(ox - cx, oy - cy, oz - cz);
+      nleaf += ol;
+      nmono += om;
+    }
+  }
+  if (has) {
+    a.ax[p] = (acc.sx - acc.cx) * a.out_scale;
+    a.ay[p] = (acc.sy - acc.cy) * a.out_scale;
+    a.az[p] = (acc.sz - acc.cz) * a.out_scale;
+    a.pcounts[2 * (int64_t)p] = nleaf;
+    a.pcounts[2 * (int64_t)p + 1] = nmono;
+  }
+  if ((uint32_t)lane >= count) nleaf = nmono = 0;  // counted once per target
+  // statistics
+  unsigned long long l = nleaf, m = nmono, x = nexact;
+  for (int off = 16; off > 0; off >>= 1) {
+    l += __shfl_down_sync(0xffffffffu, l, off);
+    m += __shfl_down_sync(0xffffffffu, m, off);
+    x += __shfl_down_sync(0xffffffffu, x, off);
+  }
+  if (lane == 0) {
+    atomicAdd(&a.stats[0], l);
+    atomicAdd(&a.stats[1], m);
+    atomicAdd(&a.stats[2], (unsigned long long)neval * 32ull / nrep);  // lane evaluations
+    atomicAdd(&a.stats[3], x);
+  }
+}
+
+// Shared memory of one warp.
+template <bool PERIODIC, int KERNEL> struct __align__(16) WarpMem {
+  Lists<PERIODIC, KERNEL> lists;
+  union {
+    struct {  // accurate: staged undecided nodes: position, half side; mask, node, image flag
+      float4 rpos[32];
+      uint4 rmask[32];
+    };
+    struct {  // parity: staged undecided nodes (half side in place of the mass), the targets that see them
+      List<32, false> nodes;
+      uint2 seen[16];
+    };
+  };
+  float4 s0[32], s1[32];  // the lanes' running sums
+  float4 tfs[32];   // target positions
+  float4 gbox[4];   // group box (accurate: corners; parity: half widths) and origin
+  uint4 queue[40];  // parity: nodes whose terminal children wait {first record, count, mask}
+  uint8_t owner[32];  // accurate: child owners of a popped batch
+};
+
+// The staged undecided nodes of an open step again (rare: a node seen at
+// another periodic image, marked in its node word, or a target inside the band
+// around r_cut^2), with the nearest image per target and the reference's
+// float64 test inside the band.
+__device__ __noinline__ uint32_t refine_exact(const WalkArgs& a, const List<32, false>& nodes, int n, uint32_t p,
+                                              float4 T, uint2* seen) {
+  const int lane = threadIdx.x & 31;
+  uint32_t nexact = 0;
+  for (int j = 0; j < n; ++j) {
+    const float* w = nodes.word(j);
+    const uint32_t node = __float_as_uint(w[10]);
+    float dx = w[0] - T.x, dy = w[2] - T.y, dz = w[4] - T.z;
+    if (node & LEAF_BIT) {
+      dx -= a.box_u * rintf(dx / a.box_u);
+      dy -= a.box_u * rintf(dy / a.box_u);
+      dz -= a.box_u * rintf(dz / a.box_u);
+    }
+    const float s = cut_s<CUT_OWN_HALF>(dx, dy, dz, 0.f, w[6]);
+    const bool in = (__float_as_uint(w[8]) >> lane) & 1u;
+    bool pass = in && s <= a.rc2_lo;
+    if (in && !pass && s <= a.rc2_hi) {
+      pass = exact_open_pass(a, p, node & ~LEAF_BIT);
+      ++nexact;
+    }
+    const uint32_t nm = __ballot_sync(0xffffffffu, pass);
+    if (lane == 0) reinterpret_cast<uint32_t*>(seen)[j] = nm;
+  }
+  return nexact;
+}
+
+// Parity walk of targets [first, first + count) (count <= 32) with one warp.
+//
+// An octree node's children are stored internal nodes first, leaves after
+// them, and internal nodes become monopoles at one depth for the whole tree.
+// So a node that stays open splits into a range of open children and a range
+// of terminal ones, and the walk has two kinds of step, each on four nodes at a
+// time with eight lanes per node (a node has at most eight children, so no
+// lane has to look up its child): an open step classifies open children
+// against the group box, tests the undecided ones per target and pushes what
+// is seen; an item step cuts terminal children against the group box and
+// appends them to the lists.  The item step, which meets most of the nodes,
+// needs neither the periodic images nor the opening test.
+template <bool PERIODIC, int KERNEL>
+__device__ __forceinline__ void walk_parity(const WalkArgs& a, uint32_t first, uint32_t count,
+                                            WarpMem<PERIODIC, KERNEL>& mem, uint4* stk) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t p = first + ((uint32_t)lane < count ? (uint32_t)lane : 0u);
+  // targets of this walk: the group's particles, or those of them the caller
+  // selected (the group box then covers only those)
+  const bool has = (uint32_t)lane < count && (!a.only || a.only[p] != 0);
+  const uint32_t mask0 = __ballot_sync(0xffffffffu, has);  // bit t: target t
+  if (mask0 == 0u) return;
+  {
+    const uint32_t tq[3] = {a.qx[p], a.qy[p], a.qz[p]};
+    uint32_t oq[3];
+    float tf[3], w[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      // positions relative to the middle of the group's box: half the extent
+      // bounds them, and with them the rounding of the pair distances
+      const uint32_t q0 = __shfl_sync(0xffffffffu, tq[d], 0);
+      const int32_t tr = rel32(tq[d], q0, PERIODIC);
+      const int32_t lo = __reduce_min_sync(0xffffffffu, has ? tr : 0x7FFFFFFF);
+      const int32_t hi = __reduce_max_sync(0xffffffffu, has ? tr : -0x7FFFFFFF);
+      const int32_t mid = lo + ((hi - lo) >> 1);
+      oq[d] = q0 + (uint32_t)mid;
+      tf[d] = (float)(tr - mid) * a.u_inv;
+      w[d] = (float)(hi - mid) * a.u_inv;
+    }
+    mem.tfs[lane] = make_float4(tf[0], tf[1], tf[2], 0.f);
+    if (lane == 0) {
+      mem.gbox[0] = make_float4(w[0], w[1], w[2], 0.f);
+      reinterpret_cast<uint4*>(mem.gbox)[1] = make_uint4(oq[0], oq[1], oq[2], 0u);
+      // the root: a terminal node by itself, or an open one
+      const bool item = a.term_depth == 0;
+      if (item) mem.queue[0] = make_uint4(0u, 1u, mask0, 0u);
+      else stk[0] = make_uint4(0u, 1u, mask0, 0u);
+    }
+  }
+  mem.s0[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+  mem.s1[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+  const uint32_t lanes = pair_lanes(lane, count);
+  uint32_t nexact = 0, neval = 0;
+  int nll = 0, nlm = 0, sp = a.term_depth == 0 ? 0 : 1, nq = 1 - sp;
+  // each step takes at least one range, and a node makes at most two: the cap
+  // turns a malformed tree into an error flag instead of an endless loop
+  uint32_t steps_left = (uint32_t)(2 * a.n_int + 4 < 0xFFFFFFFFll ? 2 * a.n_int + 4 : 0xFFFFFFFFll);
+  const uint32_t below = (1u << lane) - 1u;
+  __syncwarp();
+  const int slot = lane >> 3, child = lane & 7;
+  for (;;) {
+    if (steps_left-- == 0u) {
+      if (lane == 0) atomicOr(a.err, DEV_ERR_STACK);
+      break;
+    }
+    const float4 GW = mem.gbox[0];
+    const uint4 GO = reinterpret_cast<const uint4*>(mem.gbox)[1];
+    if (nq >= 4 || sp == 0) {  // ---- item step
+      const int np = nq < 4 ? nq : 4;
+      uint4 e = make_uint4(0u, 0u, 0u, 0u);
+      if (slot < np) e = mem.queue[nq - 1 - slot];
+      nq -= np;
+      bool keep = (uint32_t)child < e.y;
+      uint4 r0 = make_uint4(0u, 0u, 0u, 0u), r1 = r0;
+      if (keep) {
+        const uint4* rec = reinterpret_cast<const uint4*>(&a.recs[e.x + (uint32_t)child]);
+        r0 = __ldg(rec);
+        r1 = __ldg(rec + 1);
+      }
+      const bool leaf = (r1.y & WN_LEAF) != 0u;
+      const float h = !leaf ? a.h_term : (PERIODIC ? 0.f : half_side(a.h0_u, wn_depth(r1.y)));
+      const float sx = (float)rel32(r0.x, GO.x, PERIODIC) * a.u_inv, sy = (float)rel32(r0.y, GO.y, PERIODIC) * a.u_inv;
+      const float sz = (float)rel32(r0.z, GO.z, PERIODIC) * a.u_inv;
+      // the gap between the group box and the node's box
+      const float gx = fmaxf(fabsf(sx) - (GW.x + h), 0.f), gy = fmaxf(fabsf(sy) - (GW.y + h), 0.f);
+      const float gz = fmaxf(fabsf(sz) - (GW.z + h), 0.f);
+      keep = keep && !(fmaf(gx, gx, fmaf(gy, gy, gz * gz)) > a.grc2_hi);
+      const uint32_t el = __ballot_sync(0xffffffffu, keep && leaf), em = __ballot_sync(0xffffffffu, keep && !leaf);
+      if (keep) {
+        // the reference skips the target's own leaf (j != skip)
+        const uint32_t own = leaf ? r1.z - first : 32u;
+        const uint32_t see = own < count ? (e.z & ~(1u << own)) : e.z;
+        auto& list = leaf ? mem.lists.leaf : mem.lists.mono;  // the same layout
+        list.put(leaf ? nll + __popc(el & below) : nlm + __popc(em & below), sx, sy, sz, __uint_as_float(r0.w), h, see,
+                 leaf ? r1.z | LEAF_BIT : r1.z);
+      }
+      nll += __popc(el);
+      nlm += __popc(em);
+      const bool done = sp == 0 && nq == 0;
+      // the next item step adds up to 32 entries to either list (one call site
+      // of the list evaluation, the last flush included)
+      if (done || nll > CHUNK_L - 32 || nlm > chunk_m<false>() - 32) {
+        if (lane == 0) {
+          mem.lists.leaf.close(nll);
+          mem.lists.mono.close(nlm);
+        }
+        __syncwarp();
+        flush<PERIODIC, KERNEL>(a, mem.lists, nll, nlm, lane, lanes, first, mem.tfs, mem.s0, mem.s1, nexact, neval);
+        __syncwarp();
+        nll = 0;
+        nlm = 0;
+      }
+      if (done) break;
+      continue;
+    }
+    // ---- open step
+    const int np = sp < 4 ? sp : 4;
+    uint4 e = make_uint4(0u, 0u, 0u, 0u);
+    if (slot < np) e = stk[sp - 1 - slot];
+    sp -= np;
+    const bool live = (uint32_t)child < e.y;
+    uint4 r0 = make_uint4(0u, 0u, 0u, 0u), r1 = r0;
+    if (live) {
+      const uint4* rec = reinterpret_cast<const uint4*>(&a.recs[e.x + (uint32_t)child]);
+      r0 = __ldg(rec);
+      r1 = __ldg(rec + 1);
+    }
+    const int dep = wn_depth(r1.y);
+    const float h = half_side(a.h0_u, dep);
+    const float sx = (float)rel32(r0.x, GO.x, PERIODIC) * a.u_inv, sy = (float)rel32(r0.y, GO.y, PERIODIC) * a.u_inv;
+    const float sz = (float)rel32(r0.z, GO.z, PERIODIC) * a.u_inv;
+    const float ux = fabsf(sx), uy = fabsf(sy), uz = fabsf(sz);
+    // the nearest and the farthest a target can be from the node's box
+    const float gx = fmaxf(ux - (GW.x + h), 0.f), gy = fmaxf(uy - (GW.y + h), 0.f), gz = fmaxf(uz - (GW.z + h), 0.f);
+    const float fx = fmaxf(ux + (GW.x - h), 0.f), fy = fmaxf(uy + (GW.y - h), 0.f), fz = fmaxf(uz + (GW.z - h), 0.f);
+    // Nodes that part of the group sees at another periodic image are left to
+    // the per-target test, if they are wide enough for that image to come
+    // within r_cut.  The others: seen by the whole group, or undecided.
+    const float half_box = 0.5f * a.box_u;
+    const bool image = PERIODIC && live && dep < a.img_depth &&
+                       (ux + GW.x > half_box || uy + GW.y > half_box || uz + GW.z > half_box);
+    bool keep = live && (image || !(fmaf(gx, gx, fmaf(gy, gy, gz * gz)) > a.grc2_hi));
+    const bool ambig = keep && (image || !(fmaf(fx, fx, fmaf(fy, fy, fz * fz)) < a.grc2_lo));
+    const uint32_t amb = __ballot_sync(0xffffffffu, ambig);
+    uint32_t see = e.z;
+    if (amb != 0u) {
+      // Per-target refinement: each undecided node is staged once in shared
+      // memory, then tested against all targets (one per lane), two nodes at a
+      // time in packed arithmetic.  dd = COM - target in float differs from
+      // the exact minimum-image difference by ~1e-7 of r_cut, far inside the
+      // band around r_cut^2 that goes to the float64 test.
+      const int mine = __popc(amb & below), namb = __popc(amb);
+      if (ambig) mem.nodes.put(mine, sx, sy, sz, h, 0.f, e.z, image ? r1.z | LEAF_BIT : r1.z);
+      if (lane == 0) mem.nodes.close(namb);
+      const bool images = __any_sync(0xffffffffu, image);
+      __syncwarp();
+      const float4 TF = mem.tfs[lane];
+      const f32x2 ntx = pack2(-TF.x, -TF.x), nty = pack2(-TF.y, -TF.y), ntz = pack2(-TF.z, -TF.z);
+      const uint32_t tbit = 1u << lane;
+      float edge = 1e30f;
+      const f32x2 nmid = pack2(-a.rc2_mid, -a.rc2_mid);
+      for (int j = 0; j < namb; j += 2) {
+        auto& nd = mem.nodes.pair[j >> 1];
+        const float4 A = nd.xy, B = nd.zm;
+        const uint2 M = nd.mask;
+        const float2 x = unpack2(add2(pack2(A.x, A.y), ntx)), y = unpack2(add2(pack2(A.z, A.w), nty));
+        const float2 z = unpack2(add2(pack2(B.x, B.y), ntz));
+        const f32x2 ex = pack2(fmaxf(fabsf(x.x) - B.z, 0.f), fmaxf(fabsf(x.y) - B.w, 0.f));
+        const f32x2 ey = pack2(fmaxf(fabsf(y.x) - B.z, 0.f), fmaxf(fabsf(y.y) - B.w, 0.f));
+        const f32x2 ez = pack2(fmaxf(fabsf(z.x) - B.z, 0.f), fmaxf(fabsf(z.y) - B.w, 0.f));
+        const float2 q = unpack2(add2(fma2(ez, ez, fma2(ey, ey, mul2(ex, ex))), nmid));
+        edge = min3_abs(edge, q.x, q.y);
+        const uint32_t n0 = __ballot_sync(0xffffffffu, (M.x & tbit) && q.x <= 0.f);
+        const uint32_t n1 = __ballot_sync(0xffffffffu, (M.y & tbit) && q.y <= 0.f);
+        if (lane == 0) mem.seen[j >> 1] = make_uint2(n0, n1);
+      }
+      if (images || __any_sync(0xffffffffu, edge <= a.rc2_band)) nexact += refine_exact(a, mem.nodes, namb, p, TF, mem.seen);
+      __syncwarp();
+      if (ambig) see = reinterpret_cast<const uint32_t*>(mem.seen)[mine];
+      keep = keep && see != 0u;  // a node no target sees is not pushed
+    }
+    // the seen nodes' children: internal ones stay open above the terminal
+    // depth, the rest are items
+    const uint32_t inner = dep + 1 < a.term_depth ? wn_ninner(r1.y) : 0u, rest = wn_nchild(r1.y) - inner;
+    const uint32_t po = __ballot_sync(0xffffffffu, keep && inner != 0u);
+    const uint32_t pi = __ballot_sync(0xffffffffu, keep && rest != 0u);
+    if (sp + __popc(po) > STACK_ENTRIES) {
+      if (lane == 0) atomicOr(a.err, DEV_ERR_STACK);
+      break;
+    }
+    if (keep && inner != 0u) stk[sp + __popc(po & below)] = make_uint4(r1.x, inner, see, 0u);
+    if (keep && rest != 0u) mem.queue[nq + __popc(pi & below)] = make_uint4(r1.x + inner, rest, see, 0u);
+    sp += __popc(po);
+    nq += __popc(pi);
+    __syncwarp();
+    if (sp == 0 && nq == 0 && nll + nlm == 0) break;  // nothing in reach
+  }
+  __syncwarp();
+  store_sums(a, p, has, count, mem.s0[lane], mem.s1[lane], nexact, neval);
+}
+
+// Accurate walk of targets [first, first + count) (count <= 32) with one warp:
+// whether a node is opened depends on its distance from each target.
+template <bool PERIODIC>
+__device__ void walk_accurate(const WalkArgs& a, uint32_t first, uint32_t count, Lists<PERIODIC, K_ACC>& lists,
+                             uint8_t* owner, StackEntry* stk, float4* rpos, uint4* rmask, float4* s0, float4* s1,
+                             float4* tfs, float4* gbox) {
+  const int lane = threadIdx.x & 31;
+  const int tgt = lane;  // this lane's target within the group
   const uint32_t p = first + ((uint32_t)tgt < count ? (uint32_t)tgt : 0u);
   // targets of this walk: the group's particles, or those of them the caller
   // selected (the group box then covers only those)
@@ -350,7 +791,7 @@ __device__ void walk_targets(const WalkArgs& a, uint32_t first, uint32_t count, 
   float tf[3], bmin[3], bmax[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    tr[d] = rel32(tq[d], oq[d], a.periodic);
+    tr[d] = rel32(tq[d], oq[d], PERIODIC);
     tf[d] = (float)tr[d] * a.u_inv;
     int32_t mn = __reduce_min_sync(0xffffffffu, has ? tr[d] : 0x7FFFFFFF);
     int32_t mx = __reduce_max_sync(0xffffffffu, has ? tr[d] : -0x7FFFFFFF);
@@ -367,10 +808,10 @@ __device__ void walk_targets(const WalkArgs& a, uint32_t first, uint32_t count, 
     reinterpret_cast<uint4*>(gbox)[2] = make_uint4(oq[0], oq[1], oq[2], 0u);
   }
   __syncwarp();
-  const uint32_t mask0 = __ballot_sync(0xffffffffu, has && lane < TPW);  // bit t: target t
+  const uint32_t mask0 = __ballot_sync(0xffffffffu, has);  // bit t: target t
   s0[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
   s1[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
-  uint32_t nexact = 0, neval = 0;
+  uint32_t neval = 0, none = 0;
   int nll = 0, nlm = 0, sp = 0;
 
   // the first item is the root record
@@ -389,7 +830,9 @@ __device__ void walk_targets(const WalkArgs& a, uint32_t first, uint32_t count, 
     }
     // ---- classify this lane's item against the group box
     bool emit = false, push = false, ambig = false, is_leaf = false;
-    Entry ent;
+    float4 ent;  // a terminal node: group-relative position, mass
+    float ent_h = 0.f;
+    uint32_t ent_mask = 0u, ent_node = 0u;
     StackEntry se;
     float sx = 0.f, sy = 0.f, sz = 0.f, sh = 0.f;  // an undecided open node: group-relative COM, cull half side
     uint32_t simg = 0u;
@@ -400,9 +843,8 @@ __device__ void walk_targets(const WalkArgs& a, uint32_t first, uint32_t count, 
       const bool leaf = (info & WN_LEAF) != 0;
       const int dep = wn_depth(info);
       const float hnode = half_side(a.h0_u, dep);
-      // cull half side: the COM-centred AABB of the reference, or (accurate
-      // mode) twice that, which holds the whole cell
-      const float h = (leaf && a.periodic) ? 0.f : (ACC && !leaf ? 2.f * hnode : hnode);
+      // cull half side: twice the COM-centred AABB's, which holds the whole cell
+      const float h = leaf ? (PERIODIC ? 0.f : hnode) : 2.f * hnode;
       const uint32_t cq[3] = {r0.x, r0.y, r0.z};
       const float4 GL = gbox[0], GH = gbox[1];
       const uint4 GO = reinterpret_cast<const uint4*>(gbox)[2];
@@ -416,15 +858,15 @@ __device__ void walk_targets(const WalkArgs& a, uint32_t first, uint32_t count, 
       float SF[3];
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        S[d] = rel32(cq[d], oq[d], a.periodic);
+        S[d] = rel32(cq[d], oq[d], PERIODIC);
         const float sf = (float)S[d] * a.u_inv;
         SF[d] = sf;
         const float lo = sf - bmax[d], hi = sf - bmin[d];
         float dmin = lo > 0.f ? lo : (hi < 0.f ? -hi : 0.f);
         float dmax = fmaxf(fabsf(lo), fabsf(hi));
-        // the +-L images can only come within r_cut of a group (narrower than
-        // L/16) for nodes of half side near L/2: the top levels
-        if (a.periodic && dep < a.img_depth) {
+        // the +-L images can only come within r_cut of a group (no wider than
+        // max_extent) for nodes of half side near L/2: the top levels
+        if (PERIODIC && dep < a.img_depth) {
           dmin = fminf(dmin, fminf(a.box_u - hi, lo + a.box_u));
           const float half = 0.5f * a.box_u;
           if (lo <= -half || hi >= half) dmax = half;
@@ -438,7 +880,7 @@ __device__ void walk_targets(const WalkArgs& a, uint32_t first, uint32_t count, 
         dmax2 = fmaf(dmax, dmax, dmax2);
       }
       bool open, macmix = false;
-      if (ACC && !leaf) {
+      if (!leaf) {
         bool accept_all, open_all;
         if (a.relative) {
           // relative criterion (octree.rs:769-796): accept when the target is
@@ -453,7 +895,7 @@ __device__ void walk_targets(const WalkArgs& a, uint32_t first, uint32_t count, 
           bool touch = true, inside_all = true;
 #pragma unroll
           for (int d = 0; d < 3; ++d) {
-            const float c = (float)rel32(ccq[d], oq[d], a.periodic) * a.u_inv;
+            const float c = (float)rel32(ccq[d], oq[d], PERIODIC) * a.u_inv;
             const float lo = c - hnode * 1.0001f, hi = c + hnode * 1.0001f;
             touch = touch && lo <= bmax[d] && hi >= bmin[d];
             inside_all = inside_all && lo <= bmin[d] && hi >= bmax[d];
@@ -461,7 +903,7 @@ __device__ void walk_targets(const WalkArgs& a, uint32_t first, uint32_t count, 
           const float dmn = sqrtf(dmin2), dmx = sqrtf(dmax2);
           accept_all = !touch && dmin2 > 0.f &&
                        qf * (dmin2 + a.eps2_u) < a.rel_k * m * (dmin2 * dmin2 * dmn) * 0.999f;
-          open_all = (a.periodic && dep < a.img_depth) || inside_all ||
+          open_all = (PERIODIC && dep < a.img_depth) || inside_all ||
                      !(qf * (dmax2 + a.eps2_u) < a.rel_k * m * (dmax2 * dmax2 * dmx) * 1.001f);
           accept_all = accept_all && !open_all;
         } else {
@@ -475,7 +917,7 @@ __device__ void walk_targets(const WalkArgs& a, uint32_t first, uint32_t count, 
         open = !accept_all;
         macmix = !accept_all && !open_all;
       } else {
-        open = !leaf && !(info & WN_TERMINAL);
+        open = false;
       }
       if (!(emin2 > a.grc2_hi)) {
         if (open) {
@@ -490,19 +932,16 @@ __device__ void walk_targets(const WalkArgs& a, uint32_t first, uint32_t count, 
             sy = SF[1];
             sz = SF[2];
             sh = h;
-            simg = (a.periodic && dep < a.img_depth) ? 1u : 0u;
+            simg = (PERIODIC && dep < a.img_depth) ? 1u : 0u;
           }
         } else {
           emit = true;
-          ent.x = (float)S[0] * a.u_inv;
-          ent.y = (float)S[1] * a.u_inv;
-          ent.z = (float)S[2] * a.u_inv;
-          ent.m = __uint_as_float(r0.w);
-          ent.h = h;
+          ent = make_float4(SF[0], SF[1], SF[2], __uint_as_float(r0.w));
+          ent_h = h;
           // the reference skips the target's own leaf (j != skip)
           const uint32_t own = leaf ? r1.z - first : 32u;
-          ent.mask = own < count ? (imask & ~(1u << own)) : imask;
-          ent.node = leaf ? (r1.z | LEAF_BIT) : r1.z;
+          ent_mask = own < count ? (imask & ~(1u << own)) : imask;
+          ent_node = leaf ? (r1.z | LEAF_BIT) : r1.z;
           is_leaf = leaf;
         }
       }
@@ -512,10 +951,8 @@ __device__ void walk_targets(const WalkArgs& a, uint32_t first, uint32_t count, 
     const uint32_t emm = __ballot_sync(0xffffffffu, emit && !is_leaf);
     if (emit) {
       const unsigned lt = (1u << lane) - 1u;
-      Entry* dstE = is_leaf ? &Ll[nll + __popc(eml & lt)] : &Lm[nlm + __popc(emm & lt)];
-      float4* dst = reinterpret_cast<float4*>(dstE);
-      dst[0] = make_float4(ent.x, ent.y, ent.z, ent.m);
-      *reinterpret_cast<uint4*>(&dst[1]) = make_uint4(__float_as_uint(ent.h), ent.mask, ent.node, 0u);
+      if (is_leaf) lists.leaf.put(nll + __popc(eml & lt), ent.x, ent.y, ent.z, ent.w, ent_h, ent_mask, ent_node);
+      else lists.mono.put(nlm + __popc(emm & lt), ent.x, ent.y, ent.z, ent.w, ent_h, ent_mask, ent_node);
     }
     nll += __popc(eml);
     nlm += __popc(emm);
@@ -540,7 +977,7 @@ __device__ void walk_targets(const WalkArgs& a, uint32_t first, uint32_t count, 
       const float4 R = rpos[j];
       const uint4 M = rmask[j];
       bool pass = false;
-      if (has && lane < TPW && ((M.x >> tgt) & 1u)) {
+      if (has && ((M.x >> tgt) & 1u)) {
         const float rc[3] = {R.x, R.y, R.z};
         float s = 0.f;
 #pragma unroll
@@ -551,12 +988,8 @@ __device__ void walk_targets(const WalkArgs& a, uint32_t first, uint32_t count, 
           s = fmaf(ee, ee, s);
         }
         if (s <= a.rc2_lo) pass = true;
-        else if (!ACC && s <= a.rc2_hi) {
-          pass = exact_open_pass(a, p, M.y);
-          ++nexact;
-        }
       }
-      const uint32_t nm = __ballot_sync(0xffffffffu, pass);  // lanes < TPW hold the targets
+      const uint32_t nm = __ballot_sync(0xffffffffu, pass);
       if (lane == 0) rmask[j].x = nm;
     }
     __syncwarp();
@@ -581,9 +1014,15 @@ __device__ void walk_targets(const WalkArgs& a, uint32_t first, uint32_t count, 
     // (one call site of the list evaluation, the last flush included: the
     // kernel's code stays small enough for the instruction cache)
     const bool done = sp == 0;
-    if (done || nll > CHUNK_L - 32 || nlm > chunk_m<ACC>() - (ACC ? 64 : 32)) {
-      if (nll + nlm > 0)
-        flush<ACC>(a, Ll, nll, Lm, nlm, lane, count, first, tfs, s0, s1, nexact, neval);
+    if (done || nll > CHUNK_L - 32 || nlm > chunk_m<true>() - 64) {
+      if (nll + nlm > 0) {
+        if (lane == 0) {
+          lists.leaf.close(nll);
+          lists.mono.close(nlm);
+        }
+        __syncwarp();
+        flush<PERIODIC, K_ACC>(a, lists, nll, nlm, lane, pair_lanes(lane, count), first, tfs, s0, s1, none, neval);
+      }
       __syncwarp();
       nll = 0;
       nlm = 0;
@@ -602,14 +1041,14 @@ __device__ void walk_targets(const WalkArgs& a, uint32_t first, uint32_t count, 
     const int k = __popc(take);
     sp -= k;
     uint4 wrec = make_uint4(0u, 0u, 0u, 0u), crec = make_uint4(0u, 0u, 0u, 0u);
-    if (ACC && lane < k && (e.y & INFO_MAC)) {
+    if (lane < k && (e.y & INFO_MAC)) {
       wrec = __ldg(&a.walk[e.w]);
       if (a.relative) crec = __ldg(&a.cellq[e.w]);
     }
     // accurate mode: per-target opening angle for nodes undecided for the
     // group; targets that accept take the node as a monopole now, the rest
     // open it
-    uint32_t macm = ACC ? __ballot_sync(0xffffffffu, lane < k && (e.y & INFO_MAC)) : 0u;
+    uint32_t macm = __ballot_sync(0xffffffffu, lane < k && (e.y & INFO_MAC));
     while (macm) {
       const int src = __ffs(macm) - 1;
       macm &= macm - 1;
@@ -624,12 +1063,12 @@ __device__ void walk_targets(const WalkArgs& a, uint32_t first, uint32_t count, 
         cw = make_uint4(__shfl_sync(0xffffffffu, crec.x, src), __shfl_sync(0xffffffffu, crec.y, src),
                         __shfl_sync(0xffffffffu, crec.z, src), __shfl_sync(0xffffffffu, crec.w, src));
       bool accept = false;
-      if (has && lane < TPW && ((me >> tgt) & 1u)) {
+      if (has && ((me >> tgt) & 1u)) {
         float d2 = 0.f;
         const uint32_t wq[3] = {w.x, w.y, w.z};
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-          const float dd = (float)rel32(wq[d], tq[d], a.periodic) * a.u_inv;
+          const float dd = (float)rel32(wq[d], tq[d], PERIODIC) * a.u_inv;
           d2 = fmaf(dd, dd, d2);
         }
         if (a.relative) {
@@ -639,7 +1078,7 @@ __device__ void walk_targets(const WalkArgs& a, uint32_t first, uint32_t count, 
           bool inside = true;
 #pragma unroll
           for (int d = 0; d < 3; ++d)
-            inside = inside && fabsf((float)rel32(cq3[d], tq[d], a.periodic) * a.u_inv) <= hnode * 1.0001f;
+            inside = inside && fabsf((float)rel32(cq3[d], tq[d], PERIODIC) * a.u_inv) <= hnode * 1.0001f;
           const float qf = __uint_as_float(cw.w), m = __uint_as_float(w.w);
           accept = !inside && d2 > 0.f && qf * (d2 + a.eps2_u) < a.rel_k * m * (d2 * d2 * sqrtf(d2));
         } else {
@@ -651,11 +1090,9 @@ __device__ void walk_targets(const WalkArgs& a, uint32_t first, uint32_t count, 
         if (lane == src) {
           const uint4 GO = reinterpret_cast<const uint4*>(gbox)[2];
           const uint32_t oq[3] = {GO.x, GO.y, GO.z};
-          float4* dst = reinterpret_cast<float4*>(&Lm[nlm]);
-          dst[0] = make_float4((float)rel32(w.x, oq[0], a.periodic) * a.u_inv,
-                               (float)rel32(w.y, oq[1], a.periodic) * a.u_inv,
-                               (float)rel32(w.z, oq[2], a.periodic) * a.u_inv, __uint_as_float(w.w));
-          *reinterpret_cast<uint4*>(&dst[1]) = make_uint4(__float_as_uint(2.f * hnode), am, node, 0u);
+          lists.mono.put(nlm, (float)rel32(w.x, oq[0], PERIODIC) * a.u_inv,
+                         (float)rel32(w.y, oq[1], PERIODIC) * a.u_inv, (float)rel32(w.z, oq[2], PERIODIC) * a.u_inv,
+                         __uint_as_float(w.w), 2.f * hnode, am, node);
         }
         ++nlm;
       }
@@ -680,97 +1117,32 @@ __device__ void walk_targets(const WalkArgs& a, uint32_t first, uint32_t count, 
     }
   }
   __syncwarp();
-  __syncwarp();
-  const float4 S0 = s0[lane], S1 = s1[lane];
-  Acc acc = {S0.x, S0.y, S0.z, S0.w, S1.x, S1.y};
-  uint32_t nleaf = __float_as_uint(S1.z), nmono = __float_as_uint(S1.w);
-  // fold the R pair-phase lanes of each target (lanes t + j count) into lane t
-  const uint32_t nrep = 32u / count;
-  for (uint32_t j = 1; j < nrep; ++j) {
-    const int src = lane + (int)(j * count);  // in range for the lanes t < count that keep the result
-    const float ox = __shfl_sync(0xffffffffu, acc.sx, src), oy = __shfl_sync(0xffffffffu, acc.sy, src);
-    const float oz = __shfl_sync(0xffffffffu, acc.sz, src);
-    const float cx = __shfl_sync(0xffffffffu, acc.cx, src), cy = __shfl_sync(0xffffffffu, acc.cy, src);
-    const float cz = __shfl_sync(0xffffffffu, acc.cz, src);
-    const uint32_t ol = __shfl_sync(0xffffffffu, nleaf, src), om = __shfl_sync(0xffffffffu, nmono, src);
-    if ((uint32_t)lane < count) {
-      acc.add(ox - cx, oy - cy, oz - cz);
-      nleaf += ol;
-      nmono += om;
-    }
-  }
-  if (has && lane < TPW) {
-    a.ax[p] = (acc.sx - acc.cx) * a.out_scale;
-    a.ay[p] = (acc.sy - acc.cy) * a.out_scale;
-    a.az[p] = (acc.sz - acc.cz) * a.out_scale;
-    a.pcounts[2 * (int64_t)p] = nleaf;
-    a.pcounts[2 * (int64_t)p + 1] = nmono;
-  }
-  if ((uint32_t)lane >= count || lane >= TPW) nleaf = nmono = 0;  // counted once per target
-  // statistics
-  unsigned long long l = nleaf, m = nmono, x = nexact;
-  for (int off = 16; off > 0; off >>= 1) {
-    l += __shfl_down_sync(0xffffffffu, l, off);
-    m += __shfl_down_sync(0xffffffffu, m, off);
-    x += __shfl_down_sync(0xffffffffu, x, off);
-  }
-  if (lane == 0) {
-    atomicAdd(&a.stats[0], l);
-    atomicAdd(&a.stats[1], m);
-    atomicAdd(&a.stats[2], (unsigned long long)neval * 32ull / nrep);  // lane evaluations
-    atomicAdd(&a.stats[3], x);
-  }
+  store_sums(a, p, has, count, s0[lane], s1[lane], none, neval);
 }
 
-// per warp: the leaf and monopole lists, 32 staged undecided nodes (float4
-// position + uint4 mask / node / image flag), the lanes' running sums (two
-// float4 each), the child-owner bytes
-template <bool ACC> constexpr size_t walk_smem_per_warp() {
-  return sizeof(Entry) * (CHUNK_L + chunk_m<ACC>()) + 32 * (sizeof(float4) + sizeof(uint4)) + 100 * sizeof(float4) + 32;
-}
-
-template <int MIN_BLOCKS, int TPW, bool ACC>
-__global__ void __launch_bounds__(WALK_THREADS, MIN_BLOCKS) k_walk(WalkArgs a) {
+template <int MIN_BLOCKS, bool PERIODIC, int KERNEL>
+__global__ void __launch_bounds__(WALK_THREADS, MIN_BLOCKS) k_walk(const __grid_constant__ WalkArgs a) {
   extern __shared__ __align__(16) unsigned char s_walk[];
+  using Mem = WarpMem<PERIODIC, KERNEL>;
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  unsigned char* mine = s_walk + wid * walk_smem_per_warp<ACC>();
-  Entry* list_l = reinterpret_cast<Entry*>(mine);
-  Entry* list_m = list_l + CHUNK_L;
-  float4* rpos = reinterpret_cast<float4*>(list_m + chunk_m<ACC>());
-  uint4* rmask = reinterpret_cast<uint4*>(rpos + 32);
-  float4* s0 = reinterpret_cast<float4*>(rmask + 32);
-  float4* s1 = s0 + 32;
-  float4* tfs = s1 + 32;   // 32 target positions
-  float4* gbox = tfs + 32; // group box corners and origin (3, padded to 4)
-  uint8_t* owner = reinterpret_cast<uint8_t*>(gbox + 4);
+  Mem& mem = reinterpret_cast<Mem*>(s_walk)[wid];
+  // a list's unused half pair is evaluated and dropped: it must hold numbers
+  for (int i = lane; i < (int)(sizeof(mem.lists) / sizeof(uint32_t)); i += 32)
+    reinterpret_cast<uint32_t*>(&mem.lists)[i] = 0u;
+  __syncwarp();
   const int64_t gw = (int64_t)blockIdx.x * WALK_WARPS + wid;
-  StackEntry* stk = reinterpret_cast<StackEntry*>(a.stack) + gw * STACK_ENTRIES;
+  uint4* stk = reinterpret_cast<uint4*>(a.stack) + gw * STACK_ENTRIES;
   for (;;) {
     uint32_t g = 0;
     if (lane == 0) g = atomicAdd(a.work, 1u);
     g = __shfl_sync(0xffffffffu, g, 0);
     if ((int64_t)g >= a.ngroups) break;
     const uint32_t first = a.gfirst[g], count = a.gsize[g];
-    // a group wider than 1/16 of the box would break the shared-origin minimum
-    // image: walk its targets one at a time instead
-    const bool has = (uint32_t)(lane & (TPW - 1)) < count;
-    const uint32_t p = first + (has ? (lane & (TPW - 1)) : 0);
-    const uint32_t t0[3] = {a.qx[first], a.qy[first], a.qz[first]};
-    const uint32_t tq[3] = {a.qx[p], a.qy[p], a.qz[p]};
-    bool wide = false;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      int32_t r = rel32(tq[d], t0[d], a.periodic);
-      int32_t mn = __reduce_min_sync(0xffffffffu, has ? r : 0x7FFFFFFF);
-      int32_t mx = __reduce_max_sync(0xffffffffu, has ? r : -0x7FFFFFFF);
-      wide = wide || ((int64_t)mx - (int64_t)mn > WIDE_GROUP);
-    }
-    wide = wide || a.single_target;
-    // one call site: the group at once, or its targets one at a time
-    const uint32_t walks = wide ? count : 1u;
-    for (uint32_t t = 0; t < walks; ++t)
-      walk_targets<TPW, ACC>(a, wide ? first + t : first, wide ? 1u : count, list_l, list_m, owner, stk, rpos, rmask, s0,
-                             s1, tfs, gbox);
+    if constexpr (KERNEL == K_ACC)
+      walk_accurate<PERIODIC>(a, first, count, mem.lists, mem.owner, reinterpret_cast<StackEntry*>(stk), mem.rpos,
+                              mem.rmask, mem.s0, mem.s1, mem.tfs, mem.gbox);
+    else
+      walk_parity<PERIODIC, KERNEL>(a, first, count, mem, stk);
   }
 }
 
@@ -838,7 +1210,8 @@ __global__ void k_deferred(WalkArgs a, uint32_t n_items) {
       const float dx = (float)rel32(cq[0], tq[0], a.periodic) * a.u_inv;
       const float dy = (float)rel32(cq[1], tq[1], a.periodic) * a.u_inv;
       const float dz = (float)rel32(cq[2], tq[2], a.periodic) * a.u_inv;
-      const float f = pair_factor(a, fmaf(dx, dx, fmaf(dy, dy, dz * dz)), m);
+      const float r2b = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+      const float f = a.poly ? pair_factor<K_POLY>(a, r2b, m) : pair_factor<K_AS>(a, r2b, m);
       fx = fmaf(dx, f, fx);
       fy = fmaf(dy, f, fy);
       fz = fmaf(dz, f, fz);
@@ -852,91 +1225,99 @@ __global__ void k_deferred(WalkArgs a, uint32_t n_items) {
 
 }  // namespace
 
-// Variants of the walk: the register budget for 5 to 8 resident blocks of 4
-// warps per SM (TPM_WALK_BLOCKS; 7 = 72 registers by default: walk 64.7 ms at
-// 7 blocks, 64.8 at 8 on the 256^3 workload) and 32 or 16 targets per warp
-// (TPM_WALK_TARGETS; with 16, two lanes share each target).
-static int env_choice(const char* name, int dflt, int lo, int hi) {
-  const char* e = getenv(name);
-  const int v = e ? atoi(e) : dflt;
-  return (v >= lo && v <= hi) ? v : dflt;
-}
-static int walk_blocks_variant() {
-  static int v = env_choice("TPM_WALK_BLOCKS", 7, 5, 8);
-  return v;
-}
-int walk_targets_per_warp() {
-  static int v = env_choice("TPM_WALK_TARGETS", 32, 16, 32) == 16 ? 16 : 32;
-  return v;
-}
+// Resident blocks (of 4 warps) per SM, i.e. the register budget: the parity
+// walk takes 96 registers (clustered 256^3: 44.0 ms at 4 blocks, 40.3 at 5, 41.0
+// at 6 with 72 bytes of spills), the accurate one 66 (128^3: 10.7 at 5, 10.4 at
+// 6, 10.3 at 7).
+template <bool PERIODIC, int KERNEL> constexpr int walk_blocks() { return KERNEL == K_ACC ? 7 : 5; }
 
-template <int B, int T, bool ACC>
+template <bool PERIODIC, int KERNEL>
 static int blocks_for() {
-  const size_t smem = walk_smem_per_warp<ACC>() * WALK_WARPS;
-  TPM_CUDA(cudaFuncSetAttribute(k_walk<B, T, ACC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  auto k = k_walk<walk_blocks<PERIODIC, KERNEL>(), PERIODIC, KERNEL>;
+  const size_t smem = sizeof(WarpMem<PERIODIC, KERNEL>) * WALK_WARPS;
+  TPM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int nb = 0;
-  TPM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_walk<B, T, ACC>, WALK_THREADS, smem));
+  TPM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, WALK_THREADS, smem));
   return nb < 1 ? 1 : nb;
 }
 
-// the accurate mode: 5, 6 or 7 (default; 71 registers, no spills: accurate walk 88.6 ms
-// at 6, 85.5 at 7 on the 256^3 workload) blocks per SM (TPM_WALK_BLOCKS_ACC)
-static int walk_blocks_acc_variant() {
-  static int v = env_choice("TPM_WALK_BLOCKS_ACC", 7, 5, 7);
-  return v;
-}
-template <int T>
-static int blocks_t(bool accurate) {
-  if (accurate) {
-    switch (walk_blocks_acc_variant()) {
-      case 5: return blocks_for<5, T, true>();
-      case 6: return blocks_for<6, T, true>();
-      default: return blocks_for<7, T, true>();
-    }
-  }
-  switch (walk_blocks_variant()) {
-    case 5: return blocks_for<5, T, false>();
-    case 7: return blocks_for<7, T, false>();
-    case 6: return blocks_for<6, T, false>();
-    case 8: return blocks_for<8, T, false>();
-    default: return blocks_for<7, T, false>();
-  }
-}
-
-int walk_blocks_per_sm(bool accurate) {
-  return walk_targets_per_warp() == 16 ? blocks_t<16>(accurate) : blocks_t<32>(accurate);
-}
-
-template <int T>
+template <bool PERIODIC, int KERNEL>
 static void launch_t(const WalkArgs& a, int grid, cudaStream_t s) {
-  if (a.accurate) {
-    const size_t smem = walk_smem_per_warp<true>() * WALK_WARPS;
-    switch (walk_blocks_acc_variant()) {
-      case 5: k_walk<5, T, true><<<grid, WALK_THREADS, smem, s>>>(a); break;
-      case 6: k_walk<6, T, true><<<grid, WALK_THREADS, smem, s>>>(a); break;
-      default: k_walk<7, T, true><<<grid, WALK_THREADS, smem, s>>>(a); break;
-    }
-    return;
-  }
-  const size_t smem = walk_smem_per_warp<false>() * WALK_WARPS;
-  switch (walk_blocks_variant()) {
-    case 5: k_walk<5, T, false><<<grid, WALK_THREADS, smem, s>>>(a); break;
-    case 7: k_walk<7, T, false><<<grid, WALK_THREADS, smem, s>>>(a); break;
-    case 6: k_walk<6, T, false><<<grid, WALK_THREADS, smem, s>>>(a); break;
-    case 8: k_walk<8, T, false><<<grid, WALK_THREADS, smem, s>>>(a); break;
-    default: k_walk<7, T, false><<<grid, WALK_THREADS, smem, s>>>(a); break;
-  }
+  const size_t smem = sizeof(WarpMem<PERIODIC, KERNEL>) * WALK_WARPS;
+  k_walk<walk_blocks<PERIODIC, KERNEL>(), PERIODIC, KERNEL><<<grid, WALK_THREADS, smem, s>>>(a);
 }
 
-int walk_threads() { return WALK_THREADS; }
+// The kernel of a handle, by its walk and pair term; also sizes its grid.
+template <class F>
+static void with_kernel(bool periodic, bool accurate, bool poly, F&& f) {
+  using P = std::true_type;
+  using A = std::false_type;
+  if (accurate) periodic ? f(P{}, std::integral_constant<int, K_ACC>{}) : f(A{}, std::integral_constant<int, K_ACC>{});
+  else if (poly) periodic ? f(P{}, std::integral_constant<int, K_POLY>{}) : f(A{}, std::integral_constant<int, K_POLY>{});
+  else periodic ? f(P{}, std::integral_constant<int, K_AS>{}) : f(A{}, std::integral_constant<int, K_AS>{});
+}
+
+// Targets per walk group: 32 fill a warp, but a small box then leaves most of
+// the chip idle, and smaller groups share each target between lanes.  The
+// largest power of two that still makes about 1,700 groups (of ~2,960 resident
+// warps) was the fastest: walk ms at 32 / 16 / 8 / 4 / 2 / 1 targets for 4,096
+// particles .173 .123 .108 .085 .073 .082; 8,000: .218 .160 .132 .110 .134
+// .136; 13,824: .254 .181 .144 .173 .196 .244; 32,768: .356 .224 .255 .306
+// .419 .574; 110,592: .452 .467 .601 .834 1.18 1.65.
+int walk_group_size(int64_t n) {
+  int size = WALK_TARGETS;
+  while (size > 1 && n < (int64_t)size * 1700) size >>= 1;
+  return size;
+}
+
+int walk_blocks_per_sm(bool periodic, bool accurate, bool poly) {
+  int nb = 1;
+  with_kernel(periodic, accurate, poly,
+              [&](auto p, auto k) { nb = blocks_for<decltype(p)::value, decltype(k)::value>(); });
+  return nb;
+}
+
+// Interpolation at the Chebyshev nodes of [0, x_max] of log2 of the A&S
+// 7.1.26 erfc, as coefficients of powers of r = x / cx.  On x_max <= 3.6 (a cut
+// of 5 r_s is x = 3.54) the polynomial stays within 2e-8 of that function,
+// relative, and its FP32 evaluation within 7e-8 absolute (the A&S form itself
+// in FP32: 3.9e-7), so the walk takes one reciprocal less per pair; longer
+// cuts keep the A&S form.
+bool erfc_poly(double x_max, double cx, float* coef) {
+  if (!(x_max <= 3.6)) return false;
+  constexpr int N = POLY_DEGREE + 1;
+  double node[N], div[N];
+  for (int i = 0; i < N; ++i) {
+    const double x = 0.5 * x_max * (1.0 - std::cos(M_PI * (i + 0.5) / N));
+    const double t = 1.0 / (1.0 + 0.3275911 * x);
+    const double p = t * (0.254829592 + t * (-0.284496736 + t * (1.421413741 + t * (-1.453152027 + t * 1.061405429))));
+    node[i] = x;
+    div[i] = std::log2(p) - x * x / std::log(2.0);
+  }
+  for (int k = 1; k < N; ++k)  // Newton's divided differences
+    for (int i = N - 1; i >= k; --i) div[i] = (div[i] - div[i - 1]) / (node[i] - node[i - k]);
+  double c[N] = {0.0};
+  c[0] = div[N - 1];
+  for (int k = N - 2; k >= 0; --k) {  // c <- c (x - node[k]) + div[k]
+    for (int i = N - 1; i > 0; --i) c[i] = c[i - 1] - node[k] * c[i];
+    c[0] = div[k] - node[k] * c[0];
+  }
+  double scale = 1.0;
+  for (int i = 0; i < N; ++i) {
+    coef[i] = (float)(c[i] * scale);
+    scale *= cx;
+  }
+  return true;
+}
+
 size_t walk_stack_words(int grid, int stack_cap) {
   (void)stack_cap;
   return (size_t)grid * WALK_WARPS * STACK_ENTRIES * 4;  // one 16-byte entry = 4 words
 }
 
 void launch_walk(const WalkArgs& a, int grid, cudaStream_t s) {
-  if (walk_targets_per_warp() == 16) launch_t<16>(a, grid, s);
-  else launch_t<32>(a, grid, s);
+  with_kernel(a.periodic != 0, a.accurate != 0, a.poly != 0,
+              [&](auto p, auto k) { launch_t<decltype(p)::value, decltype(k)::value>(a, grid, s); });
   TPM_LAUNCH_CHECK();
 }
 

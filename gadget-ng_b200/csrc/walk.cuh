@@ -7,6 +7,11 @@
 
 namespace tpm {
 
+constexpr int POLY_DEGREE = 10;
+// Coefficients (powers of r in walk units, x = cx r) of P with erfc(x) =
+// 2^P(r) on [0, x_max]; false when x_max is beyond the fitted range.
+bool erfc_poly(double x_max, double cx, float* coef);
+
 struct WalkArgs {
   int64_t n, n_int;
   // particles, sorted order
@@ -35,10 +40,16 @@ struct WalkArgs {
   float box_u;    // box side in walk units (2^32 quanta)
   float h0_u;     // root half side in u
   float rc2_lo, rc2_hi;    // per-target ambiguity band around r_cut^2 (u^2): node refinement
+  float rc2_mid, rc2_band; // its middle, and half its width (rounded up)
   float prc2_lo, prc2_hi;  // the pair loop's (narrower) band: leaf pairs and monopoles
-  uint32_t prc2_lo_bits, pband_bits;  // the pair band as float bit patterns: (lo, lo + band]
+  float prc2_mid, pband;   // its middle, and half its width (rounded up)
   float grc2_lo, grc2_hi;  // group-level band
   float eps2_u;
+  unsigned long long eps2_2;  // two floats: max(eps^2, 1e-30) in u^2 (no quantum squared is as small)
+  int poly;       // erfc as 2^P(r): P's coefficients, each as two floats
+  unsigned long long poly2[POLY_DEGREE + 1];
+  float h_term;   // parity: cull half side of the monopoles (all at the terminal depth)
+  int term_depth; // the first depth whose half side is below 0.1 r_cut
   float pcx;      // 0.3275911 * scale*2^U / (sqrt(2) r_s)
   float ex2k;     // -(scale*2^U / (sqrt(2) r_s))^2 * log2(e)
   float tiny_u;   // (4 quanta)^2 in u^2
@@ -60,15 +71,14 @@ struct WalkArgs {
   uint32_t cap_deferred;
   uint32_t* stack;
   int stack_cap;
-  int single_target;     // walk every target alone (r_cut above a quarter box)
   uint32_t* pcounts;     // per target (sorted order): leaf pairs, monopoles
   const uint8_t* only;   // nullptr, or: walk only the targets p with only[p] != 0
   int img_depth;         // periodic: nodes shallower than this need the +-L images in the group cull
 };
 
-int walk_blocks_per_sm(bool accurate);
-int walk_targets_per_warp();
-int walk_threads();
+constexpr int WALK_TARGETS = 32;  // targets per warp at most
+int walk_group_size(int64_t n);   // targets per walk group in a box of n particles
+int walk_blocks_per_sm(bool periodic, bool accurate, bool poly);
 size_t walk_stack_words(int grid, int stack_cap);
 void launch_walk(const WalkArgs& a, int grid, cudaStream_t s);
 void launch_deferred(const WalkArgs& a, uint32_t n_items, cudaStream_t s);

@@ -1,0 +1,114 @@
+"""The short-range walk where its dispatch and its packed loops can go wrong:
+particle counts around the group sizes, lists of odd length, groups split at
+cells, periodic images inside a group's reach, a cut beyond the fitted erfc
+polynomial, a root that is a monopole itself.
+
+The interaction set must equal the oracle's particle by particle; the
+short-range forces agree within 1e-5 of their rms (FP32 pair terms: 24-bit
+positions relative to a group of a quarter box at most, 2.8 r_cut, and the
+erfc polynomial's 7e-8, summed over hundreds of pairs).
+"""
+import numpy as np
+import pytest
+
+from conftest import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _positions(kind, n, box, seed):
+    """float64 positions on the device's fixed-point lattice."""
+    rng = np.random.default_rng(seed)
+    if kind == "uniform":
+        x = rng.uniform(0.0, box, (n, 3))
+    elif kind == "lattice":
+        side = int(np.ceil(n ** (1.0 / 3.0)))
+        g = (np.indices((side,) * 3).reshape(3, -1).T + 0.5) * (box / side)
+        x = g[:n] + rng.normal(0.0, 0.3 * box / side, (n, 3))
+    elif kind == "clump":  # everything inside one terminal cell, across the corner of the box
+        x = rng.normal(0.0, 2e-4 * box, (n, 3))
+    else:  # two dense clumps on a sparse background
+        x = rng.uniform(0.0, box, (n, 3))
+        k = n // 3
+        x[:k] = 0.27 * box + rng.normal(0.0, 4e-3 * box, (k, 3))
+        x[k:2 * k] = 0.97 * box + rng.normal(0.0, 2e-2 * box, (k, 3))
+    q = np.floor(np.mod(x / box, 1.0) * 2.0 ** 32).astype(np.uint64) & np.uint64(0xFFFFFFFF)
+    return q.astype(np.float64) * (box / 2.0 ** 32)
+
+
+CASES = [
+    # kind, n, mesh, r_split cells, r_cut factor, periodic
+    ("uniform", 2, 32, 1.25, 4.5, True),
+    ("uniform", 3, 32, 2.5, 5.0, True),
+    ("uniform", 33, 16, 1.25, 4.5, True),
+    ("uniform", 500, 16, 2.5, 6.0, True),  # r_cut close to the box: targets alone, the A&S erfc
+    ("uniform", 1000, 32, 2.5, 5.0, True),  # r_cut above a fifth of the box
+    ("uniform", 3399, 32, 1.25, 4.5, True),  # one target per group
+    ("uniform", 3401, 32, 1.25, 4.5, True),  # two
+    ("lattice", 13599, 32, 1.25, 4.5, True),
+    ("lattice", 13601, 32, 1.25, 6.0, True),  # the A&S erfc with groups
+    ("lattice", 27201, 32, 1.25, 4.5, True),  # groups of a quarter box: images inside their reach
+    ("lattice", 54401, 64, 2.5, 5.0, True),
+    ("clumps", 30000, 64, 1.25, 4.5, True),
+    ("clumps", 60000, 128, 1.25, 5.0, True),
+    ("clump", 400, 16, 1.25, 4.5, True),  # the root is terminal
+    ("lattice", 13824, 32, 1.25, 4.5, False),
+    ("lattice", 29791, 32, 1.25, 6.0, False),
+    ("lattice", 59319, 64, 2.5, 5.0, False),
+]
+
+
+@pytest.mark.parametrize("kind,n,mesh,cells,factor,periodic", CASES)
+def test_interactions_and_forces_match_the_oracle(kind, n, mesh, cells, factor, periodic):
+    import treepm
+    box = 50.0
+    pos = _positions(kind, n, box, n + mesh)
+    mass = np.random.default_rng(n).uniform(0.5, 1.5, n) / n
+    r_split = cells * box / mesh
+    eps2, g = (box / max(n, 8) ** (1.0 / 3.0) / 30.0) ** 2, 1.7
+    s = treepm.TreePmSolver(mesh, box, r_split, r_cut_factor=factor, periodic_walk=periodic)
+    s.set_particles(pos, mass)
+    s.compute_forces(eps2, g)
+    _, sr = s.force_parts(n)
+    counts = s.interaction_counts(n)
+    stats = s.stats()
+    s.close()
+    ref, ref_counts = oracle().short_range(pos, mass, eps2, g, r_split, factor * r_split, box, periodic=periodic,
+                                           counts=True)
+    assert np.array_equal(counts, ref_counts)
+    assert stats["leaf_pairs"] + stats["monopoles"] == int(ref_counts.sum())
+    scale = np.sqrt(np.mean(np.sum(ref ** 2, axis=1)))
+    if scale > 0.0:
+        assert np.sqrt(np.mean(np.sum((sr - ref) ** 2, axis=1))) < 1e-5 * scale
+    else:
+        assert not sr.any()
+
+
+@pytest.mark.parametrize("n,periodic", [(31, True), (700, True), (2100, True), (700, False)])
+def test_accurate_mode_sums_the_complete_kernel(n, periodic):
+    """A small opening angle leaves (nearly) only particle pairs: the direct
+    sum of the complete split kernel inside r_cut."""
+    import treepm
+    from scipy.special import erfc
+    box, mesh = 50.0, 32
+    pos = _positions("uniform", n, box, n)
+    mass = np.full(n, 1.0 / n)
+    r_split, factor, eps2 = 1.25 * box / mesh, 4.5, 1e-3
+    s = treepm.TreePmSolver(mesh, box, r_split, r_cut_factor=factor, periodic_walk=periodic, accurate=True, theta=0.01)
+    s.set_particles(pos, mass)
+    s.compute_forces(eps2, 1.0)
+    _, sr = s.force_parts(n)
+    s.close()
+    d = pos[None] - pos[:, None]
+    if periodic:
+        d -= box * np.round(d / box)
+    r2 = np.sum(d * d, axis=2)
+    x = np.sqrt(r2 + eps2) / (np.sqrt(2.0) * r_split)
+    w = (erfc(x) + 2.0 / np.sqrt(np.pi) * x * np.exp(-x * x)) / (r2 + eps2) ** 1.5
+    w[(r2 > (factor * r_split) ** 2) & np.array(periodic)] = 0.0
+    np.fill_diagonal(w, 0.0)
+    ref = np.einsum("ijk,ij->ik", d, w) / n
+    # the aperiodic walk cuts leaves on the gap to their cell: terms between
+    # r_cut and r_cut + sqrt(3) cells stay, all below w(4.5 r_s) ~ 1e-3 of a pair at r_s
+    tol = 1e-5 if periodic else 2e-3
+    assert np.linalg.norm(sr - ref) < tol * np.linalg.norm(ref)
