@@ -730,7 +730,7 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
       a.cellq = T.o_cell;
       a.rel_k = (float)(h->cfg.err_tol_force_acc * u * u * u);
       if (a.accurate) {  // no reference decisions to reproduce: no float64 band, no COM-on-target opening
-        a.rc2_lo = a.rc2_hi = (float)rc2_u;
+        a.rc2_lo = a.rc2_hi = a.rc2_mid = (float)rc2_u;
         a.prc2_lo = a.prc2_hi = a.prc2_mid = a.rc2_lo;
         a.tiny_u = -1.f;
       }

@@ -33,7 +33,10 @@
 // took two entries per iteration in f32x2 arithmetic (63 instructions for
 // two entries, ~106 before) and the traversal was split into open and item
 // steps; 5.93e9 take 7.1 ms at 73 % after (62.7 -> 40.3 ms on the clustered
-// 256^3 box).  About half are the pair loop, its FMA pipe 56 % busy.
+// 256^3 box).  Two thirds are the pair loop (60 per iteration), its FMA pipe
+// 56 % busy.  The accurate mode took the same steps later: 10.3 -> 7.4 ms on the
+// clustered 128^3 box against its former traversal (32 children of a popped
+// batch per step, opening tests at pop time).
 #include <cmath>
 #include <type_traits>
 
@@ -47,8 +50,7 @@ namespace {
 constexpr int WALK_WARPS = 4;
 constexpr int WALK_THREADS = WALK_WARPS * 32;
 constexpr int CHUNK_L = 64;  // leaf-list capacity (walk 72.9 -> 72.5 ms at 256^3 against 48; 32 is slower)
-// monopole-list capacity: the accurate mode also emits monopoles at pop time
-template <bool ACC> constexpr int chunk_m() { return ACC ? 96 : 64; }
+constexpr int CHUNK_M = 64;  // monopole-list capacity
 
 
 // An interaction list in shared memory, kept in pairs of entries so that the
@@ -442,7 +444,7 @@ __device__ __forceinline__ Sums eval(const WalkArgs& a, const L& list, int n, ui
 template <bool PERIODIC, int KERNEL> struct Lists {
   static constexpr bool ACC = KERNEL == K_ACC;
   List<CHUNK_L, !PERIODIC> leaf;
-  List<chunk_m<ACC>(), ACC || !PERIODIC> mono;
+  List<CHUNK_M, ACC || !PERIODIC> mono;
 };
 template <bool PERIODIC, int KERNEL>
 __device__ __forceinline__ void flush(const WalkArgs& a, const Lists<PERIODIC, KERNEL>& lists, int nll, int nlm,
@@ -464,16 +466,7 @@ __device__ __forceinline__ void flush(const WalkArgs& a, const Lists<PERIODIC, K
                          __uint_as_float(__float_as_uint(B.w) + m.n));
 }
 
-// Stack entry of an open node: its children's record range, mask of the
-// targets that see it (refined per target before the push), and the octree id.
-struct __align__(16) StackEntry {
-  uint32_t first;  // record index of the first child
-  uint32_t info;   // the node's record info | INFO_MAC when its opening angle is undecided for the group
-  uint32_t mask;
-  uint32_t ref;    // octree node id
-};
 constexpr int STACK_ENTRIES = 1024;  // global, per warp
-constexpr uint32_t INFO_MAC = 0x40000000u;  // opening angle undecided for the group
 
 // End of a group's walk: fold the pair-phase lanes of each target, write its
 // acceleration and interaction counts, add to the statistics.
@@ -522,69 +515,99 @@ __device__ __forceinline__ void store_sums(const WalkArgs& a, uint32_t p, bool h
 
 // Shared memory of one warp.
 template <bool PERIODIC, int KERNEL> struct __align__(16) WarpMem {
+  static constexpr bool ACC = KERNEL == K_ACC;
   Lists<PERIODIC, KERNEL> lists;
-  union {
-    struct {  // accurate: staged undecided nodes: position, half side; mask, node, image flag
-      float4 rpos[32];
-      uint4 rmask[32];
-    };
-    struct {  // parity: staged undecided nodes (half side in place of the mass), the targets that see them
-      List<32, false> nodes;
-      uint2 seen[16];
-    };
-  };
-  float4 s0[32], s1[32];  // the lanes' running sums
-  float4 tfs[32];   // target positions
-  float4 gbox[4];   // group box (accurate: corners; parity: half widths) and origin
-  uint4 queue[40];  // parity: nodes whose terminal children wait {first record, count, mask}
-  uint8_t owner[32];  // accurate: child owners of a popped batch
+  // undecided nodes of an open step (their cull half side in place of the
+  // mass; accurate: their half side as well), the targets that go on to their
+  // children and (accurate) those that take them as monopoles
+  List<32, ACC> nodes;
+  uint32_t seen[32];
+  uint32_t taken[ACC ? 32 : 4];
+  float4 cells[ACC ? 32 : 1];  // relative criterion: cell centre, |Q|_F / M of the undecided nodes
+  float4 s0[32], s1[32];       // the lanes' running sums
+  float4 tfs[32];              // target positions
+  float4 gbox[2];              // half widths of the group box, the origin
+  uint4 queue[40];             // nodes whose terminal children wait {first record, count, mask}
 };
 
-// The staged undecided nodes of an open step again (rare: a node seen at
-// another periodic image, marked in its node word, or a target inside the band
-// around r_cut^2), with the nearest image per target and the reference's
-// float64 test inside the band.
-__device__ __noinline__ uint32_t refine_exact(const WalkArgs& a, const List<32, false>& nodes, int n, uint32_t p,
-                                              float4 T, uint2* seen) {
+// The opening decision of the accurate mode for a target at distance^2 d2 from
+// the centre of mass of a node of half side h: the opening angle s/d < theta,
+// s = 2 h (octree.rs:763-809).
+__device__ __forceinline__ bool accept_angle(const WalkArgs& a, float h, float d2) {
+  return 4.f * h * h < a.theta2 * d2;
+}
+// Relative criterion (octree.rs:769-796), qm = |Q|_F / M: the truncation
+// estimate |Q|_F (d^2 + eps^2) < k M d^5 (the caller checks that the target is
+// outside the node's cell).
+__device__ __forceinline__ bool accept_relative(const WalkArgs& a, float qm, float d2, float margin) {
+  return d2 > 0.f && qm * (d2 + a.eps2_u) < a.rel_k * (d2 * d2 * sqrtf(d2)) * margin;
+}
+
+// The staged undecided nodes of an open step, one at a time: where a node is
+// seen at another periodic image by part of the group (marked in its node
+// word), a target lies inside the band around r_cut^2 (parity: the reference's
+// float64 test decides), or the relative criterion opens nodes.
+template <bool PERIODIC, int KERNEL>
+__device__ __noinline__ uint32_t refine_slow(const WalkArgs& a, WarpMem<PERIODIC, KERNEL>& mem, int n, uint32_t p,
+                                             float4 T) {
+  constexpr bool ACC = KERNEL == K_ACC;
   const int lane = threadIdx.x & 31;
   uint32_t nexact = 0;
   for (int j = 0; j < n; ++j) {
-    const float* w = nodes.word(j);
+    const float* w = mem.nodes.word(j);
     const uint32_t node = __float_as_uint(w[10]);
     float dx = w[0] - T.x, dy = w[2] - T.y, dz = w[4] - T.z;
-    if (node & LEAF_BIT) {
+    if (PERIODIC && (node & LEAF_BIT)) {
       dx -= a.box_u * rintf(dx / a.box_u);
       dy -= a.box_u * rintf(dy / a.box_u);
       dz -= a.box_u * rintf(dz / a.box_u);
     }
     const float s = cut_s<CUT_OWN_HALF>(dx, dy, dz, 0.f, w[6]);
     const bool in = (__float_as_uint(w[8]) >> lane) & 1u;
-    bool pass = in && s <= a.rc2_lo;
-    if (in && !pass && s <= a.rc2_hi) {
+    bool pass = in && s <= a.rc2_lo, take = false;
+    if (!ACC && in && !pass && s <= a.rc2_hi) {
       pass = exact_open_pass(a, p, node & ~LEAF_BIT);
       ++nexact;
     }
-    const uint32_t nm = __ballot_sync(0xffffffffu, pass);
-    if (lane == 0) reinterpret_cast<uint32_t*>(seen)[j] = nm;
+    if (ACC && pass) {
+      const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz)), h = fabsf(w[12]);
+      if (!a.relative) {
+        take = accept_angle(a, h, d2);
+      } else if (w[12] > 0.f) {  // (nodes of the top levels are always opened)
+        // point_in_node_cell with a margin: a target on the cell's face opens the node
+        const float4 C = mem.cells[j];
+        float cx = C.x - T.x, cy = C.y - T.y, cz = C.z - T.z;
+        const bool inside = fmaxf(fabsf(cx), fmaxf(fabsf(cy), fabsf(cz))) <= h * 1.0001f;
+        take = !inside && accept_relative(a, C.w, d2, 1.f);
+      }
+    }
+    const uint32_t tm = ACC ? __ballot_sync(0xffffffffu, take) : 0u;
+    const uint32_t nm = __ballot_sync(0xffffffffu, pass) & ~tm;
+    if (lane == 0) {
+      mem.seen[j] = nm;
+      if (ACC) mem.taken[j] = tm;
+    }
   }
   return nexact;
 }
 
-// Parity walk of targets [first, first + count) (count <= 32) with one warp.
+// Walk of targets [first, first + count) (count <= 32) with one warp.
 //
 // An octree node's children are stored internal nodes first, leaves after
-// them, and internal nodes become monopoles at one depth for the whole tree.
-// So a node that stays open splits into a range of open children and a range
-// of terminal ones, and the walk has two kinds of step, each on four nodes at a
-// time with eight lanes per node (a node has at most eight children, so no
-// lane has to look up its child): an open step classifies open children
-// against the group box, tests the undecided ones per target and pushes what
-// is seen; an item step cuts terminal children against the group box and
-// appends them to the lists.  The item step, which meets most of the nodes,
-// needs neither the periodic images nor the opening test.
+// them.  Parity: internal nodes become monopoles at one depth for the whole
+// tree; accurate: where a target's distance allows it.  So a node that stays
+// open splits into a range of open children and a range of terminal ones, and
+// the walk has two kinds of step, each on four nodes at a time with eight lanes
+// per node (a node has at most eight children, so no lane has to look up its
+// child): an open step classifies open children against the group box, tests
+// the undecided ones per target and pushes what is seen; an item step cuts
+// terminal children against the group box and appends them to the lists.  The
+// item step, which meets most of the nodes, needs neither the periodic images
+// nor the opening test.
 template <bool PERIODIC, int KERNEL>
-__device__ __forceinline__ void walk_parity(const WalkArgs& a, uint32_t first, uint32_t count,
-                                            WarpMem<PERIODIC, KERNEL>& mem, uint4* stk) {
+__device__ __forceinline__ void walk_group(const WalkArgs& a, uint32_t first, uint32_t count,
+                                           WarpMem<PERIODIC, KERNEL>& mem, uint4* stk) {
+  constexpr bool ACC = KERNEL == K_ACC;
   const int lane = threadIdx.x & 31;
   const uint32_t p = first + ((uint32_t)lane < count ? (uint32_t)lane : 0u);
   // targets of this walk: the group's particles, or those of them the caller
@@ -592,6 +615,7 @@ __device__ __forceinline__ void walk_parity(const WalkArgs& a, uint32_t first, u
   const bool has = (uint32_t)lane < count && (!a.only || a.only[p] != 0);
   const uint32_t mask0 = __ballot_sync(0xffffffffu, has);  // bit t: target t
   if (mask0 == 0u) return;
+  const int term_depth = ACC ? 64 : a.term_depth;
   {
     const uint32_t tq[3] = {a.qx[p], a.qy[p], a.qz[p]};
     uint32_t oq[3];
@@ -614,8 +638,7 @@ __device__ __forceinline__ void walk_parity(const WalkArgs& a, uint32_t first, u
       mem.gbox[0] = make_float4(w[0], w[1], w[2], 0.f);
       reinterpret_cast<uint4*>(mem.gbox)[1] = make_uint4(oq[0], oq[1], oq[2], 0u);
       // the root: a terminal node by itself, or an open one
-      const bool item = a.term_depth == 0;
-      if (item) mem.queue[0] = make_uint4(0u, 1u, mask0, 0u);
+      if (term_depth == 0) mem.queue[0] = make_uint4(0u, 1u, mask0, 0u);
       else stk[0] = make_uint4(0u, 1u, mask0, 0u);
     }
   }
@@ -623,7 +646,7 @@ __device__ __forceinline__ void walk_parity(const WalkArgs& a, uint32_t first, u
   mem.s1[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
   const uint32_t lanes = pair_lanes(lane, count);
   uint32_t nexact = 0, neval = 0;
-  int nll = 0, nlm = 0, sp = a.term_depth == 0 ? 0 : 1, nq = 1 - sp;
+  int nll = 0, nlm = 0, sp = term_depth == 0 ? 0 : 1, nq = 1 - sp;
   // each step takes at least one range, and a node makes at most two: the cap
   // turns a malformed tree into an error flag instead of an endless loop
   uint32_t steps_left = (uint32_t)(2 * a.n_int + 4 < 0xFFFFFFFFll ? 2 * a.n_int + 4 : 0xFFFFFFFFll);
@@ -631,6 +654,21 @@ __device__ __forceinline__ void walk_parity(const WalkArgs& a, uint32_t first, u
   __syncwarp();
   const int slot = lane >> 3, child = lane & 7;
   for (;;) {
+    // a step adds up to 32 entries to either list (one call site of the list
+    // evaluation, the last flush included)
+    const bool done = sp == 0 && nq == 0;
+    if (done || nll > CHUNK_L - 32 || nlm > CHUNK_M - 32) {
+      if (lane == 0) {
+        mem.lists.leaf.close(nll);
+        mem.lists.mono.close(nlm);
+      }
+      __syncwarp();
+      flush<PERIODIC, KERNEL>(a, mem.lists, nll, nlm, lane, lanes, first, mem.tfs, mem.s0, mem.s1, nexact, neval);
+      __syncwarp();
+      nll = 0;
+      nlm = 0;
+      if (done) break;
+    }
     if (steps_left-- == 0u) {
       if (lane == 0) atomicOr(a.err, DEV_ERR_STACK);
       break;
@@ -649,7 +687,7 @@ __device__ __forceinline__ void walk_parity(const WalkArgs& a, uint32_t first, u
         r0 = __ldg(rec);
         r1 = __ldg(rec + 1);
       }
-      const bool leaf = (r1.y & WN_LEAF) != 0u;
+      const bool leaf = ACC || (r1.y & WN_LEAF) != 0u;
       const float h = !leaf ? a.h_term : (PERIODIC ? 0.f : half_side(a.h0_u, wn_depth(r1.y)));
       const float sx = (float)rel32(r0.x, GO.x, PERIODIC) * a.u_inv, sy = (float)rel32(r0.y, GO.y, PERIODIC) * a.u_inv;
       const float sz = (float)rel32(r0.z, GO.z, PERIODIC) * a.u_inv;
@@ -657,32 +695,23 @@ __device__ __forceinline__ void walk_parity(const WalkArgs& a, uint32_t first, u
       const float gx = fmaxf(fabsf(sx) - (GW.x + h), 0.f), gy = fmaxf(fabsf(sy) - (GW.y + h), 0.f);
       const float gz = fmaxf(fabsf(sz) - (GW.z + h), 0.f);
       keep = keep && !(fmaf(gx, gx, fmaf(gy, gy, gz * gz)) > a.grc2_hi);
-      const uint32_t el = __ballot_sync(0xffffffffu, keep && leaf), em = __ballot_sync(0xffffffffu, keep && !leaf);
+      const uint32_t el = __ballot_sync(0xffffffffu, keep && leaf);
+      const uint32_t em = ACC ? 0u : __ballot_sync(0xffffffffu, keep && !leaf);
       if (keep) {
         // the reference skips the target's own leaf (j != skip)
         const uint32_t own = leaf ? r1.z - first : 32u;
         const uint32_t see = own < count ? (e.z & ~(1u << own)) : e.z;
-        auto& list = leaf ? mem.lists.leaf : mem.lists.mono;  // the same layout
-        list.put(leaf ? nll + __popc(el & below) : nlm + __popc(em & below), sx, sy, sz, __uint_as_float(r0.w), h, see,
-                 leaf ? r1.z | LEAF_BIT : r1.z);
+        if constexpr (ACC) {
+          mem.lists.leaf.put(nll + __popc(el & below), sx, sy, sz, __uint_as_float(r0.w), h, see, r1.z | LEAF_BIT);
+        } else {
+          auto& list = leaf ? mem.lists.leaf : mem.lists.mono;  // the same layout
+          list.put(leaf ? nll + __popc(el & below) : nlm + __popc(em & below), sx, sy, sz, __uint_as_float(r0.w), h,
+                   see, leaf ? r1.z | LEAF_BIT : r1.z);
+        }
       }
       nll += __popc(el);
       nlm += __popc(em);
-      const bool done = sp == 0 && nq == 0;
-      // the next item step adds up to 32 entries to either list (one call site
-      // of the list evaluation, the last flush included)
-      if (done || nll > CHUNK_L - 32 || nlm > chunk_m<false>() - 32) {
-        if (lane == 0) {
-          mem.lists.leaf.close(nll);
-          mem.lists.mono.close(nlm);
-        }
-        __syncwarp();
-        flush<PERIODIC, KERNEL>(a, mem.lists, nll, nlm, lane, lanes, first, mem.tfs, mem.s0, mem.s1, nexact, neval);
-        __syncwarp();
-        nll = 0;
-        nlm = 0;
-      }
-      if (done) break;
+      __syncwarp();
       continue;
     }
     // ---- open step
@@ -698,7 +727,10 @@ __device__ __forceinline__ void walk_parity(const WalkArgs& a, uint32_t first, u
       r1 = __ldg(rec + 1);
     }
     const int dep = wn_depth(r1.y);
-    const float h = half_side(a.h0_u, dep);
+    const float hnode = half_side(a.h0_u, dep);
+    // cull half side: the COM-centred AABB's, or (accurate) twice that, which
+    // holds the whole cell
+    const float h = ACC ? 2.f * hnode : hnode;
     const float sx = (float)rel32(r0.x, GO.x, PERIODIC) * a.u_inv, sy = (float)rel32(r0.y, GO.y, PERIODIC) * a.u_inv;
     const float sz = (float)rel32(r0.z, GO.z, PERIODIC) * a.u_inv;
     const float ux = fabsf(sx), uy = fabsf(sy), uz = fabsf(sz);
@@ -709,12 +741,44 @@ __device__ __forceinline__ void walk_parity(const WalkArgs& a, uint32_t first, u
     // the per-target test, if they are wide enough for that image to come
     // within r_cut.  The others: seen by the whole group, or undecided.
     const float half_box = 0.5f * a.box_u;
-    const bool image = PERIODIC && live && dep < a.img_depth &&
-                       (ux + GW.x > half_box || uy + GW.y > half_box || uz + GW.z > half_box);
+    const bool top = PERIODIC && dep < a.img_depth;
+    const bool image = top && live && (ux + GW.x > half_box || uy + GW.y > half_box || uz + GW.z > half_box);
     bool keep = live && (image || !(fmaf(gx, gx, fmaf(gy, gy, gz * gz)) > a.grc2_hi));
-    const bool ambig = keep && (image || !(fmaf(fx, fx, fmaf(fy, fy, fz * fz)) < a.grc2_lo));
+    bool ambig = keep && (image || !(fmaf(fx, fx, fmaf(fy, fy, fz * fz)) < a.grc2_lo));
+    uint32_t see = e.z, take = 0u;  // targets that open the node, that take it as a monopole
+    float4 cell = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (ACC && keep && !image) {
+      // opening test for the whole group by its nearest and farthest distances
+      // from the centre of mass (both criteria are monotone in it), with a
+      // margin that leaves the float-rounding cases to the per-target test
+      const float nx = fmaxf(ux - GW.x, 0.f), ny = fmaxf(uy - GW.y, 0.f), nz = fmaxf(uz - GW.z, 0.f);
+      const float ox = ux + GW.x, oy = uy + GW.y, oz = uz + GW.z;
+      const float dmin2 = fmaf(nx, nx, fmaf(ny, ny, nz * nz)), dmax2 = fmaf(ox, ox, fmaf(oy, oy, oz * oz));
+      bool all, none;
+      if (a.relative) {
+        // the target must be outside the node's cell: a group box touching the
+        // cell leaves the node to the per-target test
+        const uint4 cc = __ldg(&a.cellq[r1.z]);
+        cell = make_float4((float)rel32(cc.x, GO.x, PERIODIC) * a.u_inv, (float)rel32(cc.y, GO.y, PERIODIC) * a.u_inv,
+                           (float)rel32(cc.z, GO.z, PERIODIC) * a.u_inv, __uint_as_float(cc.w) / __uint_as_float(r0.w));
+        const float hc = hnode * 1.0001f;
+        const bool touch = fabsf(cell.x) <= GW.x + hc && fabsf(cell.y) <= GW.y + hc && fabsf(cell.z) <= GW.z + hc;
+        const bool inside = fabsf(cell.x) + GW.x <= hc && fabsf(cell.y) + GW.y <= hc && fabsf(cell.z) + GW.z <= hc;
+        none = top || inside || !accept_relative(a, cell.w, dmax2, 1.001f);
+        all = !none && !touch && accept_relative(a, cell.w, dmin2, 0.999f);
+      } else {
+        all = accept_angle(a, hnode, dmin2 * 0.999f);
+        none = !accept_angle(a, hnode, dmax2 * 1.001f);
+      }
+      if (all) {  // the pair loop cuts it per target
+        take = e.z;
+        see = 0u;
+        ambig = false;
+      } else {
+        ambig = ambig || !none;
+      }
+    }
     const uint32_t amb = __ballot_sync(0xffffffffu, ambig);
-    uint32_t see = e.z;
     if (amb != 0u) {
       // Per-target refinement: each undecided node is staged once in shared
       // memory, then tested against all targets (one per lane), two nodes at a
@@ -722,38 +786,63 @@ __device__ __forceinline__ void walk_parity(const WalkArgs& a, uint32_t first, u
       // the exact minimum-image difference by ~1e-7 of r_cut, far inside the
       // band around r_cut^2 that goes to the float64 test.
       const int mine = __popc(amb & below), namb = __popc(amb);
-      if (ambig) mem.nodes.put(mine, sx, sy, sz, h, 0.f, e.z, image ? r1.z | LEAF_BIT : r1.z);
+      if (ambig) {
+        mem.nodes.put(mine, sx, sy, sz, h, top ? -hnode : hnode, e.z, image ? r1.z | LEAF_BIT : r1.z);
+        if (ACC && a.relative) mem.cells[mine] = cell;
+      }
       if (lane == 0) mem.nodes.close(namb);
-      const bool images = __any_sync(0xffffffffu, image);
+      bool slow = __any_sync(0xffffffffu, image) || (ACC && a.relative);
       __syncwarp();
       const float4 TF = mem.tfs[lane];
-      const f32x2 ntx = pack2(-TF.x, -TF.x), nty = pack2(-TF.y, -TF.y), ntz = pack2(-TF.z, -TF.z);
-      const uint32_t tbit = 1u << lane;
-      float edge = 1e30f;
-      const f32x2 nmid = pack2(-a.rc2_mid, -a.rc2_mid);
-      for (int j = 0; j < namb; j += 2) {
-        auto& nd = mem.nodes.pair[j >> 1];
-        const float4 A = nd.xy, B = nd.zm;
-        const uint2 M = nd.mask;
-        const float2 x = unpack2(add2(pack2(A.x, A.y), ntx)), y = unpack2(add2(pack2(A.z, A.w), nty));
-        const float2 z = unpack2(add2(pack2(B.x, B.y), ntz));
-        const f32x2 ex = pack2(fmaxf(fabsf(x.x) - B.z, 0.f), fmaxf(fabsf(x.y) - B.w, 0.f));
-        const f32x2 ey = pack2(fmaxf(fabsf(y.x) - B.z, 0.f), fmaxf(fabsf(y.y) - B.w, 0.f));
-        const f32x2 ez = pack2(fmaxf(fabsf(z.x) - B.z, 0.f), fmaxf(fabsf(z.y) - B.w, 0.f));
-        const float2 q = unpack2(add2(fma2(ez, ez, fma2(ey, ey, mul2(ex, ex))), nmid));
-        edge = min3_abs(edge, q.x, q.y);
-        const uint32_t n0 = __ballot_sync(0xffffffffu, (M.x & tbit) && q.x <= 0.f);
-        const uint32_t n1 = __ballot_sync(0xffffffffu, (M.y & tbit) && q.y <= 0.f);
-        if (lane == 0) mem.seen[j >> 1] = make_uint2(n0, n1);
+      if (!slow) {
+        const f32x2 ntx = pack2(-TF.x, -TF.x), nty = pack2(-TF.y, -TF.y), ntz = pack2(-TF.z, -TF.z);
+        const uint32_t tbit = 1u << lane;
+        float edge = 1e30f;
+        const f32x2 nmid = pack2(-a.rc2_mid, -a.rc2_mid);
+        for (int j = 0; j < namb; j += 2) {
+          auto& nd = mem.nodes.pair[j >> 1];
+          const float4 A = nd.xy, B = nd.zm;
+          const uint2 M = nd.mask;
+          const f32x2 dx = add2(pack2(A.x, A.y), ntx), dy = add2(pack2(A.z, A.w), nty);
+          const f32x2 dz = add2(pack2(B.x, B.y), ntz);
+          const float2 x = unpack2(dx), y = unpack2(dy), z = unpack2(dz);
+          const f32x2 ex = pack2(fmaxf(fabsf(x.x) - B.z, 0.f), fmaxf(fabsf(x.y) - B.w, 0.f));
+          const f32x2 ey = pack2(fmaxf(fabsf(y.x) - B.z, 0.f), fmaxf(fabsf(y.y) - B.w, 0.f));
+          const f32x2 ez = pack2(fmaxf(fabsf(z.x) - B.z, 0.f), fmaxf(fabsf(z.y) - B.w, 0.f));
+          const float2 q = unpack2(add2(fma2(ez, ez, fma2(ey, ey, mul2(ex, ex))), nmid));
+          const bool p0 = (M.x & tbit) && q.x <= 0.f, p1 = (M.y & tbit) && q.y <= 0.f;
+          uint32_t n0 = __ballot_sync(0xffffffffu, p0), n1 = __ballot_sync(0xffffffffu, p1);
+          if constexpr (ACC) {
+            const float2 d2 = unpack2(fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)))), hn = nd.h;
+            const uint32_t t0 = __ballot_sync(0xffffffffu, p0 && accept_angle(a, hn.x, d2.x));
+            const uint32_t t1 = __ballot_sync(0xffffffffu, p1 && accept_angle(a, hn.y, d2.y));
+            n0 &= ~t0;
+            n1 &= ~t1;
+            if (lane == 0) *reinterpret_cast<uint2*>(&mem.taken[j]) = make_uint2(t0, t1);
+          } else {
+            edge = min3_abs(edge, q.x, q.y);
+          }
+          if (lane == 0) *reinterpret_cast<uint2*>(&mem.seen[j]) = make_uint2(n0, n1);
+        }
+        if (!ACC) slow = __any_sync(0xffffffffu, edge <= a.rc2_band);
       }
-      if (images || __any_sync(0xffffffffu, edge <= a.rc2_band)) nexact += refine_exact(a, mem.nodes, namb, p, TF, mem.seen);
+      if (slow) nexact += refine_slow<PERIODIC, KERNEL>(a, mem, namb, p, TF);
       __syncwarp();
-      if (ambig) see = reinterpret_cast<const uint32_t*>(mem.seen)[mine];
-      keep = keep && see != 0u;  // a node no target sees is not pushed
+      if (ambig) {
+        see = mem.seen[mine];
+        if (ACC) take = mem.taken[mine];
+      }
     }
+    if constexpr (ACC) {
+      const uint32_t em = __ballot_sync(0xffffffffu, keep && take != 0u);
+      if (keep && take != 0u)
+        mem.lists.mono.put(nlm + __popc(em & below), sx, sy, sz, __uint_as_float(r0.w), h, take, r1.z);
+      nlm += __popc(em);
+    }
+    keep = keep && see != 0u;  // a node no target opens is not pushed
     // the seen nodes' children: internal ones stay open above the terminal
     // depth, the rest are items
-    const uint32_t inner = dep + 1 < a.term_depth ? wn_ninner(r1.y) : 0u, rest = wn_nchild(r1.y) - inner;
+    const uint32_t inner = dep + 1 < term_depth ? wn_ninner(r1.y) : 0u, rest = wn_nchild(r1.y) - inner;
     const uint32_t po = __ballot_sync(0xffffffffu, keep && inner != 0u);
     const uint32_t pi = __ballot_sync(0xffffffffu, keep && rest != 0u);
     if (sp + __popc(po) > STACK_ENTRIES) {
@@ -765,359 +854,9 @@ __device__ __forceinline__ void walk_parity(const WalkArgs& a, uint32_t first, u
     sp += __popc(po);
     nq += __popc(pi);
     __syncwarp();
-    if (sp == 0 && nq == 0 && nll + nlm == 0) break;  // nothing in reach
   }
   __syncwarp();
   store_sums(a, p, has, count, mem.s0[lane], mem.s1[lane], nexact, neval);
-}
-
-// Accurate walk of targets [first, first + count) (count <= 32) with one warp:
-// whether a node is opened depends on its distance from each target.
-template <bool PERIODIC>
-__device__ void walk_accurate(const WalkArgs& a, uint32_t first, uint32_t count, Lists<PERIODIC, K_ACC>& lists,
-                             uint8_t* owner, StackEntry* stk, float4* rpos, uint4* rmask, float4* s0, float4* s1,
-                             float4* tfs, float4* gbox) {
-  const int lane = threadIdx.x & 31;
-  const int tgt = lane;  // this lane's target within the group
-  const uint32_t p = first + ((uint32_t)tgt < count ? (uint32_t)tgt : 0u);
-  // targets of this walk: the group's particles, or those of them the caller
-  // selected (the group box then covers only those)
-  const bool has = (uint32_t)tgt < count && (!a.only || a.only[p] != 0);
-  const uint32_t tq[3] = {a.qx[p], a.qy[p], a.qz[p]};
-  uint32_t oq[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) oq[d] = __shfl_sync(0xffffffffu, tq[d], 0);
-  int32_t tr[3];
-  float tf[3], bmin[3], bmax[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    tr[d] = rel32(tq[d], oq[d], PERIODIC);
-    tf[d] = (float)tr[d] * a.u_inv;
-    int32_t mn = __reduce_min_sync(0xffffffffu, has ? tr[d] : 0x7FFFFFFF);
-    int32_t mx = __reduce_max_sync(0xffffffffu, has ? tr[d] : -0x7FFFFFFF);
-    bmin[d] = (float)mn * a.u_inv;
-    bmax[d] = (float)mx * a.u_inv;
-  }
-  // the group box, its origin and the targets' positions wait in shared
-  // memory (read when a node is classified, refined or flushed): registers
-  // for the traversal
-  tfs[lane] = make_float4(tf[0], tf[1], tf[2], 0.f);
-  if (lane == 0) {
-    gbox[0] = make_float4(bmin[0], bmin[1], bmin[2], 0.f);
-    gbox[1] = make_float4(bmax[0], bmax[1], bmax[2], 0.f);
-    reinterpret_cast<uint4*>(gbox)[2] = make_uint4(oq[0], oq[1], oq[2], 0u);
-  }
-  __syncwarp();
-  const uint32_t mask0 = __ballot_sync(0xffffffffu, has);  // bit t: target t
-  s0[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
-  s1[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
-  uint32_t neval = 0, none = 0;
-  int nll = 0, nlm = 0, sp = 0;
-
-  // the first item is the root record
-  bool have = lane == 0;
-  uint32_t item = 0;
-  uint32_t imask = mask0;
-  // each iteration pops at least one node, so a walk over a well-formed tree
-  // ends within (internal nodes + 1) iterations; the cap turns a malformed
-  // tree into an error flag instead of an endless loop
-  uint32_t iter_left = (uint32_t)(a.n_int + 2 < 0xFFFFFFFFll ? a.n_int + 2 : 0xFFFFFFFFll);
-
-  for (;;) {
-    if (iter_left-- == 0u) {
-      if (lane == 0) atomicOr(a.err, DEV_ERR_STACK);
-      break;
-    }
-    // ---- classify this lane's item against the group box
-    bool emit = false, push = false, ambig = false, is_leaf = false;
-    float4 ent;  // a terminal node: group-relative position, mass
-    float ent_h = 0.f;
-    uint32_t ent_mask = 0u, ent_node = 0u;
-    StackEntry se;
-    float sx = 0.f, sy = 0.f, sz = 0.f, sh = 0.f;  // an undecided open node: group-relative COM, cull half side
-    uint32_t simg = 0u;
-    if (have && imask != 0u) {
-      const uint4 r0 = __ldg(reinterpret_cast<const uint4*>(&a.recs[item]));
-      const uint4 r1 = __ldg(reinterpret_cast<const uint4*>(&a.recs[item]) + 1);
-      const uint32_t info = r1.y;
-      const bool leaf = (info & WN_LEAF) != 0;
-      const int dep = wn_depth(info);
-      const float hnode = half_side(a.h0_u, dep);
-      // cull half side: twice the COM-centred AABB's, which holds the whole cell
-      const float h = leaf ? (PERIODIC ? 0.f : hnode) : 2.f * hnode;
-      const uint32_t cq[3] = {r0.x, r0.y, r0.z};
-      const float4 GL = gbox[0], GH = gbox[1];
-      const uint4 GO = reinterpret_cast<const uint4*>(gbox)[2];
-      const float bmin[3] = {GL.x, GL.y, GL.z}, bmax[3] = {GH.x, GH.y, GH.z};
-      const uint32_t oq[3] = {GO.x, GO.y, GO.z};
-      // Per axis, the targets see the node at the minimum image of S - t for t
-      // in [bmin, bmax]: bound min / max of |wrap(S - t)| over that interval
-      // (images at 0 and +-L), then the AABB gap.
-      float emin2 = 0.f, emax2 = 0.f, dmin2 = 0.f, dmax2 = 0.f;
-      int32_t S[3];
-      float SF[3];
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        S[d] = rel32(cq[d], oq[d], PERIODIC);
-        const float sf = (float)S[d] * a.u_inv;
-        SF[d] = sf;
-        const float lo = sf - bmax[d], hi = sf - bmin[d];
-        float dmin = lo > 0.f ? lo : (hi < 0.f ? -hi : 0.f);
-        float dmax = fmaxf(fabsf(lo), fabsf(hi));
-        // the +-L images can only come within r_cut of a group (no wider than
-        // max_extent) for nodes of half side near L/2: the top levels
-        if (PERIODIC && dep < a.img_depth) {
-          dmin = fminf(dmin, fminf(a.box_u - hi, lo + a.box_u));
-          const float half = 0.5f * a.box_u;
-          if (lo <= -half || hi >= half) dmax = half;
-          else dmax = fminf(dmax, half);
-        }
-        const float gap = fmaxf(dmin - h, 0.f);
-        const float far = fmaxf(dmax - h, 0.f);
-        emin2 = fmaf(gap, gap, emin2);
-        emax2 = fmaf(far, far, emax2);
-        dmin2 = fmaf(dmin, dmin, dmin2);
-        dmax2 = fmaf(dmax, dmax, dmax2);
-      }
-      bool open, macmix = false;
-      if (!leaf) {
-        bool accept_all, open_all;
-        if (a.relative) {
-          // relative criterion (octree.rs:769-796): accept when the target is
-          // outside the node's cell and |Q|_F (d^2 + eps^2) < k M d^5; that
-          // bound falls with d, so the group's nearest and farthest COM
-          // distances decide it for every target, and a group box touching
-          // the cell leaves the node to the per-target test.  Nodes at the
-          // top levels (periodic images) are always opened.
-          const uint4 cc = __ldg(&a.cellq[r1.z]);
-          const float qf = __uint_as_float(cc.w), m = __uint_as_float(r0.w);
-          const uint32_t ccq[3] = {cc.x, cc.y, cc.z};
-          bool touch = true, inside_all = true;
-#pragma unroll
-          for (int d = 0; d < 3; ++d) {
-            const float c = (float)rel32(ccq[d], oq[d], PERIODIC) * a.u_inv;
-            const float lo = c - hnode * 1.0001f, hi = c + hnode * 1.0001f;
-            touch = touch && lo <= bmax[d] && hi >= bmin[d];
-            inside_all = inside_all && lo <= bmin[d] && hi >= bmax[d];
-          }
-          const float dmn = sqrtf(dmin2), dmx = sqrtf(dmax2);
-          accept_all = !touch && dmin2 > 0.f &&
-                       qf * (dmin2 + a.eps2_u) < a.rel_k * m * (dmin2 * dmin2 * dmn) * 0.999f;
-          open_all = (PERIODIC && dep < a.img_depth) || inside_all ||
-                     !(qf * (dmax2 + a.eps2_u) < a.rel_k * m * (dmax2 * dmax2 * dmx) * 1.001f);
-          accept_all = accept_all && !open_all;
-        } else {
-          // opening angle s/d < theta, s = 2 * half side (octree.rs:763-809);
-          // a margin on both sides leaves the float-rounding cases to the
-          // per-target test at pop time
-          const float s2 = 4.f * hnode * hnode;
-          accept_all = s2 < a.theta2 * dmin2 * 0.999f;
-          open_all = s2 >= a.theta2 * dmax2 * 1.001f;
-        }
-        open = !accept_all;
-        macmix = !accept_all && !open_all;
-      } else {
-        open = false;
-      }
-      if (!(emin2 > a.grc2_hi)) {
-        if (open) {
-          push = true;
-          ambig = !(emax2 < a.grc2_lo);
-          se.first = r1.x;
-          se.info = info | (macmix ? INFO_MAC : 0u);
-          se.mask = imask;
-          se.ref = r1.z;
-          if (ambig) {
-            sx = SF[0];
-            sy = SF[1];
-            sz = SF[2];
-            sh = h;
-            simg = (PERIODIC && dep < a.img_depth) ? 1u : 0u;
-          }
-        } else {
-          emit = true;
-          ent = make_float4(SF[0], SF[1], SF[2], __uint_as_float(r0.w));
-          ent_h = h;
-          // the reference skips the target's own leaf (j != skip)
-          const uint32_t own = leaf ? r1.z - first : 32u;
-          ent_mask = own < count ? (imask & ~(1u << own)) : imask;
-          ent_node = leaf ? (r1.z | LEAF_BIT) : r1.z;
-          is_leaf = leaf;
-        }
-      }
-    }
-    // ---- append terminal entries to the leaf and monopole lists
-    const uint32_t eml = __ballot_sync(0xffffffffu, emit && is_leaf);
-    const uint32_t emm = __ballot_sync(0xffffffffu, emit && !is_leaf);
-    if (emit) {
-      const unsigned lt = (1u << lane) - 1u;
-      if (is_leaf) lists.leaf.put(nll + __popc(eml & lt), ent.x, ent.y, ent.z, ent.w, ent_h, ent_mask, ent_node);
-      else lists.mono.put(nlm + __popc(emm & lt), ent.x, ent.y, ent.z, ent.w, ent_h, ent_mask, ent_node);
-    }
-    nll += __popc(eml);
-    nlm += __popc(emm);
-    // ---- per-target refinement of open nodes undecided for the group, before
-    // they are pushed: each node is staged once (group-relative COM, cull half
-    // side) in shared memory, then tested against all targets (one per lane)
-    // from a broadcast load.  dd = COM - target in float differs from the exact
-    // minimum-image difference by ~1e-7 of r_cut, far inside the band that goes
-    // to the float64 test.  A node no target sees is not pushed.
-    const uint32_t below = (1u << lane) - 1u;
-    const uint32_t amb = __ballot_sync(0xffffffffu, push && ambig);
-    if (push && ambig) {
-      const int j = __popc(amb & below);
-      rpos[j] = make_float4(sx, sy, sz, sh);
-      rmask[j] = make_uint4(se.mask, se.ref, simg, 0u);
-    }
-    __syncwarp();
-    const int namb = __popc(amb);
-    const float4 TF = tfs[lane];
-    const float tfl[3] = {TF.x, TF.y, TF.z};
-    for (int j = 0; j < namb; ++j) {
-      const float4 R = rpos[j];
-      const uint4 M = rmask[j];
-      bool pass = false;
-      if (has && ((M.x >> tgt) & 1u)) {
-        const float rc[3] = {R.x, R.y, R.z};
-        float s = 0.f;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          float dd = rc[d] - tfl[d];
-          if (M.z) dd -= a.box_u * rintf(dd / a.box_u);  // top levels: the nearest periodic image
-          const float ee = fmaxf(fabsf(dd) - R.w, 0.f);
-          s = fmaf(ee, ee, s);
-        }
-        if (s <= a.rc2_lo) pass = true;
-      }
-      const uint32_t nm = __ballot_sync(0xffffffffu, pass);
-      if (lane == 0) rmask[j].x = nm;
-    }
-    __syncwarp();
-    if (push && ambig) {
-      se.mask = rmask[__popc(amb & below)].x;
-      push = se.mask != 0u;
-    }
-    // ---- push open nodes
-    const uint32_t pm = __ballot_sync(0xffffffffu, push);
-    if (sp + __popc(pm) > STACK_ENTRIES) {
-      if (lane == 0) atomicOr(a.err, DEV_ERR_STACK);
-      break;
-    }
-    if (push) {
-      const int slot = sp + __popc(pm & ((1u << lane) - 1u));
-      *reinterpret_cast<uint4*>(&stk[slot]) = make_uint4(se.first, se.info, se.mask, se.ref);
-    }
-    sp += __popc(pm);
-    __syncwarp();
-    // before the next check the pop adds up to 32 monopole entries (accurate
-    // mode) and the next classification up to 32 to either list
-    // (one call site of the list evaluation, the last flush included: the
-    // kernel's code stays small enough for the instruction cache)
-    const bool done = sp == 0;
-    if (done || nll > CHUNK_L - 32 || nlm > chunk_m<true>() - 64) {
-      if (nll + nlm > 0) {
-        if (lane == 0) {
-          lists.leaf.close(nll);
-          lists.mono.close(nlm);
-        }
-        __syncwarp();
-        flush<PERIODIC, K_ACC>(a, lists, nll, nlm, lane, pair_lanes(lane, count), first, tfs, s0, s1, none, neval);
-      }
-      __syncwarp();
-      nll = 0;
-      nlm = 0;
-    }
-    if (done) break;
-    // ---- pop a batch whose children fill at most one warp
-    const int avail = sp < 32 ? sp : 32;
-    uint4 e = make_uint4(0u, 0u, 0u, 0u);
-    uint32_t nc = 0;
-    if (lane < avail) {
-      e = *reinterpret_cast<const uint4*>(&stk[sp - 1 - lane]);
-      nc = wn_nchild(e.y);
-    }
-    const uint32_t incl = warp_incl_scan(nc, lane);
-    const uint32_t take = __ballot_sync(0xffffffffu, lane < avail && incl <= 32u);
-    const int k = __popc(take);
-    sp -= k;
-    uint4 wrec = make_uint4(0u, 0u, 0u, 0u), crec = make_uint4(0u, 0u, 0u, 0u);
-    if (lane < k && (e.y & INFO_MAC)) {
-      wrec = __ldg(&a.walk[e.w]);
-      if (a.relative) crec = __ldg(&a.cellq[e.w]);
-    }
-    // accurate mode: per-target opening angle for nodes undecided for the
-    // group; targets that accept take the node as a monopole now, the rest
-    // open it
-    uint32_t macm = __ballot_sync(0xffffffffu, lane < k && (e.y & INFO_MAC));
-    while (macm) {
-      const int src = __ffs(macm) - 1;
-      macm &= macm - 1;
-      const uint32_t node = __shfl_sync(0xffffffffu, e.w, src);
-      const uint32_t me = __shfl_sync(0xffffffffu, e.z, src);
-      const int dep = wn_depth(__shfl_sync(0xffffffffu, e.y, src));
-      const uint4 w = make_uint4(__shfl_sync(0xffffffffu, wrec.x, src), __shfl_sync(0xffffffffu, wrec.y, src),
-                                 __shfl_sync(0xffffffffu, wrec.z, src), __shfl_sync(0xffffffffu, wrec.w, src));
-      const float hnode = half_side(a.h0_u, dep);
-      uint4 cw = make_uint4(0u, 0u, 0u, 0u);
-      if (a.relative)
-        cw = make_uint4(__shfl_sync(0xffffffffu, crec.x, src), __shfl_sync(0xffffffffu, crec.y, src),
-                        __shfl_sync(0xffffffffu, crec.z, src), __shfl_sync(0xffffffffu, crec.w, src));
-      bool accept = false;
-      if (has && ((me >> tgt) & 1u)) {
-        float d2 = 0.f;
-        const uint32_t wq[3] = {w.x, w.y, w.z};
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          const float dd = (float)rel32(wq[d], tq[d], PERIODIC) * a.u_inv;
-          d2 = fmaf(dd, dd, d2);
-        }
-        if (a.relative) {
-          // point_in_node_cell with a margin (a target on the cell's face
-          // opens the node), then the truncation estimate
-          const uint32_t cq3[3] = {cw.x, cw.y, cw.z};
-          bool inside = true;
-#pragma unroll
-          for (int d = 0; d < 3; ++d)
-            inside = inside && fabsf((float)rel32(cq3[d], tq[d], PERIODIC) * a.u_inv) <= hnode * 1.0001f;
-          const float qf = __uint_as_float(cw.w), m = __uint_as_float(w.w);
-          accept = !inside && d2 > 0.f && qf * (d2 + a.eps2_u) < a.rel_k * m * (d2 * d2 * sqrtf(d2));
-        } else {
-          accept = 4.f * hnode * hnode < a.theta2 * d2;
-        }
-      }
-      const uint32_t am = __ballot_sync(0xffffffffu, accept);
-      if (am) {  // one monopole entry for the accepting targets (same slot on every lane)
-        if (lane == src) {
-          const uint4 GO = reinterpret_cast<const uint4*>(gbox)[2];
-          const uint32_t oq[3] = {GO.x, GO.y, GO.z};
-          lists.mono.put(nlm, (float)rel32(w.x, oq[0], PERIODIC) * a.u_inv,
-                         (float)rel32(w.y, oq[1], PERIODIC) * a.u_inv, (float)rel32(w.z, oq[2], PERIODIC) * a.u_inv,
-                         __uint_as_float(w.w), 2.f * hnode, am, node);
-        }
-        ++nlm;
-      }
-      if (lane == src) e.z = me & ~am;
-    }
-    __syncwarp();
-    // distribute the children of the popped entries over the lanes
-    const uint32_t excl = incl - nc;
-    if (lane < k)
-      for (uint32_t c = 0; c < nc; ++c) owner[excl + c] = (uint8_t)lane;
-    __syncwarp();
-    const uint32_t total = __shfl_sync(0xffffffffu, incl, k - 1);
-    have = (uint32_t)lane < total;
-    const int o = have ? owner[lane] : 0;
-    const uint32_t ofirst = __shfl_sync(0xffffffffu, e.x, o);
-    const uint32_t omask = __shfl_sync(0xffffffffu, e.z, o);
-    const uint32_t oexcl = __shfl_sync(0xffffffffu, excl, o);
-    __syncwarp();
-    if (have) {
-      item = ofirst + ((uint32_t)lane - oexcl);
-      imask = omask;
-    }
-  }
-  __syncwarp();
-  store_sums(a, p, has, count, s0[lane], s1[lane], none, neval);
 }
 
 template <int MIN_BLOCKS, bool PERIODIC, int KERNEL>
@@ -1138,11 +877,7 @@ __global__ void __launch_bounds__(WALK_THREADS, MIN_BLOCKS) k_walk(const __grid_
     g = __shfl_sync(0xffffffffu, g, 0);
     if ((int64_t)g >= a.ngroups) break;
     const uint32_t first = a.gfirst[g], count = a.gsize[g];
-    if constexpr (KERNEL == K_ACC)
-      walk_accurate<PERIODIC>(a, first, count, mem.lists, mem.owner, reinterpret_cast<StackEntry*>(stk), mem.rpos,
-                              mem.rmask, mem.s0, mem.s1, mem.tfs, mem.gbox);
-    else
-      walk_parity<PERIODIC, KERNEL>(a, first, count, mem, stk);
+    walk_group<PERIODIC, KERNEL>(a, first, count, mem, stk);
   }
 }
 
@@ -1227,9 +962,9 @@ __global__ void k_deferred(WalkArgs a, uint32_t n_items) {
 
 // Resident blocks (of 4 warps) per SM, i.e. the register budget: the parity
 // walk takes 96 registers (clustered 256^3: 44.0 ms at 4 blocks, 40.3 at 5, 41.0
-// at 6 with 72 bytes of spills), the accurate one 66 (128^3: 10.7 at 5, 10.4 at
-// 6, 10.3 at 7).
-template <bool PERIODIC, int KERNEL> constexpr int walk_blocks() { return KERNEL == K_ACC ? 7 : 5; }
+// at 6 with 72 bytes of spills), the accurate one 64 (clustered 128^3: 7.46 at 5,
+// 7.40 at 6, 7.51 at 7, where shared memory leaves the L1 cache 16 KB).
+template <bool PERIODIC, int KERNEL> constexpr int walk_blocks() { return KERNEL == K_ACC ? 6 : 5; }
 
 template <bool PERIODIC, int KERNEL>
 static int blocks_for() {
