@@ -831,8 +831,8 @@ void launch_octree_links(int64_t n, int64_t n_int, TreeBuffers& t, void* scan_sc
 // Level by level from the deepest internal nodes to the root: each launch
 // finishes one depth, so every node reads finished children without atomics
 // or fences.  One host synchronisation brings the per-depth counts back.
-void launch_aggregate(const Particles& p, int64_t n, int64_t n_int, double box, TreeBuffers& t, cudaStream_t s,
-                      bool with_quad) {
+void launch_aggregate(const Particles& p, int64_t n, int64_t n_int, double box, TreeBuffers& t, uint32_t* host_counts,
+                      cudaStream_t s, bool with_quad) {
   (void)n;
   if (n_int <= 0) return;
   uint32_t* hist = t.depth_tab;
@@ -841,8 +841,8 @@ void launch_aggregate(const Particles& p, int64_t n, int64_t n_int, double box, 
   TPM_LAUNCH_CHECK();
   k_depth_offsets<<<1, 32, 0, s>>>(t.depth_tab);
   TPM_LAUNCH_CHECK();
-  uint32_t counts[DEPTH_BINS];
-  TPM_CUDA(cudaMemcpyAsync(counts, hist, sizeof(counts), cudaMemcpyDeviceToHost, s));
+  const uint32_t* counts = host_counts;
+  TPM_CUDA(cudaMemcpyAsync(host_counts, hist, DEPTH_BINS * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   k_depth_scatter<<<grid_for(n_int, 256, 1ll << 30), 256, 0, s>>>(n_int, t.o_depth, t.depth_tab + 2 * DEPTH_BINS + 1,
                                                                    t.o_cnt);
   TPM_LAUNCH_CHECK();

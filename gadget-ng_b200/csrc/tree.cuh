@@ -111,8 +111,9 @@ void launch_octree_nodes(int64_t n, TreeBuffers& t, cudaStream_t s);
 void launch_octree_links(int64_t n, int64_t n_int, TreeBuffers& t, void* scan_scratch, cudaStream_t s);
 // Level-synchronous moments, deepest level first: mass and centre of mass, and
 // with_quad the quadrupole tensors too.
-void launch_aggregate(const Particles& p, int64_t n, int64_t n_int, double box, TreeBuffers& t, cudaStream_t s,
-                      bool with_quad = false);
+// host_counts: DEPTH_BINS words of pinned host memory.
+void launch_aggregate(const Particles& p, int64_t n, int64_t n_int, double box, TreeBuffers& t, uint32_t* host_counts,
+                      cudaStream_t s, bool with_quad = false);
 void launch_walk_records(const Particles& p, int64_t n, int64_t n_int, TreeBuffers& t, cudaStream_t s);
 // Per internal node: the centre of its octree cell (child_center replayed
 // along the node's octant path, octree.rs:446-465) in fixed point and the

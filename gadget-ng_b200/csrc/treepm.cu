@@ -209,8 +209,22 @@ struct Cosmo {
 
 }  // namespace
 
+// What the host reads back from the device during a force evaluation, in pinned
+// memory: the copies queue behind the kernels and one synchronisation serves
+// them all.
+struct Readback {
+  uint32_t err, pm_err;
+  uint32_t scalars[4];
+  uint32_t depth_counts[DEPTH_BINS];
+  uint32_t learned_groups;
+  unsigned long long learned_count;
+  unsigned long long stats[8];
+  TreeParams params;
+};
+
 struct tpm_handle {
   tpm_config cfg{};
+  Readback* back = nullptr;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   double r_s = 0, r_cut = 0, rc2 = 0, thr = 0;
@@ -308,7 +322,6 @@ struct tpm_handle {
     int phase = 0;  // 0 idle, 1 sorted + deposited, 2 short range done (domain-decomposed calls)
     unsigned long long launches0 = 0;
     bool use_net = false;
-    int64_t walk_groups = 0;
     double eps2 = 0.0;
   } fe;
 
@@ -346,11 +359,16 @@ int fail(tpm_handle* h, const Error& e) {
   return e.code ? e.code : TPM_ERR_CUDA;
 }
 
+// Wait for the stream (and for any other readback queued on it) and raise
+// what the device flagged.
 void check_dev_err(tpm_handle* h) {
-  if (h->pm.err) pm_check(h->pm, h->stream);
-  uint32_t e = 0;
-  TPM_CUDA(cudaMemcpyAsync(&e, h->T.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
+  h->back->pm_err = 0;
+  if (h->pm.err)
+    TPM_CUDA(cudaMemcpyAsync(&h->back->pm_err, h->pm.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
+  TPM_CUDA(cudaMemcpyAsync(&h->back->err, h->T.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
   TPM_CUDA(cudaStreamSynchronize(h->stream));
+  if (h->back->pm_err) pm_check(h->pm, h->stream);
+  const uint32_t e = h->back->err;
   if (!e) return;
   TPM_CUDA(cudaMemsetAsync(h->T.err, 0, sizeof(uint32_t), h->stream));
   if (e & DEV_ERR_NONFINITE) throw Error(TPM_ERR_NONFINITE, "non-finite position or mass");
@@ -561,16 +579,18 @@ void fe_sort(tpm_handle* h) {
   const double box = h->cfg.box_size;
   h->fe.launches0 = g_kernel_launches;
   TPM_CUDA(cudaEventRecord(h->ev[0], s));
-  TPM_CUDA(cudaMemsetAsync(h->stats_dev, 0, 8 * sizeof(unsigned long long), s));
+  // the statistics, the walk's work counter and its deferred count: one block
+  TPM_CUDA(cudaMemsetAsync(h->stats_dev, 0, 10 * sizeof(unsigned long long), s));
   const bool need_tree = !h->pm_only;
   h->fe.use_net = need_tree && h->learned && h->net_attached;
-  h->fe.walk_groups = 0;
   h->tree_valid = false;
   if (need_tree) {
     launch_bbox_root(h->P[h->cur], n, box, T, s);
     launch_tree_keys(h->P[h->cur], n, box, T, s);
     TPM_CUDA(cudaEventRecord(h->ev[1], s));
-    radix_sort_u64(T.key_hi, T.perm, n, 63, h->sort_scratch, h->sort_bytes, s);
+    // every digit of an octant path varies in a box that is not a clump of
+    // lattice points, so all eight passes run without asking the host
+    radix_sort_u64_all_passes(T.key_hi, T.perm, n, h->sort_scratch, h->sort_bytes, s);
     launch_fix_ties(h->P[h->cur], n, box, T, s);
     launch_permute(h->P[h->cur], h->P[1 - h->cur], n, T.perm, s);
     h->cur = 1 - h->cur;
@@ -591,7 +611,6 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
   const double box = h->cfg.box_size;
   const bool need_tree = !h->pm_only;
   const bool use_net = h->fe.use_net;
-  int64_t walk_groups = 0;
   h->fe.eps2 = eps2;
   if (need_tree) {
     // ---- tree
@@ -600,18 +619,18 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
       TPM_CUDA(cudaMemsetAsync(T.scalars, 0, 4 * sizeof(uint32_t), s));
       launch_karras(n, T, s);
       exclusive_scan_u32(T.oct_count, T.oct_base, n - 1, &T.scalars[0], h->scan_scratch, s);
-      uint32_t sc[4];
-      TPM_CUDA(cudaMemcpyAsync(sc, T.scalars, sizeof(sc), cudaMemcpyDeviceToHost, s));
-      TPM_CUDA(cudaMemcpyAsync(&h->params_host, T.params, sizeof(TreeParams), cudaMemcpyDeviceToHost, s));
+      TPM_CUDA(cudaMemcpyAsync(h->back->scalars, T.scalars, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+      TPM_CUDA(cudaMemcpyAsync(&h->back->params, T.params, sizeof(TreeParams), cudaMemcpyDeviceToHost, s));
       TPM_CUDA(cudaStreamSynchronize(s));
-      h->n_int = sc[0];
+      h->params_host = h->back->params;
+      h->n_int = h->back->scalars[0];
       ensure_tree_capacity(h, h->n_int);
       launch_octree_nodes(n, T, s);
       launch_octree_links(n, h->n_int, T, h->scan_scratch, s);
       // the accurate walk's relative opening criterion reads |Q|_F and the
       // cell centres: the quadrupole pass runs only for it
       const bool rel = relative_mac(h);
-      launch_aggregate(h->P[h->cur], n, h->n_int, box, T, s, rel);
+      launch_aggregate(h->P[h->cur], n, h->n_int, box, T, h->back->depth_counts, s, rel);
       h->quad_valid = rel;
       if (rel) launch_cell_q(h->n_int, box, T, s);
       launch_walk_records(h->P[h->cur], n, h->n_int, T, s);
@@ -619,18 +638,18 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
       const double extent = max_extent(h);
       while (pack_depth < DEPTH_BINS && !(std::ldexp(2.0 * h->params_host.half, -pack_depth) <= extent)) ++pack_depth;
       launch_groups(n, h->n_int, walk_group_size(n), pack_depth, T, h->scan_scratch, s);
-      TPM_CUDA(cudaMemcpyAsync(sc, T.scalars, sizeof(sc), cudaMemcpyDeviceToHost, s));
-      TPM_CUDA(cudaStreamSynchronize(s));
-      h->n_groups = sc[1];
-      h->stats.max_tree_depth = (int32_t)sc[2];
+      // the group count and the tree depth stay on the device until the end of
+      // the evaluation (the learned path sizes a launch by the group count)
+      TPM_CUDA(cudaMemcpyAsync(h->back->scalars, T.scalars, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+      if (use_net) TPM_CUDA(cudaStreamSynchronize(s));
     } else {
-      TPM_CUDA(cudaMemcpyAsync(&h->params_host, T.params, sizeof(TreeParams), cudaMemcpyDeviceToHost, s));
+      TPM_CUDA(cudaMemcpyAsync(&h->back->params, T.params, sizeof(TreeParams), cudaMemcpyDeviceToHost, s));
       TPM_CUDA(cudaStreamSynchronize(s));
-      h->n_groups = 0;
+      h->params_host = h->back->params;
+      std::memset(h->back->scalars, 0, sizeof(h->back->scalars));
     }
     h->tree_valid = true;
     TPM_CUDA(cudaEventRecord(h->ev[3], s));
-    walk_groups = h->n_groups;
     if (use_net) {
       // the network and the dense-cell mask read the mesh: long range first
       const Particles& P = h->P[h->cur];
@@ -645,12 +664,9 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
       if (h->net.near_cells > 0.f) {  // exact pairs below the mesh scale for the network's particles
         near_of(h, eps2, h->fallback, h->srx, h->sry, h->srz);
       }
-      learned_groups(T.grp_first, T.grp_size, h->n_groups, h->fallback, h->lgrp_first, h->lgrp_size, h->lgrp_count,
+      learned_groups(T.grp_first, T.grp_size, n >= 2 ? h->back->scalars[1] : 0, h->fallback, h->lgrp_first, h->lgrp_size, h->lgrp_count,
                      s);
-      uint32_t ng = 0;
-      TPM_CUDA(cudaMemcpyAsync(&ng, h->lgrp_count, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-      TPM_CUDA(cudaStreamSynchronize(s));
-      walk_groups = ng;
+      TPM_CUDA(cudaMemcpyAsync(&h->back->learned_groups, h->lgrp_count, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
       TPM_CUDA(cudaEventRecord(h->ev[8], s));
     }
     // ---- short-range walk
@@ -669,7 +685,7 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
       a.child_ids = T.child_ids; a.o_com = T.o_com; a.leaf_depth = T.leaf_depth;
       a.gfirst = use_net ? h->lgrp_first : T.grp_first;
       a.gsize = use_net ? h->lgrp_size : T.grp_size;
-      a.ngroups = walk_groups;
+      a.ngroups = use_net ? h->lgrp_count : &T.scalars[1];
       a.work = h->work;
       a.scale = scale; a.box = box; a.rc2 = h->rc2; a.thr = h->thr; a.h0 = h0;
       a.periodic = h->periodic ? 1 : 0;
@@ -760,13 +776,8 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
       h->stats.terminal_depth = dstar;
       a.h_term = std::ldexp(a.h0_u, -dstar);
       a.term_depth = dstar;
-      TPM_CUDA(cudaMemsetAsync(h->work, 0, sizeof(uint32_t), s));
-      TPM_CUDA(cudaMemsetAsync(h->ndeferred, 0, sizeof(uint32_t), s));
       launch_walk(a, h->walk_grid, s);
-      uint32_t nd = 0;
-      TPM_CUDA(cudaMemcpyAsync(&nd, h->ndeferred, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-      TPM_CUDA(cudaStreamSynchronize(s));
-      if (nd) launch_deferred(a, std::min(nd, DEFERRED_CAP), s);
+      launch_deferred(a, s);
     } else {
       TPM_CUDA(cudaMemsetAsync(h->srx, 0, sizeof(float) * n, s));
       TPM_CUDA(cudaMemsetAsync(h->sry, 0, sizeof(float) * n, s));
@@ -780,7 +791,6 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
     TPM_CUDA(cudaEventRecord(h->ev[3], s));
   }
   TPM_CUDA(cudaEventRecord(h->ev[4], s));
-  h->fe.walk_groups = walk_groups;
 }
 
 // fe_long_range: CIC deposit (unless the caller deposited already), FFT
@@ -789,7 +799,6 @@ void fe_long_range(tpm_handle* h, double g, double kick, bool deposit, bool solv
   cudaStream_t s = h->stream;
   const int64_t n = h->n;
   const bool use_net = h->fe.use_net;
-  const int64_t walk_groups = h->fe.walk_groups;
   const double eps2 = h->fe.eps2;
   const Particles& P = h->P[h->cur];
   if (!use_net) {
@@ -812,9 +821,15 @@ void fe_long_range(tpm_handle* h, double g, double kick, bool deposit, bool solv
   ga.kick = kick;
   pm_gather_kick(h->pm, ga, s);
   TPM_CUDA(cudaEventRecord(h->ev[6], s));
+  Readback& rb = *h->back;
+  TPM_CUDA(cudaMemcpyAsync(rb.stats, h->stats_dev, sizeof(rb.stats), cudaMemcpyDeviceToHost, s));
+  if (use_net)
+    TPM_CUDA(cudaMemcpyAsync(&rb.learned_count, h->learned_count, sizeof(rb.learned_count), cudaMemcpyDeviceToHost, s));
   check_dev_err(h);
-  unsigned long long st[8];
-  TPM_CUDA(cudaMemcpy(st, h->stats_dev, sizeof(st), cudaMemcpyDeviceToHost));
+  const unsigned long long* st = rb.stats;
+  h->n_groups = h->pm_only ? 0 : rb.scalars[1];
+  if (!h->pm_only && n >= 2) h->stats.max_tree_depth = (int32_t)rb.scalars[2];
+  const int64_t walk_groups = use_net ? rb.learned_groups : h->n_groups;
   h->stats.n_particles = n;
   h->stats.n_tree_nodes = h->n_int;
   h->stats.n_groups = h->n_groups;
@@ -827,9 +842,7 @@ void fe_long_range(tpm_handle* h, double g, double kick, bool deposit, bool solv
   h->stats.ms_sort = ms_between(h->ev[1], h->ev[2]);
   h->stats.ms_build = ms_between(h->ev[2], h->ev[3]);
   if (use_net) {
-    unsigned long long nl = 0;
-    TPM_CUDA(cudaMemcpy(&nl, h->learned_count, sizeof(nl), cudaMemcpyDeviceToHost));
-    h->stats.learned_particles = (int64_t)nl;
+    h->stats.learned_particles = (int64_t)rb.learned_count;
     h->stats.walk_groups = walk_groups;
     h->stats.ms_pm = ms_between(h->ev[3], h->ev[7]);
     h->stats.ms_learned = ms_between(h->ev[7], h->ev[8]);
@@ -940,10 +953,22 @@ void kdk_device(tpm_handle* h, double kick_half, double drift, double kick_half2
   h->stats.kernel_launches += 1;  // the kick-drift kernel
 }
 
-void upload(tpm_handle* h, const double* pos, const double* vel, const double* mass, int64_t n) {
+// Queue the copies of a state into the staging buffer (positions 3n, masses n,
+// momenta 3n): the resident state is not touched yet.
+void stage_upload(tpm_handle* h, const double* pos, const double* vel, const double* mass, int64_t n) {
+  cudaStream_t s = h->stream;
+  TPM_CUDA(cudaMemcpyAsync(h->staging, pos, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, s));
+  TPM_CUDA(cudaMemcpyAsync(h->staging + 3 * n, mass, sizeof(double) * n, cudaMemcpyHostToDevice, s));
+  if (vel) TPM_CUDA(cudaMemcpyAsync(h->staging + 4 * n, vel, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, s));
+}
+
+void check_upload(const double* pos, const double* mass, int64_t n) {
   if (n < 0 || n >= (int64_t)1 << 31) throw Error(TPM_ERR_INVALID_ARGUMENT, "particle count out of range");
   if (n > 0 && (!pos || !mass)) throw Error(TPM_ERR_INVALID_ARGUMENT, "positions and masses are required");
-  ensure_capacity(h, std::max<int64_t>(n, 1));
+}
+
+// The staged state becomes the resident one.
+void take_upload(tpm_handle* h, bool vel, int64_t n) {
   h->n = n;
   h->n_owned = n;
   h->cur = 0;
@@ -952,18 +977,26 @@ void upload(tpm_handle* h, const double* pos, const double* vel, const double* m
   h->m_total_valid = false;
   if (n == 0) return;
   cudaStream_t s = h->stream;
-  double* dpos = h->staging;
-  double* dmass = h->staging + 3 * n;
-  TPM_CUDA(cudaMemcpyAsync(dpos, pos, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, s));
-  TPM_CUDA(cudaMemcpyAsync(dmass, mass, sizeof(double) * n, cudaMemcpyHostToDevice, s));
-  double* dvel = nullptr;
-  if (vel) {
-    dvel = h->staging + 4 * n;
-    TPM_CUDA(cudaMemcpyAsync(dvel, vel, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, s));
-  }
-  k_encode<<<grid_for(n, 256, 1ll << 30), 256, 0, s>>>(dpos, dvel, dmass, n, h->cfg.box_size, h->P[0], h->T.err);
+  k_encode<<<grid_for(n, 256, 1ll << 30), 256, 0, s>>>(h->staging, vel ? h->staging + 4 * n : nullptr,
+                                                       h->staging + 3 * n, n, h->cfg.box_size, h->P[0], h->T.err);
   TPM_LAUNCH_CHECK();
   check_dev_err(h);
+}
+
+void upload(tpm_handle* h, const double* pos, const double* vel, const double* mass, int64_t n) {
+  check_upload(pos, mass, n);
+  ensure_capacity(h, std::max<int64_t>(n, 1));
+  if (n > 0) stage_upload(h, pos, vel, mass, n);
+  take_upload(h, vel != nullptr, n);
+}
+
+// Is every index below n?  (No branch in the loop: it runs at the speed of the
+// host's memory.)
+bool indices_below(const uint64_t* idx, int64_t count, int64_t n) {
+  uint64_t over = 0;  // the sign bit of n - 1 - idx, or of idx itself
+  const uint64_t top = (uint64_t)n - 1u;
+  for (int64_t k = 0; k < count; ++k) over |= (top - idx[k]) | idx[k];
+  return n > 0 ? (over >> 63) == 0 : count == 0;
 }
 
 }  // namespace
@@ -1023,8 +1056,11 @@ int tpm_create(const tpm_config* cfg, tpm_handle** out) {
     h->T.scalars = h->alloc<uint32_t>(8, 0);
     h->T.depth_tab = h->alloc<uint32_t>(3 * DEPTH_BINS + 1, 0);
     h->T.err = h->alloc<uint32_t>(1, 0);
-    h->stats_dev = h->alloc<unsigned long long>(8, 0);
-    h->work = h->alloc<uint32_t>(1, 0);
+    h->stats_dev = h->alloc<unsigned long long>(10, 0);
+    h->work = reinterpret_cast<uint32_t*>(h->stats_dev + 8);
+    h->ndeferred = reinterpret_cast<uint32_t*>(h->stats_dev + 9);
+    TPM_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&h->back), sizeof(Readback), cudaHostAllocDefault));
+    std::memset(h->back, 0, sizeof(Readback));
     h->dom_counts = h->alloc<unsigned long long>(MAX_RANKS + 8, 0);
     h->lgrp_count = h->alloc<uint32_t>(1, 0);
     if (h->learned) {
@@ -1034,7 +1070,6 @@ int tpm_create(const tpm_config* cfg, tpm_handle** out) {
       h->cell_scan = h->alloc<char>(scan_scratch_bytes(nm3 + 1), 0);
     }
     h->learned_count = h->alloc<unsigned long long>(1, 0);
-    h->ndeferred = h->alloc<uint32_t>(1, 0);
     h->deferred = h->alloc<uint2>(DEFERRED_CAP, 0);
     int sms = prop.multiProcessorCount;
     {
@@ -1061,6 +1096,7 @@ void tpm_destroy(tpm_handle* h) {
   cudaSetDevice(h->cfg.device);
   if (h->stream) cudaStreamSynchronize(h->stream);
   for (const auto& a : h->allocs) cudaFree(a.p);
+  if (h->back) cudaFreeHost(h->back);
   pm_slab_free(h->slab);
   pm_plan_free(h->pm);
   for (auto& e : h->ev)
@@ -1396,20 +1432,52 @@ int tpm_accelerations_for_indices(tpm_handle* h, const double* pos, const double
   try {
     TPM_CUDA(cudaSetDevice(h->cfg.device));
     if (n_idx < 0 || (n_idx > 0 && (!idx || !out))) throw Error(TPM_ERR_INVALID_ARGUMENT, "bad index arrays");
-    for (int64_t k = 0; k < n_idx; ++k)
-      if ((int64_t)idx[k] >= n) throw Error(TPM_ERR_INVALID_ARGUMENT, "global index out of range");
-    upload(h, pos, nullptr, mass, n);
-    if (n_idx == 0) return TPM_OK;
-    force_eval(h, eps2, g, 0.0);
+    const auto refuse = [] { throw Error(TPM_ERR_INVALID_ARGUMENT, "global index out of range"); };
     cudaStream_t s = h->stream;
+    // The state's copies run while the host looks through the indices; a
+    // refused call leaves the resident state as it was, so nothing is staged
+    // where staging would first have to reallocate it.
+    const bool overlap = n > 0 && n <= h->cap && pos && mass && n_idx > 0;
+    const int64_t m0 = std::min<int64_t>(n, n_idx);  // indices of the first chunk
+    if (overlap) {
+      if (!h->copy_stream) TPM_CUDA(cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));
+      if (!h->ev_pos) TPM_CUDA(cudaEventCreateWithFlags(&h->ev_pos, cudaEventDisableTiming));
+      if (!h->ev_done) TPM_CUDA(cudaEventCreateWithFlags(&h->ev_done, cudaEventDisableTiming));
+      stage_upload(h, pos, nullptr, mass, n);
+      TPM_CUDA(cudaEventRecord(h->ev_pos, s));
+      const bool good = indices_below(idx, n_idx, n);
+      if (!good) {
+        TPM_CUDA(cudaStreamSynchronize(s));  // the caller's buffers are free on return
+        refuse();
+      }
+      // the indices follow on the copy stream, beside the force evaluation
+      // (dom_flags: domain scratch, unused in this call)
+      TPM_CUDA(cudaStreamWaitEvent(h->copy_stream, h->ev_pos, 0));
+      TPM_CUDA(cudaMemcpyAsync(h->dom_flags, idx, sizeof(uint64_t) * m0, cudaMemcpyHostToDevice, h->copy_stream));
+      TPM_CUDA(cudaEventRecord(h->ev_done, h->copy_stream));
+      try {
+        take_upload(h, false, n);
+        force_eval(h, eps2, g, 0.0);
+      } catch (...) {
+        cudaStreamSynchronize(h->copy_stream);
+        throw;
+      }
+      TPM_CUDA(cudaStreamWaitEvent(s, h->ev_done, 0));
+    } else {
+      if (!indices_below(idx, n_idx, n)) refuse();
+      upload(h, pos, nullptr, mass, n);
+      if (n_idx == 0) return TPM_OK;
+      force_eval(h, eps2, g, 0.0);
+    }
     uint32_t* inv = h->T.perm;  // free after the build
     k_inverse_perm<<<grid_for(n, 256, 1ll << 30), 256, 0, s>>>(h->P[h->cur].id, n, inv);
     TPM_LAUNCH_CHECK();
-    uint64_t* didx = (uint64_t*)h->sort_scratch;
+    uint64_t* didx = h->dom_flags;
     double* dout = h->staging;
     for (int64_t k0 = 0; k0 < n_idx; k0 += n) {  // chunks of at most n indices
       const int64_t m = std::min<int64_t>(n, n_idx - k0);
-      TPM_CUDA(cudaMemcpyAsync(didx, idx + k0, sizeof(uint64_t) * m, cudaMemcpyHostToDevice, s));
+      if (!overlap || k0 > 0)
+        TPM_CUDA(cudaMemcpyAsync(didx, idx + k0, sizeof(uint64_t) * m, cudaMemcpyHostToDevice, s));
       k_pick<<<grid_for(m, 256, 1ll << 30), 256, 0, s>>>(inv, didx, m, h->ax, h->ay, h->az, dout);
       TPM_LAUNCH_CHECK();
       TPM_CUDA(cudaMemcpyAsync(out + 3 * k0, dout, sizeof(double) * 3 * m, cudaMemcpyDeviceToHost, s));
@@ -2151,7 +2219,7 @@ int64_t tpm_export_tree(tpm_handle* h, int64_t cap, int32_t* depth, double* mass
       throw Error(TPM_ERR_INVALID_ARGUMENT, "null export array");
     cudaStream_t s = h->stream;
     if (!h->quad_valid && ni > 0) {  // the force evaluation made mass and centre of mass only
-      launch_aggregate(h->P[h->cur], n, ni, h->cfg.box_size, h->T, s, true);
+      launch_aggregate(h->P[h->cur], n, ni, h->cfg.box_size, h->T, h->back->depth_counts, s, true);
       h->quad_valid = true;
     }
     int32_t* dd;

@@ -140,15 +140,6 @@ __device__ __forceinline__ int32_t rel32(uint32_t a, uint32_t b, int periodic) {
 }
 
 
-__device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v, int lane) {
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    uint32_t y = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= o) v += y;
-  }
-  return v;
-}
-
 // h0 * 2^-dep by exponent arithmetic: h0 (the root half side in walk units,
 // O(r_cut / cell)) stays a normal float for every tree depth (-1 <= dep < 64).
 __device__ __forceinline__ float half_side(float h0, int dep) {
@@ -871,11 +862,12 @@ __global__ void __launch_bounds__(WALK_THREADS, MIN_BLOCKS) k_walk(const __grid_
   __syncwarp();
   const int64_t gw = (int64_t)blockIdx.x * WALK_WARPS + wid;
   uint4* stk = reinterpret_cast<uint4*>(a.stack) + gw * STACK_ENTRIES;
+  const uint32_t ngroups = *a.ngroups;
   for (;;) {
     uint32_t g = 0;
     if (lane == 0) g = atomicAdd(a.work, 1u);
     g = __shfl_sync(0xffffffffu, g, 0);
-    if ((int64_t)g >= a.ngroups) break;
+    if (g >= ngroups) break;
     const uint32_t first = a.gfirst[g], count = a.gsize[g];
     walk_group<PERIODIC, KERNEL>(a, first, count, mem, stk);
   }
@@ -883,10 +875,7 @@ __global__ void __launch_bounds__(WALK_THREADS, MIN_BLOCKS) k_walk(const __grid_
 
 // ---- per-target exact walk below a node whose centre of mass coincides with
 // the target (the reference opens such a monopole, short_range.rs:316-330)
-__global__ void k_deferred(WalkArgs a, uint32_t n_items) {
-  uint32_t it = blockIdx.x * blockDim.x + threadIdx.x;
-  if (it >= n_items || it >= a.cap_deferred) return;
-  const uint2 job = a.deferred[it];
+__device__ void deferred_walk(const WalkArgs& a, uint2 job) {
   const uint32_t p = job.x;
   double xi[3];
   target_pos(a, p, xi);
@@ -956,6 +945,12 @@ __global__ void k_deferred(WalkArgs a, uint32_t n_items) {
   atomicAdd(&a.ay[p], fy * a.out_scale);
   atomicAdd(&a.az[p], fz * a.out_scale);
   atomicAdd(&a.stats[4], 1ull);
+}
+
+__global__ void k_deferred(const __grid_constant__ WalkArgs a) {
+  const uint32_t n = min(*a.ndeferred, a.cap_deferred);
+  for (uint32_t it = blockIdx.x * blockDim.x + threadIdx.x; it < n; it += gridDim.x * blockDim.x)
+    deferred_walk(a, a.deferred[it]);
 }
 
 }  // namespace
@@ -1056,9 +1051,9 @@ void launch_walk(const WalkArgs& a, int grid, cudaStream_t s) {
   TPM_LAUNCH_CHECK();
 }
 
-void launch_deferred(const WalkArgs& a, uint32_t n_items, cudaStream_t s) {
-  if (n_items == 0) return;
-  k_deferred<<<grid_for(n_items, 64, 1ll << 20), 64, 0, s>>>(a, n_items);
+// The count is on the device (zero in nearly every evaluation): one wave.
+void launch_deferred(const WalkArgs& a, cudaStream_t s) {
+  k_deferred<<<148, 64, 0, s>>>(a);
   TPM_LAUNCH_CHECK();
 }
 

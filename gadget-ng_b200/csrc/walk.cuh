@@ -31,7 +31,7 @@ struct WalkArgs {
   // groups
   const uint32_t* gfirst;
   const uint32_t* gsize;
-  int64_t ngroups;
+  const uint32_t* ngroups;  // on the device
   uint32_t* work;
   // geometry (float64 = the reference's decisions; float32 = the fast path)
   double scale, box, rc2, thr, h0;
@@ -81,6 +81,6 @@ int walk_group_size(int64_t n);   // targets per walk group in a box of n partic
 int walk_blocks_per_sm(bool periodic, bool accurate, bool poly);
 size_t walk_stack_words(int grid, int stack_cap);
 void launch_walk(const WalkArgs& a, int grid, cudaStream_t s);
-void launch_deferred(const WalkArgs& a, uint32_t n_items, cudaStream_t s);
+void launch_deferred(const WalkArgs& a, cudaStream_t s);
 
 }  // namespace tpm
