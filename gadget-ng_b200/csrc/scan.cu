@@ -82,6 +82,36 @@ __global__ void k_apply(const uint32_t* __restrict__ in, int64_t n, const uint32
   }
 }
 
+// Short arrays in one block: the three launches above cost more than the
+// passes of a single block (1,000-particle box: three scans, 9 -> 3 launches).
+__global__ void k_scan_one(const uint32_t* __restrict__ in, int64_t n, uint32_t* __restrict__ out,
+                           uint32_t* __restrict__ total_out) {
+  __shared__ uint32_t sh[32];
+  uint32_t carry = 0;
+  for (int64_t c0 = 0; c0 < n; c0 += SCAN_TILE) {
+    uint32_t v[SCAN_ITEMS];
+    uint32_t s = 0;
+    for (int j = 0; j < SCAN_ITEMS; ++j) {
+      const int64_t i = c0 + (int64_t)threadIdx.x * SCAN_ITEMS + j;
+      v[j] = i < n ? in[i] : 0u;
+      s += v[j];
+    }
+    uint32_t tot;
+    uint32_t e = carry + block_excl_scan(s, &tot, sh);
+    for (int j = 0; j < SCAN_ITEMS; ++j) {
+      const int64_t i = c0 + (int64_t)threadIdx.x * SCAN_ITEMS + j;
+      if (i < n) out[i] = e;
+      e += v[j];
+    }
+    carry += tot;
+  }
+  if (threadIdx.x == 0 && total_out) *total_out = carry;
+}
+
+// Up to here one block takes no longer than three launches (~1.5 us per 4,096
+// counts against ~7 us).
+constexpr int64_t SCAN_ONE_MAX = 16384;
+
 }  // namespace
 
 size_t scan_scratch_bytes(int64_t n) { return (size_t)((n + SCAN_TILE - 1) / SCAN_TILE + 1) * sizeof(uint32_t) + 256; }
@@ -90,6 +120,11 @@ void exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* 
                         cudaStream_t s) {
   if (n <= 0) {
     if (total_dev) TPM_CUDA(cudaMemsetAsync(total_dev, 0, sizeof(uint32_t), s));
+    return;
+  }
+  if (n <= SCAN_ONE_MAX) {
+    k_scan_one<<<1, SCAN_BLOCK, 0, s>>>(in, n, out, total_dev);
+    TPM_LAUNCH_CHECK();
     return;
   }
   int64_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;

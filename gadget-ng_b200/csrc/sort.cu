@@ -181,6 +181,106 @@ __global__ void __launch_bounds__(SORT_BLOCK) k_downsweep(const uint64_t* __rest
   }
 }
 
+// Small sorts in one block: all eight digit passes with the pairs in registers
+// and shared memory.  The same stable ranking as k_downsweep (warp match, warps
+// in order), so the result is the same; 24 launches of three kernels per pass,
+// ~6 us each whatever n, become one of ~4 us per pass.
+constexpr int SMALL_THREADS = 1024;
+constexpr int SMALL_WARPS = SMALL_THREADS / 32;
+template <int ITEMS> constexpr size_t small_sort_smem() {
+  return (size_t)SMALL_THREADS * ITEMS * (sizeof(uint64_t) + sizeof(uint32_t)) +
+         (size_t)SMALL_WARPS * 256 * sizeof(uint32_t) + 256 * sizeof(uint32_t);
+}
+template <int ITEMS>
+__global__ void __launch_bounds__(SMALL_THREADS) k_sort_small(uint64_t* __restrict__ keys, uint32_t* __restrict__ vals,
+                                                              int n) {
+  constexpr int TILE = SMALL_THREADS * ITEMS;
+  extern __shared__ __align__(16) unsigned char ss_smem[];
+  uint64_t* s_k = reinterpret_cast<uint64_t*>(ss_smem);
+  uint32_t* s_v = reinterpret_cast<uint32_t*>(s_k + TILE);
+  uint32_t(*wcnt)[256] = reinterpret_cast<uint32_t(*)[256]>(s_v + TILE);
+  uint32_t* lstart = reinterpret_cast<uint32_t*>(wcnt + SMALL_WARPS);
+  __shared__ uint32_t wsum[8];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int seg = warp * (32 * ITEMS);
+  const unsigned lt_mask = (1u << lane) - 1u;
+  uint64_t k[ITEMS];
+  uint32_t v[ITEMS];
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const int idx = seg + j * 32 + lane;
+    k[j] = idx < n ? keys[idx] : ~0ull;  // past the end: stays there, being last in order and in rank
+    v[j] = idx < n ? vals[idx] : 0u;
+  }
+  for (int shift = 0; shift < 64; shift += 8) {
+    for (int i = tid; i < SMALL_WARPS * 256; i += SMALL_THREADS) (&wcnt[0][0])[i] = 0;
+    __syncthreads();
+    uint32_t rk[ITEMS];
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      const uint32_t d = (uint32_t)(k[j] >> shift) & 255u;
+      const unsigned peers = __match_any_sync(0xffffffffu, d);
+      const uint32_t c = wcnt[warp][d];
+      __syncwarp();
+      if (lane == __ffs(peers) - 1) wcnt[warp][d] = c + __popc(peers);
+      __syncwarp();
+      rk[j] = c + __popc(peers & lt_mask);
+    }
+    __syncthreads();
+    // per digit: warp offsets in place and the total, then the digits' starts
+    uint32_t tot = 0, x = 0;
+    if (tid < 256) {
+      for (int w = 0; w < SMALL_WARPS; ++w) {
+        const uint32_t c = wcnt[w][tid];
+        wcnt[w][tid] = tot;
+        tot += c;
+      }
+      x = tot;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (lane == 31) wsum[warp] = x;
+    }
+    __syncthreads();
+    if (tid < 256) {
+      uint32_t before = 0;
+      for (int w = 0; w < warp; ++w) before += wsum[w];
+      lstart[tid] = before + x - tot;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      const uint32_t d = (uint32_t)(k[j] >> shift) & 255u;
+      const uint32_t pos = lstart[d] + wcnt[warp][d] + rk[j];
+      s_k[pos] = k[j];
+      s_v[pos] = v[j];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      k[j] = s_k[seg + j * 32 + lane];
+      v[j] = s_v[seg + j * 32 + lane];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const int idx = seg + j * 32 + lane;
+    if (idx < n) {
+      keys[idx] = k[j];
+      vals[idx] = v[j];
+    }
+  }
+}
+
+template <int ITEMS>
+void sort_small(uint64_t* keys, uint32_t* vals, int64_t n, cudaStream_t s) {
+  TPM_CUDA(cudaFuncSetAttribute(k_sort_small<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)small_sort_smem<ITEMS>()));
+  k_sort_small<ITEMS><<<1, SMALL_THREADS, small_sort_smem<ITEMS>(), s>>>(keys, vals, (int)n);
+  TPM_LAUNCH_CHECK();
+}
+
 }  // namespace
 
 void radix_sort_u64(uint64_t* keys, uint32_t* vals, int64_t n, int key_bits, void* scratch, size_t scratch_bytes,
@@ -240,6 +340,13 @@ void radix_sort_u64_all_passes(uint64_t* keys, uint32_t* vals, int64_t n, void* 
                                cudaStream_t s) {
   if (n <= 1) return;
   if (scratch_bytes < radix_sort_scratch_bytes(n)) throw Error(1, "radix sort scratch too small");
+  if (n <= SORT_SMALL_MAX) {
+    if (n <= SMALL_THREADS) sort_small<1>(keys, vals, n, s);
+    else if (n <= 2 * SMALL_THREADS) sort_small<2>(keys, vals, n, s);
+    else if (n <= 4 * SMALL_THREADS) sort_small<4>(keys, vals, n, s);
+    else sort_small<8>(keys, vals, n, s);
+    return;
+  }
   int64_t ntiles = (n + SORT_TILE - 1) / SORT_TILE;
   char* p = (char*)scratch;
   auto carve = [&](size_t bytes) {

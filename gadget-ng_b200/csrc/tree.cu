@@ -424,13 +424,10 @@ __global__ void k_depth_scatter(int64_t n_int, const uint8_t* __restrict__ o_dep
 // QUAD: also the quadrupole tensors (the walk reads mass and centre of mass
 // only; the quadrupoles are made when the tree is exported).
 template <bool QUAD>
-__global__ void k_aggregate_level(const uint32_t* __restrict__ nodes, int64_t count, double scale,
-                                  const uint32_t* __restrict__ qx, const uint32_t* __restrict__ qy,
-                                  const uint32_t* __restrict__ qz, const double* __restrict__ pmass,
-                                  const uint32_t* __restrict__ slots, double* o_mass, double* o_com, double* o_quad) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  const uint32_t P = nodes[i];
+__device__ __forceinline__ void aggregate_node(uint32_t P, double scale, const uint32_t* __restrict__ qx,
+                                               const uint32_t* __restrict__ qy, const uint32_t* __restrict__ qz,
+                                               const double* __restrict__ pmass, const uint32_t* __restrict__ slots,
+                                               double* o_mass, double* o_com, double* o_quad) {
   // pass 1: mass and centre of mass over the children in octant order
   uint32_t cs[8];
   double mt = 0.0, ax = 0.0, ay = 0.0, az = 0.0;
@@ -493,6 +490,53 @@ __global__ void k_aggregate_level(const uint32_t* __restrict__ nodes, int64_t co
 #pragma unroll
   for (int k = 0; k < 6; ++k) __stcg(&o_quad[6 * (int64_t)P + k], qd[k]);
 }
+
+template <bool QUAD>
+__global__ void k_aggregate_level(const uint32_t* __restrict__ nodes, int64_t count, double scale,
+                                  const uint32_t* __restrict__ qx, const uint32_t* __restrict__ qy,
+                                  const uint32_t* __restrict__ qz, const double* __restrict__ pmass,
+                                  const uint32_t* __restrict__ slots, double* o_mass, double* o_com, double* o_quad) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < count) aggregate_node<QUAD>(nodes[i], scale, qx, qy, qz, pmass, slots, o_mass, o_com, o_quad);
+}
+
+// Small trees in one block: the nodes bucketed by depth, then every level from
+// the deepest up with a block barrier between levels, in place of three
+// bucketing launches, one host synchronisation and one launch per depth.
+constexpr int AGG_SMALL_THREADS = 512;
+template <bool QUAD>
+__global__ void __launch_bounds__(AGG_SMALL_THREADS)
+    k_aggregate_small(int n_int, const uint8_t* __restrict__ o_depth, uint32_t* by_depth, double scale,
+                      const uint32_t* __restrict__ qx, const uint32_t* __restrict__ qy, const uint32_t* __restrict__ qz,
+                      const double* __restrict__ pmass, const uint32_t* __restrict__ slots, double* o_mass,
+                      double* o_com, double* o_quad) {
+  __shared__ uint32_t off[DEPTH_BINS + 1], cur[DEPTH_BINS];
+  if (threadIdx.x < DEPTH_BINS) cur[threadIdx.x] = 0u;
+  __syncthreads();
+  for (int i = threadIdx.x; i < n_int; i += AGG_SMALL_THREADS) atomicAdd(&cur[o_depth[i] & (DEPTH_BINS - 1)], 1u);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t acc = 0;
+    for (int d = 0; d < DEPTH_BINS; ++d) {
+      off[d] = acc;
+      acc += cur[d];
+      cur[d] = off[d];
+    }
+    off[DEPTH_BINS] = acc;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n_int; i += AGG_SMALL_THREADS)
+    by_depth[atomicAdd(&cur[o_depth[i] & (DEPTH_BINS - 1)], 1u)] = (uint32_t)i;
+  for (int d = DEPTH_BINS - 1; d >= 0; --d) {
+    if (off[d] == off[d + 1]) continue;  // the same for the whole block
+    __syncthreads();  // the bucketing, then the deeper level
+    for (uint32_t i = off[d] + threadIdx.x; i < off[d + 1]; i += AGG_SMALL_THREADS)
+      aggregate_node<QUAD>(by_depth[i], scale, qx, qy, qz, pmass, slots, o_mass, o_com, o_quad);
+  }
+}
+
+// Up to here one block is faster than the launches per level.
+constexpr int64_t AGG_SMALL_MAX = 8192;
 
 __global__ void k_walk_nodes(int64_t n_int, double inv_scale, const double* __restrict__ o_mass,
                              const double* __restrict__ o_com, uint4* __restrict__ walk) {
@@ -835,6 +879,19 @@ void launch_aggregate(const Particles& p, int64_t n, int64_t n_int, double box, 
                       cudaStream_t s, bool with_quad) {
   (void)n;
   if (n_int <= 0) return;
+  if (n_int <= AGG_SMALL_MAX) {
+    if (with_quad)
+      k_aggregate_small<true><<<1, AGG_SMALL_THREADS, 0, s>>>((int)n_int, t.o_depth, t.o_cnt, box / TWO32, p.qx, p.qy,
+                                                              p.qz, p.mass, t.o_slots, t.o_mass, t.o_com, t.o_quad);
+    else
+      k_aggregate_small<false><<<1, AGG_SMALL_THREADS, 0, s>>>((int)n_int, t.o_depth, t.o_cnt, box / TWO32, p.qx,
+                                                               p.qy, p.qz, p.mass, t.o_slots, t.o_mass, t.o_com,
+                                                               t.o_quad);
+    TPM_LAUNCH_CHECK();
+    k_walk_nodes<<<grid_for(n_int, 256, 1ll << 30), 256, 0, s>>>(n_int, TWO32 / box, t.o_mass, t.o_com, t.o_walk);
+    TPM_LAUNCH_CHECK();
+    return;
+  }
   uint32_t* hist = t.depth_tab;
   TPM_CUDA(cudaMemsetAsync(hist, 0, DEPTH_BINS * sizeof(uint32_t), s));
   k_depth_count<<<grid_for(n_int, 256, 1ll << 30), 256, 0, s>>>(n_int, t.o_depth, hist);
