@@ -15,6 +15,20 @@ namespace {
 
 constexpr int SORT_WARPS = SORT_BLOCK / 32;
 
+// Lanes with the same digit (9 bits: 256 marks a lane past the end), by one
+// ballot per bit: match.any on the digit took longer (128^3: keys sorted and
+// particles permuted in .417 ms with it, .359 ms with ballots; 256^3 2.24 / 2.11).
+__device__ __forceinline__ unsigned match_digit(uint32_t d) {
+  unsigned peers = 0xffffffffu;
+#pragma unroll
+  for (int b = 0; b < 9; ++b) {
+    const bool bit = (d >> b) & 1u;
+    const unsigned m = __ballot_sync(0xffffffffu, bit);
+    peers &= bit ? m : ~m;
+  }
+  return peers;
+}
+
 __global__ void k_hist8(const uint64_t* __restrict__ keys, int64_t n, uint32_t* __restrict__ hist) {
   __shared__ uint32_t h[8][256];
   for (int i = threadIdx.x; i < 8 * 256; i += blockDim.x) (&h[0][0])[i] = 0;
@@ -127,7 +141,7 @@ __global__ void __launch_bounds__(SORT_BLOCK) k_downsweep(const uint64_t* __rest
     k[j] = ok ? keys_in[idx] : 0ull;
     v[j] = ok ? vals_in[idx] : 0u;
     uint32_t d = ok ? (uint32_t)((k[j] >> shift) & 255u) : 256u;
-    unsigned peers = __match_any_sync(0xffffffffu, d);
+    unsigned peers = match_digit(d);
     int leader = __ffs(peers) - 1;
     uint32_t c = d < 256u ? wcnt[warp][d] : 0u;
     __syncwarp();
@@ -219,7 +233,7 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_sort_small(uint64_t* __restri
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j) {
       const uint32_t d = (uint32_t)(k[j] >> shift) & 255u;
-      const unsigned peers = __match_any_sync(0xffffffffu, d);
+      const unsigned peers = match_digit(d);
       const uint32_t c = wcnt[warp][d];
       __syncwarp();
       if (lane == __ffs(peers) - 1) wcnt[warp][d] = c + __popc(peers);
