@@ -8,10 +8,8 @@
 // insertion order: a cell is internal iff it holds two or more particles.
 // So the device computes, per particle, the exact sequence of octant choices
 // the insertion would make (same float64 centres, same comparisons), sorts by
-// that path key, and recovers the nodes from the sorted keys with a binary
-// radix tree (Karras 2012, "Maximizing parallelism in the construction of
-// BVHs, octrees and k-d trees"), whose prefix lengths, read in 3-bit digits,
-// give the octree levels.  Mass, centre of mass and quadrupole are then
+// that path key, and reads the nodes off the numbers of octant levels that
+// neighbours in the sorted order share.  Mass, centre of mass and quadrupole are then
 // aggregated bottom-up in float64 with the reference's operation order
 // (aggregate :547-629), so they are bit-identical to the reference's nodes.
 #include "common.cuh"
@@ -186,72 +184,44 @@ __global__ void k_permute(Particles src, Particles dst, int64_t n, const uint32_
 }
 
 // ---------------------------------------------------------------------------
-// binary radix tree (Karras 2012, section 4)
+// octree nodes from the sorted keys
 // ---------------------------------------------------------------------------
-// Common prefix, in bits of the 126-bit digit string, of sorted keys i
-// (preloaded) and j; j out of [0, n) on either side gives -1.
-__device__ __forceinline__ int delta_i(const uint64_t* __restrict__ hi, const uint64_t* __restrict__ lo, int64_t n,
-                                       uint64_t hi_i, uint64_t lo_i, int64_t i, int64_t j) {
-  if ((uint64_t)j >= (uint64_t)n) return -1;
-  const uint64_t a = hi_i ^ __ldg(&hi[j]);
-  if (a) return __clzll((long long)a) - 1;
-  const uint64_t b = lo_i ^ __ldg(&lo[j]);
-  if (b) return 63 + __clzll((long long)b) - 1;
-  return 126 + __clzll((long long)(i ^ j));
+// lev[i] = octant levels that particles i - 1 and i share (-1 at both ends).
+// The cell of depth d that holds particle i starts there iff lev[i] < d, and
+// holds a second particle iff lev[i + 1] >= d: particle i starts the internal
+// nodes of depths lev[i] + 1 .. lev[i + 1], one after the other in the node
+// order.  So nodes, parents and ranges come from one byte per particle and short
+// scans of it, where a binary radix tree over the keys (searched twice per node,
+// six words stored per node, then climbed) took 1.46 of the 2.88 ms of the
+// build at 256^3.
+constexpr int LEV_SCAN = 16;  // neighbours looked at one by one before the search turns to the keys
+
+// Levels shared by two sorted keys.
+__device__ __forceinline__ int shared_levels(uint64_t hi_a, uint64_t lo_a, uint64_t hi_b, uint64_t lo_b) {
+  const uint64_t x = hi_a ^ hi_b;
+  if (x) return (__clzll((long long)x) - 1) / 3;
+  const uint64_t y = lo_a ^ lo_b;
+  return y ? KEY_LEVELS / 2 + (__clzll((long long)y) - 1) / 3 : KEY_LEVELS;
 }
 
-__global__ void k_karras(int64_t n, const uint64_t* __restrict__ hi, const uint64_t* __restrict__ lo,
-                         uint32_t* __restrict__ bl, uint32_t* __restrict__ br, int32_t* __restrict__ bpre,
-                         uint32_t* __restrict__ bfirst, uint32_t* __restrict__ blast, int32_t* __restrict__ bparent,
-                         int32_t* __restrict__ leaf_bparent) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n - 1) return;
-  const uint64_t hi_i = hi[i], lo_i = lo[i];
-  // the direction d and the steps along it (i + k d as a sign choice, not a product)
-  const bool up = delta_i(hi, lo, n, hi_i, lo_i, i, i + 1) - delta_i(hi, lo, n, hi_i, lo_i, i, i - 1) >= 0;
-  auto at = [&](int64_t k) { return up ? i + k : i - k; };
-  const int dmin = delta_i(hi, lo, n, hi_i, lo_i, i, at(-1));
-  int64_t lmax = 2;
-  while (delta_i(hi, lo, n, hi_i, lo_i, i, at(lmax)) > dmin) lmax <<= 1;
-  int64_t l = 0;
-  for (int64_t t = lmax >> 1; t >= 1; t >>= 1)
-    if (delta_i(hi, lo, n, hi_i, lo_i, i, at(l + t)) > dmin) l += t;
-  const int64_t j = at(l);
-  const int dnode = delta_i(hi, lo, n, hi_i, lo_i, i, j);
-  int64_t s = 0, t = l;
-  do {
-    t = (t + 1) >> 1;
-    if (delta_i(hi, lo, n, hi_i, lo_i, i, at(s + t)) > dnode) s += t;
-  } while (t > 1);
-  const int64_t gamma = at(s) + (up ? 0 : -1);
-  const int64_t first = i < j ? i : j, last = i < j ? j : i;
-  const bool left_leaf = first == gamma, right_leaf = last == gamma + 1;
-  bl[i] = (uint32_t)gamma | (left_leaf ? LEAF_BIT : 0u);
-  br[i] = (uint32_t)(gamma + 1) | (right_leaf ? LEAF_BIT : 0u);
-  bpre[i] = dnode;
-  bfirst[i] = (uint32_t)first;
-  blast[i] = (uint32_t)last;
-  if (left_leaf) leaf_bparent[gamma] = (int32_t)i; else bparent[gamma] = (int32_t)i;
-  if (right_leaf) leaf_bparent[gamma + 1] = (int32_t)i; else bparent[gamma + 1] = (int32_t)i;
-  if (i == 0) bparent[0] = -1;
+// Do particles i and j lie in the same cell of depth d (1 .. KEY_LEVELS)?
+__device__ __forceinline__ bool same_cell(const uint64_t* __restrict__ hi, const uint64_t* __restrict__ lo,
+                                          uint64_t hi_i, uint64_t lo_i, int64_t j, int d) {
+  const uint64_t x = hi_i ^ __ldg(&hi[j]);
+  if (d <= KEY_LEVELS / 2) return (x >> (63 - 3 * d)) == 0;
+  return x == 0 && ((lo_i ^ __ldg(&lo[j])) >> (63 - 3 * (d - KEY_LEVELS / 2))) == 0;
 }
 
-// Octree nodes owned by binary node B: depths floor(p_parent/3)+1 .. floor(p_B/3).
-__global__ void k_oct_count(int64_t nb, const int32_t* __restrict__ bpre, const int32_t* __restrict__ bparent,
-                            uint32_t* __restrict__ cnt) {
-  int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (b >= nb) return;
-  const int par = bparent[b];
-  const int dpar = par < 0 ? -1 : bpre[par] / 3;
-  cnt[b] = (uint32_t)(bpre[b] / 3 - dpar);
-}
-
-__device__ __forceinline__ int32_t owner_deepest(int32_t b, const int32_t* __restrict__ bparent,
-                                                 const uint32_t* __restrict__ cnt,
-                                                 const uint32_t* __restrict__ base) {
-  // at most three binary levels share one 3-bit octree level
-  for (int guard = 0; cnt[b] == 0 && guard < 8; ++guard) b = bparent[b];
-  return (int32_t)(base[b] + cnt[b] - 1);
+__global__ void k_levels(int64_t n, const uint64_t* __restrict__ hi, const uint64_t* __restrict__ lo,
+                         int8_t* __restrict__ lev, uint32_t* __restrict__ cnt) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint64_t h = hi[i], l = lo[i];
+  const int before = i > 0 ? shared_levels(hi[i - 1], lo[i - 1], h, l) : -1;
+  const int after = i + 1 < n ? shared_levels(h, l, hi[i + 1], lo[i + 1]) : -1;
+  lev[i] = (int8_t)before;
+  if (i + 1 == n) lev[n] = -1;
+  cnt[i] = after > before ? (uint32_t)(after - before) : 0u;
 }
 
 __device__ __forceinline__ uint32_t digit_at(uint64_t hi, uint64_t lo, int depth) {
@@ -259,64 +229,93 @@ __device__ __forceinline__ uint32_t digit_at(uint64_t hi, uint64_t lo, int depth
   return depth <= 21 ? (uint32_t)((hi >> (63 - 3 * depth)) & 7u) : (uint32_t)((lo >> (63 - 3 * (depth - 21))) & 7u);
 }
 
-__global__ void k_oct_nodes(int64_t nb, const int32_t* __restrict__ bpre, const int32_t* __restrict__ bparent,
-                            const uint32_t* __restrict__ bfirst, const uint32_t* __restrict__ blast,
-                            const uint32_t* __restrict__ cnt, const uint32_t* __restrict__ base,
+// Per particle: the nodes that start there, their ranges and parents, its leaf,
+// and the child slots of all of them.
+__global__ void k_oct_nodes(int64_t n, int64_t n_int, const int8_t* __restrict__ lev, const uint64_t* __restrict__ hi,
+                            const uint64_t* __restrict__ lo, const uint32_t* __restrict__ base,
                             int32_t* __restrict__ o_parent, uint8_t* __restrict__ o_depth,
                             uint32_t* __restrict__ o_first, uint32_t* __restrict__ o_last,
+                            uint8_t* __restrict__ leaf_depth, uint32_t* __restrict__ slots,
                             uint32_t* __restrict__ max_depth) {
-  int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   uint32_t deep = 0;
-  const uint32_t c = b < nb ? cnt[b] : 0u;
-  if (c != 0) {
-    const int32_t par = bparent[b];
-    const int start = (par < 0 ? -1 : bpre[par] / 3) + 1;
-    const int32_t p0 = par < 0 ? -1 : owner_deepest(par, bparent, cnt, base);
-    const uint32_t id0 = base[b];
-    for (uint32_t k = 0; k < c; ++k) {
-      const uint32_t id = id0 + k;
-      o_parent[id] = k == 0 ? p0 : (int32_t)(id - 1);
-      o_depth[id] = (uint8_t)(start + k);
-      o_first[id] = bfirst[b];
-      o_last[id] = blast[b];
+  if (i < n) {
+    const uint64_t h = hi[i], l = lo[i];
+    const int before = lev[i], after = lev[i + 1];
+    const uint32_t id0 = base[i];
+    // the node of depth `before` that holds the particle: it starts at the
+    // nearest earlier particle that shares fewer levels with its predecessor
+    int32_t up = -1;
+    if (before >= 0) {
+      int64_t j = i - 1;
+      int scanned = 1;
+      while (lev[j] >= before && scanned < LEV_SCAN) {  // (lev[0] = -1 ends it)
+        --j;
+        ++scanned;
+      }
+      if (lev[j] >= before) {  // a wide cell: double the step, then halve it
+        int64_t in = j, out = -1;
+        for (int64_t step = LEV_SCAN; in - step >= 0; step <<= 1) {
+          if (!same_cell(hi, lo, h, l, in - step, before)) {
+            out = in - step;
+            break;
+          }
+          in -= step;
+        }
+        while (in - out > 1) {
+          const int64_t mid = out + ((in - out) >> 1);
+          if (before == 0 || same_cell(hi, lo, h, l, mid, before)) in = mid;
+          else out = mid;
+        }
+        j = in;
+      }
+      // (in range by construction; a run of ties that was refused leaves low
+      // keys in no order, and must not write outside the nodes)
+      const int64_t u = (int64_t)base[j] + (before - lev[j] - 1);
+      up = u >= 0 && u < n_int ? (int32_t)u : -1;
     }
-    deep = (uint32_t)(start + c);
+    const uint32_t c = after > before ? (uint32_t)(after - before) : 0u;
+    int64_t end = i + 2;  // first particle outside the node, deepest node first
+    int left = LEV_SCAN;
+    for (int d = after; d > before; --d) {
+      const uint32_t id = id0 + (uint32_t)(d - before - 1);
+      while (left > 0 && lev[end] >= d) {  // (lev[n] = -1 ends it)
+        ++end;
+        --left;
+      }
+      if (lev[end] >= d) {
+        int64_t in = end, out = n;
+        for (int64_t step = LEV_SCAN; in + step < n; step <<= 1) {
+          if (d > 0 && !same_cell(hi, lo, h, l, in + step, d)) {
+            out = in + step;
+            break;
+          }
+          in += step;
+        }
+        while (out - in > 1) {
+          const int64_t mid = in + ((out - in) >> 1);
+          if (d == 0 || same_cell(hi, lo, h, l, mid, d)) in = mid;
+          else out = mid;
+        }
+        end = in + 1;
+      }
+      const int32_t parent = d == before + 1 ? up : (int32_t)(id - 1);
+      o_parent[id] = parent;
+      o_depth[id] = (uint8_t)d;
+      o_first[id] = (uint32_t)i;
+      o_last[id] = (uint32_t)(end - 1);
+      if (parent >= 0) slots[(int64_t)parent * 8 + digit_at(h, l, d)] = id;
+    }
+    const int ld = (c ? after : before) + 1;
+    const int32_t lp = c ? (int32_t)(id0 + c - 1) : up;
+    leaf_depth[i] = (uint8_t)ld;
+    if (lp >= 0 && ld <= KEY_LEVELS) slots[(int64_t)lp * 8 + digit_at(h, l, ld)] = (uint32_t)i | LEAF_BIT;
+    if (c) deep = (uint32_t)(after + 1);
   }
   // deepest leaf bound: one atomic per warp (one per thread on a single
   // address serialised the kernel)
   deep = __reduce_max_sync(0xffffffffu, deep);
   if ((threadIdx.x & 31) == 0 && deep) atomicMax(max_depth, deep);
-}
-
-__global__ void k_leaf_parents(int64_t n, const int32_t* __restrict__ leaf_bparent,
-                               const int32_t* __restrict__ bparent, const uint32_t* __restrict__ cnt,
-                               const uint32_t* __restrict__ base, const uint8_t* __restrict__ o_depth,
-                               int32_t* __restrict__ leaf_oparent, uint8_t* __restrict__ leaf_depth) {
-  int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  const int32_t P = owner_deepest(leaf_bparent[p], bparent, cnt, base);
-  leaf_oparent[p] = P;
-  leaf_depth[p] = (uint8_t)(o_depth[P] + 1);
-}
-
-__global__ void k_oct_slots_nodes(int64_t n_int, const int32_t* __restrict__ o_parent,
-                                  const uint8_t* __restrict__ o_depth, const uint32_t* __restrict__ o_first,
-                                  const uint64_t* __restrict__ hi, const uint64_t* __restrict__ lo,
-                                  uint32_t* __restrict__ slots) {
-  int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (id >= n_int) return;
-  const int32_t P = o_parent[id];
-  if (P < 0) return;
-  const uint32_t f = o_first[id];
-  slots[(int64_t)P * 8 + digit_at(hi[f], lo[f], o_depth[id])] = (uint32_t)id;
-}
-
-__global__ void k_oct_slots_leaves(int64_t n, const int32_t* __restrict__ leaf_oparent,
-                                   const uint8_t* __restrict__ leaf_depth, const uint64_t* __restrict__ hi,
-                                   const uint64_t* __restrict__ lo, uint32_t* __restrict__ slots) {
-  int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  slots[(int64_t)leaf_oparent[p] * 8 + digit_at(hi[p], lo[p], leaf_depth[p])] = (uint32_t)p | LEAF_BIT;
 }
 
 __global__ void k_oct_nchild(int64_t n_int, const uint32_t* __restrict__ slots, uint32_t* __restrict__ nchild) {
@@ -836,33 +835,17 @@ void launch_permute(const Particles& src, const Particles& dst, int64_t n, const
   TPM_LAUNCH_CHECK();
 }
 
-void launch_karras(int64_t n, TreeBuffers& t, cudaStream_t s) {
+void launch_levels(int64_t n, TreeBuffers& t, cudaStream_t s) {
   if (n < 2) return;
-  k_karras<<<grid_for(n - 1, 256, 1ll << 30), 256, 0, s>>>(n, t.key_hi, t.key_lo, t.bin_left, t.bin_right,
-                                                           t.bin_prefix, t.bin_first, t.bin_last, t.bin_parent,
-                                                           t.leaf_bparent);
-  TPM_LAUNCH_CHECK();
-  k_oct_count<<<grid_for(n - 1, 256, 1ll << 30), 256, 0, s>>>(n - 1, t.bin_prefix, t.bin_parent, t.oct_count);
+  k_levels<<<grid_for(n, 256, 1ll << 30), 256, 0, s>>>(n, t.key_hi, t.key_lo, t.lev, t.oct_count);
   TPM_LAUNCH_CHECK();
 }
 
-void launch_octree_nodes(int64_t n, TreeBuffers& t, cudaStream_t s) {
-  k_oct_nodes<<<grid_for(n - 1, 256, 1ll << 30), 256, 0, s>>>(n - 1, t.bin_prefix, t.bin_parent, t.bin_first,
-                                                              t.bin_last, t.oct_count, t.oct_base, t.o_parent,
-                                                              t.o_depth, t.o_first, t.o_last, &t.scalars[2]);
-  TPM_LAUNCH_CHECK();
-  k_leaf_parents<<<grid_for(n, 256, 1ll << 30), 256, 0, s>>>(n, t.leaf_bparent, t.bin_parent, t.oct_count,
-                                                             t.oct_base, t.o_depth, t.leaf_oparent, t.leaf_depth);
-  TPM_LAUNCH_CHECK();
-}
-
-void launch_octree_links(int64_t n, int64_t n_int, TreeBuffers& t, void* scan_scratch, cudaStream_t s) {
+void launch_octree_nodes(int64_t n, int64_t n_int, TreeBuffers& t, void* scan_scratch, cudaStream_t s) {
   TPM_CUDA(cudaMemsetAsync(t.o_slots, 0xFF, (size_t)n_int * 8 * sizeof(uint32_t), s));
-  k_oct_slots_nodes<<<grid_for(n_int, 256, 1ll << 30), 256, 0, s>>>(n_int, t.o_parent, t.o_depth, t.o_first,
-                                                                    t.key_hi, t.key_lo, t.o_slots);
-  TPM_LAUNCH_CHECK();
-  k_oct_slots_leaves<<<grid_for(n, 256, 1ll << 30), 256, 0, s>>>(n, t.leaf_oparent, t.leaf_depth, t.key_hi,
-                                                                 t.key_lo, t.o_slots);
+  k_oct_nodes<<<grid_for(n, 256, 1ll << 30), 256, 0, s>>>(n, n_int, t.lev, t.key_hi, t.key_lo, t.oct_base, t.o_parent,
+                                                          t.o_depth, t.o_first, t.o_last, t.leaf_depth, t.o_slots,
+                                                          &t.scalars[2]);
   TPM_LAUNCH_CHECK();
   k_oct_nchild<<<grid_for(n_int, 256, 1ll << 30), 256, 0, s>>>(n_int, t.o_slots, t.o_nchild);
   TPM_LAUNCH_CHECK();

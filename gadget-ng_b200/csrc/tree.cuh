@@ -55,14 +55,9 @@ struct TreeBuffers {
   uint64_t* key_lo;      // by storage index before the permutation, sorted after
   uint64_t* key_lo_tmp;
   uint32_t* perm;
-  // binary radix tree over the sorted keys (n - 1 internal nodes)
-  uint32_t* bin_left;
-  uint32_t* bin_right;
-  int32_t* bin_prefix;
-  uint32_t* bin_first;
-  uint32_t* bin_last;
-  int32_t* bin_parent;
-  int32_t* leaf_bparent;
+  // octant levels shared with the previous particle (n + 1), internal nodes
+  // that start at each particle and their exclusive sums
+  int8_t* lev;
   uint32_t* oct_count;
   uint32_t* oct_base;
   // octree internal nodes
@@ -84,7 +79,6 @@ struct TreeBuffers {
   uint4* o_cell;   // relative opening criterion: fixed-point cell centre (x, y, z), |Q|_F float bits
   WalkNode* recs;  // n_int + n walk records
   // leaves
-  int32_t* leaf_oparent;
   uint8_t* leaf_depth;
   // walk groups
   uint32_t* grp_count_per_node;
@@ -106,9 +100,10 @@ void launch_bbox_root(const Particles& p, int64_t n, double box, TreeBuffers& t,
 void launch_tree_keys(const Particles& p, int64_t n, double box, TreeBuffers& t, cudaStream_t s);
 void launch_fix_ties(const Particles& p, int64_t n, double box, TreeBuffers& t, cudaStream_t s);
 void launch_permute(const Particles& src, const Particles& dst, int64_t n, const uint32_t* perm, cudaStream_t s);
-void launch_karras(int64_t n, TreeBuffers& t, cudaStream_t s);
-void launch_octree_nodes(int64_t n, TreeBuffers& t, cudaStream_t s);
-void launch_octree_links(int64_t n, int64_t n_int, TreeBuffers& t, void* scan_scratch, cudaStream_t s);
+// Levels shared by neighbours and node counts per particle (oct_count, to be
+// summed into oct_base); then the nodes with their child lists.
+void launch_levels(int64_t n, TreeBuffers& t, cudaStream_t s);
+void launch_octree_nodes(int64_t n, int64_t n_int, TreeBuffers& t, void* scan_scratch, cudaStream_t s);
 // Level-synchronous moments, deepest level first: mass and centre of mass, and
 // with_quad the quadrupole tensors too.
 // host_counts: DEPTH_BINS words of pinned host memory.

@@ -418,17 +418,9 @@ void ensure_capacity(tpm_handle* h, int64_t n) {
   T.key_lo = h->alloc<uint64_t>(c, 1);
   T.key_lo_tmp = h->alloc<uint64_t>(c, 1);
   T.perm = h->alloc<uint32_t>(c, 1);
-  const int64_t cb = c > 1 ? c - 1 : 1;
-  T.bin_left = h->alloc<uint32_t>(cb, 1);
-  T.bin_right = h->alloc<uint32_t>(cb, 1);
-  T.bin_prefix = h->alloc<int32_t>(cb, 1);
-  T.bin_first = h->alloc<uint32_t>(cb, 1);
-  T.bin_last = h->alloc<uint32_t>(cb, 1);
-  T.bin_parent = h->alloc<int32_t>(cb, 1);
-  T.oct_count = h->alloc<uint32_t>(cb, 1);
-  T.oct_base = h->alloc<uint32_t>(cb, 1);
-  T.leaf_bparent = h->alloc<int32_t>(c, 1);
-  T.leaf_oparent = h->alloc<int32_t>(c, 1);
+  T.lev = h->alloc<int8_t>(c + 1, 1);
+  T.oct_count = h->alloc<uint32_t>(c, 1);
+  T.oct_base = h->alloc<uint32_t>(c, 1);
   T.leaf_depth = h->alloc<uint8_t>(c, 1);
   h->sort_bytes = radix_sort_scratch_bytes(c);
   h->sort_scratch = h->alloc<char>(h->sort_bytes, 1);
@@ -617,16 +609,15 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
     h->n_int = 0;
     if (n >= 2) {
       TPM_CUDA(cudaMemsetAsync(T.scalars, 0, 4 * sizeof(uint32_t), s));
-      launch_karras(n, T, s);
-      exclusive_scan_u32(T.oct_count, T.oct_base, n - 1, &T.scalars[0], h->scan_scratch, s);
+      launch_levels(n, T, s);
+      exclusive_scan_u32(T.oct_count, T.oct_base, n, &T.scalars[0], h->scan_scratch, s);
       TPM_CUDA(cudaMemcpyAsync(h->back->scalars, T.scalars, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
       TPM_CUDA(cudaMemcpyAsync(&h->back->params, T.params, sizeof(TreeParams), cudaMemcpyDeviceToHost, s));
       TPM_CUDA(cudaStreamSynchronize(s));
       h->params_host = h->back->params;
       h->n_int = h->back->scalars[0];
       ensure_tree_capacity(h, h->n_int);
-      launch_octree_nodes(n, T, s);
-      launch_octree_links(n, h->n_int, T, h->scan_scratch, s);
+      launch_octree_nodes(n, h->n_int, T, h->scan_scratch, s);
       // the accurate walk's relative opening criterion reads |Q|_F and the
       // cell centres: the quadrupole pass runs only for it
       const bool rel = relative_mac(h);
