@@ -45,14 +45,15 @@ __global__ void k_hist8(const uint64_t* __restrict__ keys, int64_t n, uint32_t* 
   }
 }
 
+template <int ITEMS>
 __global__ void k_upsweep(const uint64_t* __restrict__ keys, int64_t n, int shift, int64_t ntiles,
                           uint32_t* __restrict__ tile_counts) {
   __shared__ uint32_t h[256];
   for (int i = threadIdx.x; i < 256; i += blockDim.x) h[i] = 0;
   __syncthreads();
-  int64_t base = (int64_t)blockIdx.x * SORT_TILE;
+  int64_t base = (int64_t)blockIdx.x * (SORT_BLOCK * ITEMS);
 #pragma unroll 4
-  for (int j = 0; j < SORT_ITEMS; ++j) {
+  for (int j = 0; j < ITEMS; ++j) {
     int64_t idx = base + (int64_t)j * SORT_BLOCK + threadIdx.x;
     if (idx < n) atomicAdd(&h[(keys[idx] >> shift) & 255u], 1u);
   }
@@ -61,8 +62,9 @@ __global__ void k_upsweep(const uint64_t* __restrict__ keys, int64_t n, int shif
 }
 
 // One block per digit: offsets[d][t] = base(d) + sum_{t' < t} tile_counts[d][t'].
-__global__ void k_scan_tiles(const uint32_t* __restrict__ tile_counts, const uint32_t* __restrict__ digit_hist,
-                             int64_t ntiles, uint32_t* __restrict__ offsets) {
+// In place: offsets over the counts.
+__global__ void k_scan_tiles(uint32_t* __restrict__ tile_counts, const uint32_t* __restrict__ digit_hist,
+                             int64_t ntiles) {
   __shared__ uint32_t warp_sums[32];
   __shared__ uint32_t s_base;
   const int d = blockIdx.x;
@@ -74,8 +76,7 @@ __global__ void k_scan_tiles(const uint32_t* __restrict__ tile_counts, const uin
   }
   __syncthreads();
   uint32_t carry = s_base;
-  const uint32_t* row = tile_counts + (int64_t)d * ntiles;
-  uint32_t* orow = offsets + (int64_t)d * ntiles;
+  uint32_t* row = tile_counts + (int64_t)d * ntiles;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int64_t c0 = 0; c0 < ntiles; c0 += blockDim.x) {
     int64_t i = c0 + threadIdx.x;
@@ -97,7 +98,7 @@ __global__ void k_scan_tiles(const uint32_t* __restrict__ tile_counts, const uin
     }
     __syncthreads();
     uint32_t before = (warp > 0 ? warp_sums[warp - 1] : 0u) + x - v;
-    if (i < ntiles) orow[i] = carry + before;
+    if (i < ntiles) row[i] = carry + before;
     uint32_t total = warp_sums[nw - 1];
     __syncthreads();
     carry += total;
@@ -109,14 +110,18 @@ __global__ void k_scan_tiles(const uint32_t* __restrict__ tile_counts, const uin
 // contiguous runs per digit, so consecutive threads store to consecutive
 // addresses.
 static_assert(SORT_BLOCK == 256, "the downsweep's digit scan maps one thread to one digit");
-constexpr size_t DOWNSWEEP_SMEM = (size_t)SORT_TILE * (sizeof(uint64_t) + sizeof(uint32_t)) +
-                                  (size_t)SORT_WARPS * 256 * sizeof(uint32_t) + 2 * 256 * sizeof(uint32_t);
+template <int ITEMS> constexpr size_t downsweep_smem() {
+  return (size_t)SORT_BLOCK * ITEMS * (sizeof(uint64_t) + sizeof(uint32_t)) +
+         (size_t)SORT_WARPS * 256 * sizeof(uint32_t) + 2 * 256 * sizeof(uint32_t);
+}
 
+template <int ITEMS>
 __global__ void __launch_bounds__(SORT_BLOCK) k_downsweep(const uint64_t* __restrict__ keys_in,
                                                           const uint32_t* __restrict__ vals_in,
                                                           uint64_t* __restrict__ keys_out,
                                                           uint32_t* __restrict__ vals_out, int64_t n, int shift,
                                                           int64_t ntiles, const uint32_t* __restrict__ offsets) {
+  constexpr int SORT_ITEMS = ITEMS, SORT_TILE = SORT_BLOCK * ITEMS;
   extern __shared__ __align__(16) unsigned char ds_smem[];
   uint64_t* s_k = reinterpret_cast<uint64_t*>(ds_smem);
   uint32_t* s_v = reinterpret_cast<uint32_t*>(s_k + SORT_TILE);
@@ -297,36 +302,69 @@ void sort_small(uint64_t* keys, uint32_t* vals, int64_t n, cudaStream_t s) {
 
 }  // namespace
 
+namespace {
+
+// The scratch arrays and the launches of one digit pass.
+struct Passes {
+  uint64_t* keys_alt;
+  uint32_t *vals_alt, *tiles, *hist;
+  int64_t n, ntiles;
+  int items;
+  cudaStream_t s;
+
+  Passes(int64_t n_, void* scratch, cudaStream_t s_) : n(n_), s(s_) {
+    items = sort_items(n);
+    ntiles = (n + SORT_BLOCK * items - 1) / (SORT_BLOCK * items);
+    char* p = (char*)scratch;
+    auto carve = [&](size_t bytes) {
+      char* r = p;
+      p += (bytes + 255) & ~(size_t)255;
+      return (void*)r;
+    };
+    keys_alt = (uint64_t*)carve((size_t)n * sizeof(uint64_t));
+    vals_alt = (uint32_t*)carve((size_t)n * sizeof(uint32_t));
+    tiles = (uint32_t*)carve((size_t)ntiles * 256 * sizeof(uint32_t));
+    hist = (uint32_t*)carve(8 * 256 * sizeof(uint32_t));
+  }
+  void histogram(const uint64_t* keys) const {
+    TPM_CUDA(cudaMemsetAsync(hist, 0, 8 * 256 * sizeof(uint32_t), s));
+    k_hist8<<<grid_for(n, 256, 148 * 8), 256, 0, s>>>(keys, n, hist);
+    TPM_LAUNCH_CHECK();
+  }
+  template <int ITEMS>
+  void run(const uint64_t* kin, const uint32_t* vin, uint64_t* kout, uint32_t* vout, int pass) const {
+    constexpr size_t smem = downsweep_smem<ITEMS>();
+    TPM_CUDA(cudaFuncSetAttribute(k_downsweep<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_upsweep<ITEMS><<<(unsigned)ntiles, SORT_BLOCK, 0, s>>>(kin, n, 8 * pass, ntiles, tiles);
+    TPM_LAUNCH_CHECK();
+    k_scan_tiles<<<256, ntiles <= 256 ? 256 : 1024, 0, s>>>(tiles, hist + pass * 256, ntiles);
+    TPM_LAUNCH_CHECK();
+    k_downsweep<ITEMS><<<(unsigned)ntiles, SORT_BLOCK, smem, s>>>(kin, vin, kout, vout, n, 8 * pass, ntiles, tiles);
+    TPM_LAUNCH_CHECK();
+  }
+  void operator()(const uint64_t* kin, const uint32_t* vin, uint64_t* kout, uint32_t* vout, int pass) const {
+    if (items == 2) run<2>(kin, vin, kout, vout, pass);
+    else if (items == 4) run<4>(kin, vin, kout, vout, pass);
+    else run<8>(kin, vin, kout, vout, pass);
+  }
+};
+
+}  // namespace
+
 void radix_sort_u64(uint64_t* keys, uint32_t* vals, int64_t n, int key_bits, void* scratch, size_t scratch_bytes,
                     cudaStream_t s) {
   if (n <= 1) return;
   if (scratch_bytes < radix_sort_scratch_bytes(n)) throw Error(1, "radix sort scratch too small");
-  int64_t ntiles = (n + SORT_TILE - 1) / SORT_TILE;
-  char* p = (char*)scratch;
-  auto carve = [&](size_t bytes) {
-    char* r = p;
-    p += (bytes + 255) & ~(size_t)255;
-    return (void*)r;
-  };
-  uint64_t* keys_alt = (uint64_t*)carve((size_t)n * sizeof(uint64_t));
-  uint32_t* vals_alt = (uint32_t*)carve((size_t)n * sizeof(uint32_t));
-  uint32_t* tile_counts = (uint32_t*)carve((size_t)ntiles * 256 * sizeof(uint32_t));
-  uint32_t* offsets = (uint32_t*)carve((size_t)ntiles * 256 * sizeof(uint32_t));
-  uint32_t* hist = (uint32_t*)carve(8 * 256 * sizeof(uint32_t));
-  (void)p;
-
-  TPM_CUDA(cudaFuncSetAttribute(k_downsweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DOWNSWEEP_SMEM));
-  TPM_CUDA(cudaMemsetAsync(hist, 0, 8 * 256 * sizeof(uint32_t), s));
-  k_hist8<<<grid_for(n, 256, 148 * 8), 256, 0, s>>>(keys, n, hist);
-  TPM_LAUNCH_CHECK();
+  const Passes p(n, scratch, s);
+  p.histogram(keys);
   uint32_t hh[8 * 256];
-  TPM_CUDA(cudaMemcpyAsync(hh, hist, sizeof(hh), cudaMemcpyDeviceToHost, s));
+  TPM_CUDA(cudaMemcpyAsync(hh, p.hist, sizeof(hh), cudaMemcpyDeviceToHost, s));
   TPM_CUDA(cudaStreamSynchronize(s));
 
   uint64_t* kin = keys;
   uint32_t* vin = vals;
-  uint64_t* kout = keys_alt;
-  uint32_t* vout = vals_alt;
+  uint64_t* kout = p.keys_alt;
+  uint32_t* vout = p.vals_alt;
   int npass = (key_bits + 7) / 8;
   if (npass > 8) npass = 8;
   for (int pass = 0; pass < npass; ++pass) {
@@ -334,13 +372,7 @@ void radix_sort_u64(uint64_t* keys, uint32_t* vals, int64_t n, int key_bits, voi
     for (int d = 0; d < 256; ++d)
       if (hh[pass * 256 + d] == (uint32_t)n) constant = true;
     if (constant) continue;
-    int shift = 8 * pass;
-    k_upsweep<<<(unsigned)ntiles, SORT_BLOCK, 0, s>>>(kin, n, shift, ntiles, tile_counts);
-    TPM_LAUNCH_CHECK();
-    k_scan_tiles<<<256, 1024, 0, s>>>(tile_counts, hist + pass * 256, ntiles, offsets);
-    TPM_LAUNCH_CHECK();
-    k_downsweep<<<(unsigned)ntiles, SORT_BLOCK, DOWNSWEEP_SMEM, s>>>(kin, vin, kout, vout, n, shift, ntiles, offsets);
-    TPM_LAUNCH_CHECK();
+    p(kin, vin, kout, vout, pass);
     std::swap(kin, kout);
     std::swap(vin, vout);
   }
@@ -361,34 +393,14 @@ void radix_sort_u64_all_passes(uint64_t* keys, uint32_t* vals, int64_t n, void* 
     else sort_small<8>(keys, vals, n, s);
     return;
   }
-  int64_t ntiles = (n + SORT_TILE - 1) / SORT_TILE;
-  char* p = (char*)scratch;
-  auto carve = [&](size_t bytes) {
-    char* r = p;
-    p += (bytes + 255) & ~(size_t)255;
-    return (void*)r;
-  };
-  uint64_t* keys_alt = (uint64_t*)carve((size_t)n * sizeof(uint64_t));
-  uint32_t* vals_alt = (uint32_t*)carve((size_t)n * sizeof(uint32_t));
-  uint32_t* tile_counts = (uint32_t*)carve((size_t)ntiles * 256 * sizeof(uint32_t));
-  uint32_t* offsets = (uint32_t*)carve((size_t)ntiles * 256 * sizeof(uint32_t));
-  uint32_t* hist = (uint32_t*)carve(8 * 256 * sizeof(uint32_t));
-  TPM_CUDA(cudaFuncSetAttribute(k_downsweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DOWNSWEEP_SMEM));
-  TPM_CUDA(cudaMemsetAsync(hist, 0, 8 * 256 * sizeof(uint32_t), s));
-  k_hist8<<<grid_for(n, 256, 148 * 8), 256, 0, s>>>(keys, n, hist);
-  TPM_LAUNCH_CHECK();
+  const Passes p(n, scratch, s);
+  p.histogram(keys);
   uint64_t* kin = keys;
   uint32_t* vin = vals;
-  uint64_t* kout = keys_alt;
-  uint32_t* vout = vals_alt;
+  uint64_t* kout = p.keys_alt;
+  uint32_t* vout = p.vals_alt;
   for (int pass = 0; pass < 8; ++pass) {  // eight passes: the result ends in keys / vals
-    const int shift = 8 * pass;
-    k_upsweep<<<(unsigned)ntiles, SORT_BLOCK, 0, s>>>(kin, n, shift, ntiles, tile_counts);
-    TPM_LAUNCH_CHECK();
-    k_scan_tiles<<<256, 1024, 0, s>>>(tile_counts, hist + pass * 256, ntiles, offsets);
-    TPM_LAUNCH_CHECK();
-    k_downsweep<<<(unsigned)ntiles, SORT_BLOCK, DOWNSWEEP_SMEM, s>>>(kin, vin, kout, vout, n, shift, ntiles, offsets);
-    TPM_LAUNCH_CHECK();
+    p(kin, vin, kout, vout, pass);
     std::swap(kin, kout);
     std::swap(vin, vout);
   }

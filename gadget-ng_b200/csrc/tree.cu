@@ -212,16 +212,41 @@ __device__ __forceinline__ bool same_cell(const uint64_t* __restrict__ hi, const
   return x == 0 && ((lo_i ^ __ldg(&lo[j])) >> (63 - 3 * (d - KEY_LEVELS / 2))) == 0;
 }
 
+// Also counts the nodes of each depth (hist), so that the host learns the
+// levels' sizes together with the number of nodes.
 __global__ void k_levels(int64_t n, const uint64_t* __restrict__ hi, const uint64_t* __restrict__ lo,
-                         int8_t* __restrict__ lev, uint32_t* __restrict__ cnt) {
+                         int8_t* __restrict__ lev, uint32_t* __restrict__ cnt, uint32_t* __restrict__ hist) {
+  __shared__ uint32_t sh[DEPTH_BINS];
+  if (threadIdx.x < DEPTH_BINS) sh[threadIdx.x] = 0u;
+  __syncthreads();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint64_t h = hi[i], l = lo[i];
-  const int before = i > 0 ? shared_levels(hi[i - 1], lo[i - 1], h, l) : -1;
-  const int after = i + 1 < n ? shared_levels(h, l, hi[i + 1], lo[i + 1]) : -1;
-  lev[i] = (int8_t)before;
-  if (i + 1 == n) lev[n] = -1;
-  cnt[i] = after > before ? (uint32_t)(after - before) : 0u;
+  if (i < n) {
+    const uint64_t h = hi[i], l = lo[i];
+    const int before = i > 0 ? shared_levels(hi[i - 1], lo[i - 1], h, l) : -1;
+    const int after = i + 1 < n ? shared_levels(h, l, hi[i + 1], lo[i + 1]) : -1;
+    lev[i] = (int8_t)before;
+    if (i + 1 == n) lev[n] = -1;
+    cnt[i] = after > before ? (uint32_t)(after - before) : 0u;
+    for (int d = before + 1; d <= after; ++d) atomicAdd(&sh[d], 1u);
+  }
+  __syncthreads();
+  if (threadIdx.x < DEPTH_BINS && sh[threadIdx.x]) atomicAdd(&hist[threadIdx.x], sh[threadIdx.x]);
+}
+
+// hist -> exclusive offsets (DEPTH_BINS + 1) and cursors; one warp
+__global__ void k_depth_offsets(uint32_t* tab) {
+  uint32_t* hist = tab;
+  uint32_t* off = tab + DEPTH_BINS;
+  uint32_t* cur = tab + 2 * DEPTH_BINS + 1;
+  if (threadIdx.x == 0) {
+    uint32_t acc = 0;
+    for (int d = 0; d < DEPTH_BINS; ++d) {
+      off[d] = acc;
+      cur[d] = acc;
+      acc += hist[d];
+    }
+    off[DEPTH_BINS] = acc;
+  }
 }
 
 __device__ __forceinline__ uint32_t digit_at(uint64_t hi, uint64_t lo, int depth) {
@@ -236,8 +261,22 @@ __global__ void k_oct_nodes(int64_t n, int64_t n_int, const int8_t* __restrict__
                             int32_t* __restrict__ o_parent, uint8_t* __restrict__ o_depth,
                             uint32_t* __restrict__ o_first, uint32_t* __restrict__ o_last,
                             uint8_t* __restrict__ leaf_depth, uint32_t* __restrict__ slots,
-                            uint32_t* __restrict__ max_depth) {
+                            uint32_t* __restrict__ max_depth, uint32_t* __restrict__ cursor,
+                            uint32_t* __restrict__ by_depth) {
+  // the nodes bucketed by depth for the moments: one reserved range per
+  // (block, depth); the order inside a bucket is free
+  __shared__ uint32_t here[DEPTH_BINS], start[DEPTH_BINS];
+  if (threadIdx.x < DEPTH_BINS) here[threadIdx.x] = 0u;
+  __syncthreads();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < n)
+    for (int d = lev[i] + 1; d <= lev[i + 1]; ++d) atomicAdd(&here[d], 1u);
+  __syncthreads();
+  if (threadIdx.x < DEPTH_BINS && here[threadIdx.x]) {
+    start[threadIdx.x] = atomicAdd(&cursor[threadIdx.x], here[threadIdx.x]);
+    here[threadIdx.x] = 0u;
+  }
+  __syncthreads();
   uint32_t deep = 0;
   if (i < n) {
     const uint64_t h = hi[i], l = lo[i];
@@ -300,6 +339,7 @@ __global__ void k_oct_nodes(int64_t n, int64_t n_int, const int8_t* __restrict__
         end = in + 1;
       }
       const int32_t parent = d == before + 1 ? up : (int32_t)(id - 1);
+      by_depth[start[d] + atomicAdd(&here[d], 1u)] = id;
       o_parent[id] = parent;
       o_depth[id] = (uint8_t)d;
       o_first[id] = (uint32_t)i;
@@ -316,35 +356,6 @@ __global__ void k_oct_nodes(int64_t n, int64_t n_int, const int8_t* __restrict__
   // address serialised the kernel)
   deep = __reduce_max_sync(0xffffffffu, deep);
   if ((threadIdx.x & 31) == 0 && deep) atomicMax(max_depth, deep);
-}
-
-__global__ void k_oct_nchild(int64_t n_int, const uint32_t* __restrict__ slots, uint32_t* __restrict__ nchild) {
-  int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (id >= n_int) return;
-  uint32_t c = 0;
-#pragma unroll
-  for (int s = 0; s < 8; ++s) c += slots[id * 8 + s] != EMPTY_SLOT;
-  nchild[id] = c;
-}
-
-__global__ void k_oct_childlist(int64_t n_int, const uint32_t* __restrict__ slots,
-                                const uint32_t* __restrict__ first, uint32_t* __restrict__ ids,
-                                uint8_t* __restrict__ ninner) {
-  int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (id >= n_int) return;
-  const uint32_t f = first[id];
-  uint32_t w = f;
-#pragma unroll
-  for (int s = 0; s < 8; ++s) {  // internal children first (EMPTY_SLOT has the leaf bit)
-    const uint32_t c = slots[id * 8 + s];
-    if (!(c & LEAF_BIT)) ids[w++] = c;
-  }
-  ninner[id] = (uint8_t)(w - f);
-#pragma unroll
-  for (int s = 0; s < 8; ++s) {
-    const uint32_t c = slots[id * 8 + s];
-    if ((c & LEAF_BIT) && c != EMPTY_SLOT) ids[w++] = c;
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -369,52 +380,6 @@ __device__ __forceinline__ void child_moments(uint32_t c, double scale, const ui
   }
 }
 
-// Internal nodes by depth: per-block histograms, then one reserved range per
-// (block, depth) into the depth buckets (the order inside a bucket is free).
-__global__ void k_depth_count(int64_t n_int, const uint8_t* __restrict__ o_depth, uint32_t* __restrict__ hist) {
-  __shared__ uint32_t sh[DEPTH_BINS];
-  if (threadIdx.x < DEPTH_BINS) sh[threadIdx.x] = 0u;
-  __syncthreads();
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < n_int) atomicAdd(&sh[o_depth[i] & (DEPTH_BINS - 1)], 1u);
-  __syncthreads();
-  if (threadIdx.x < DEPTH_BINS && sh[threadIdx.x]) atomicAdd(&hist[threadIdx.x], sh[threadIdx.x]);
-}
-
-// hist -> exclusive offsets (DEPTH_BINS + 1) and cursors; one warp
-__global__ void k_depth_offsets(uint32_t* tab) {
-  uint32_t* hist = tab;
-  uint32_t* off = tab + DEPTH_BINS;
-  uint32_t* cur = tab + 2 * DEPTH_BINS + 1;
-  if (threadIdx.x == 0) {
-    uint32_t acc = 0;
-    for (int d = 0; d < DEPTH_BINS; ++d) {
-      off[d] = acc;
-      cur[d] = acc;
-      acc += hist[d];
-    }
-    off[DEPTH_BINS] = acc;
-  }
-}
-
-__global__ void k_depth_scatter(int64_t n_int, const uint8_t* __restrict__ o_depth, uint32_t* __restrict__ cur,
-                                uint32_t* __restrict__ by_depth) {
-  __shared__ uint32_t cnt[DEPTH_BINS], base[DEPTH_BINS];
-  if (threadIdx.x < DEPTH_BINS) cnt[threadIdx.x] = 0u;
-  __syncthreads();
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  int d = 0;
-  uint32_t r = 0;
-  if (i < n_int) {
-    d = o_depth[i] & (DEPTH_BINS - 1);
-    r = atomicAdd(&cnt[d], 1u);
-  }
-  __syncthreads();
-  if (threadIdx.x < DEPTH_BINS && cnt[threadIdx.x]) base[threadIdx.x] = atomicAdd(&cur[threadIdx.x], cnt[threadIdx.x]);
-  __syncthreads();
-  if (i < n_int) by_depth[base[d] + r] = (uint32_t)i;
-}
-
 // Moments of the internal nodes at one depth (octree.rs:547-629) from their
 // children, which are leaves or nodes one level deeper (finished by the
 // previous launch): mass and centre of mass summed over the children in
@@ -422,19 +387,22 @@ __global__ void k_depth_scatter(int64_t n_int, const uint8_t* __restrict__ o_dep
 // (outer_traceless :197-207), all float64 in the reference's operation order.
 // QUAD: also the quadrupole tensors (the walk reads mass and centre of mass
 // only; the quadrupoles are made when the tree is exported).
+// Returns the number of children.
 template <bool QUAD>
-__device__ __forceinline__ void aggregate_node(uint32_t P, double scale, const uint32_t* __restrict__ qx,
+__device__ __forceinline__ uint32_t aggregate_node(uint32_t P, double scale, const uint32_t* __restrict__ qx,
                                                const uint32_t* __restrict__ qy, const uint32_t* __restrict__ qz,
                                                const double* __restrict__ pmass, const uint32_t* __restrict__ slots,
-                                               double* o_mass, double* o_com, double* o_quad) {
+                                               double* o_mass, double* o_com, double* o_quad, double inv_scale,
+                                               uint4* __restrict__ walk, uint8_t* __restrict__ kids) {
   // pass 1: mass and centre of mass over the children in octant order
-  uint32_t cs[8];
+  uint32_t cs[8], nk = 0;  // children, internal ones in the high half byte
   double mt = 0.0, ax = 0.0, ay = 0.0, az = 0.0;
 #pragma unroll
   for (int s = 0; s < 8; ++s) {
     const uint32_t c = slots[(int64_t)P * 8 + s];
     cs[s] = c;
     if (c == EMPTY_SLOT) continue;
+    nk += (c & LEAF_BIT) ? 1u : 17u;
     double m, x, y, z;
     child_moments(c, scale, qx, qy, qz, pmass, o_mass, o_com, &m, &x, &y, &z);
     mt = dadd(mt, m);
@@ -448,12 +416,20 @@ __device__ __forceinline__ void aggregate_node(uint32_t P, double scale, const u
     comy = ddiv(ay, mt);
     comz = ddiv(az, mt);
   }
+  kids[P] = (uint8_t)nk;
+  {  // the walk's fixed-point centre of mass (in [0, 2^32]) and float mass
+    const double v[3] = {comx, comy, comz};
+    uint32_t q[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) q[d] = (uint32_t)((unsigned long long)llrint(v[d] * inv_scale) & 0xFFFFFFFFull);
+    walk[P] = make_uint4(q[0], q[1], q[2], __float_as_uint((float)mt));
+  }
   if (!QUAD) {
     __stcg(&o_mass[P], mt);
     __stcg(&o_com[3 * (int64_t)P], comx);
     __stcg(&o_com[3 * (int64_t)P + 1], comy);
     __stcg(&o_com[3 * (int64_t)P + 2], comz);
-    return;
+    return nk & 15u;
   }
   // pass 2: the children are read again (cache hits) rather than held in registers
   double qd[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
@@ -488,67 +464,70 @@ __device__ __forceinline__ void aggregate_node(uint32_t P, double scale, const u
   __stcg(&o_com[3 * (int64_t)P + 2], comz);
 #pragma unroll
   for (int k = 0; k < 6; ++k) __stcg(&o_quad[6 * (int64_t)P + k], qd[k]);
+  return nk & 15u;
+}
+
+// Space for the walk records of this lane's node (nk children, 0: none), one
+// atomic per warp: the ranges need no order among the nodes, so no prefix sum.
+// All lanes of the warp call it.
+__device__ __forceinline__ void reserve_children(bool live, uint32_t P, uint32_t nk, uint32_t* total,
+                                                 uint32_t* __restrict__ child_first) {
+  const int lane = threadIdx.x & 31;
+  if (!live) nk = 0u;
+  uint32_t x = nk;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  uint32_t base = 0;
+  if (lane == 31 && x) base = atomicAdd(total, x);
+  base = __shfl_sync(0xffffffffu, base, 31);
+  if (live) child_first[P] = base + x - nk;
 }
 
 template <bool QUAD>
 __global__ void k_aggregate_level(const uint32_t* __restrict__ nodes, int64_t count, double scale,
                                   const uint32_t* __restrict__ qx, const uint32_t* __restrict__ qy,
                                   const uint32_t* __restrict__ qz, const double* __restrict__ pmass,
-                                  const uint32_t* __restrict__ slots, double* o_mass, double* o_com, double* o_quad) {
+                                  const uint32_t* __restrict__ slots, double* o_mass, double* o_com, double* o_quad,
+                                  double inv_scale, uint4* __restrict__ walk, uint8_t* __restrict__ kids,
+                                  uint32_t* total, uint32_t* __restrict__ child_first) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < count) aggregate_node<QUAD>(nodes[i], scale, qx, qy, qz, pmass, slots, o_mass, o_com, o_quad);
+  const bool live = i < count;
+  const uint32_t P = live ? nodes[i] : 0u;
+  uint32_t nk = 0u;
+  if (live) nk = aggregate_node<QUAD>(P, scale, qx, qy, qz, pmass, slots, o_mass, o_com, o_quad, inv_scale, walk, kids);
+  if (total) reserve_children(live, P, nk, total, child_first);
 }
 
-// Small trees in one block: the nodes bucketed by depth, then every level from
-// the deepest up with a block barrier between levels, in place of three
-// bucketing launches, one host synchronisation and one launch per depth.
+// Small trees in one block: every level from the deepest up with a block
+// barrier between levels, in place of one launch per depth.
 constexpr int AGG_SMALL_THREADS = 512;
 template <bool QUAD>
 __global__ void __launch_bounds__(AGG_SMALL_THREADS)
-    k_aggregate_small(int n_int, const uint8_t* __restrict__ o_depth, uint32_t* by_depth, double scale,
+    k_aggregate_small(const uint32_t* __restrict__ off, const uint32_t* __restrict__ by_depth, double scale,
                       const uint32_t* __restrict__ qx, const uint32_t* __restrict__ qy, const uint32_t* __restrict__ qz,
                       const double* __restrict__ pmass, const uint32_t* __restrict__ slots, double* o_mass,
-                      double* o_com, double* o_quad) {
-  __shared__ uint32_t off[DEPTH_BINS + 1], cur[DEPTH_BINS];
-  if (threadIdx.x < DEPTH_BINS) cur[threadIdx.x] = 0u;
-  __syncthreads();
-  for (int i = threadIdx.x; i < n_int; i += AGG_SMALL_THREADS) atomicAdd(&cur[o_depth[i] & (DEPTH_BINS - 1)], 1u);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t acc = 0;
-    for (int d = 0; d < DEPTH_BINS; ++d) {
-      off[d] = acc;
-      acc += cur[d];
-      cur[d] = off[d];
-    }
-    off[DEPTH_BINS] = acc;
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < n_int; i += AGG_SMALL_THREADS)
-    by_depth[atomicAdd(&cur[o_depth[i] & (DEPTH_BINS - 1)], 1u)] = (uint32_t)i;
+                      double* o_com, double* o_quad, double inv_scale, uint4* __restrict__ walk,
+                      uint8_t* __restrict__ kids, uint32_t* total, uint32_t* __restrict__ child_first) {
   for (int d = DEPTH_BINS - 1; d >= 0; --d) {
     if (off[d] == off[d + 1]) continue;  // the same for the whole block
-    __syncthreads();  // the bucketing, then the deeper level
-    for (uint32_t i = off[d] + threadIdx.x; i < off[d + 1]; i += AGG_SMALL_THREADS)
-      aggregate_node<QUAD>(by_depth[i], scale, qx, qy, qz, pmass, slots, o_mass, o_com, o_quad);
+    const uint32_t end = off[d + 1];
+    for (uint32_t i0 = off[d]; i0 < end; i0 += AGG_SMALL_THREADS) {
+      const uint32_t i = i0 + threadIdx.x;
+      const bool live = i < end;
+      const uint32_t P = live ? by_depth[i] : 0u;
+      uint32_t nk = 0u;
+      if (live)
+        nk = aggregate_node<QUAD>(P, scale, qx, qy, qz, pmass, slots, o_mass, o_com, o_quad, inv_scale, walk, kids);
+      if (total) reserve_children(live, P, nk, total, child_first);
+    }
+    __syncthreads();
   }
 }
 
 // Up to here one block is faster than the launches per level.
 constexpr int64_t AGG_SMALL_MAX = 8192;
-
-__global__ void k_walk_nodes(int64_t n_int, double inv_scale, const double* __restrict__ o_mass,
-                             const double* __restrict__ o_com, uint4* __restrict__ walk) {
-  int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (id >= n_int) return;
-  uint32_t q[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    double v = o_com[3 * id + d] * inv_scale;  // in [0, 2^32]
-    q[d] = (uint32_t)((unsigned long long)llrint(v) & 0xFFFFFFFFull);
-  }
-  walk[id] = make_uint4(q[0], q[1], q[2], __float_as_uint((float)o_mass[id]));
-}
 
 // Cell centre and |Q|_F of each internal node (relative opening criterion).
 // The node's octant path is the first `depth` digits of any of its particles'
@@ -589,17 +568,43 @@ __global__ void k_cell_q(int64_t n_int, double inv_scale, const TreeParams* __re
 // ---------------------------------------------------------------------------
 // walk records: children of each internal node contiguous
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ WalkNode make_record(uint32_t c, const uint32_t* __restrict__ qx,
-                                                const uint32_t* __restrict__ qy, const uint32_t* __restrict__ qz,
-                                                const float* __restrict__ massf, const uint8_t* __restrict__ leaf_depth,
-                                                const uint4* __restrict__ walk, const uint8_t* __restrict__ o_depth,
-                                                const uint32_t* __restrict__ nchild,
-                                                const uint32_t* __restrict__ child_first,
-                                                const uint8_t* __restrict__ ninner) {
-  WalkNode r;
-  r.pad = 0;
-  if (c & LEAF_BIT) {
-    const uint32_t j = c & ~LEAF_BIT;
+// One thread per node gathers its children's records, internal ones first, into
+// the node's range (1 + child_first[P] onward; the root's own record is number 0).
+__global__ void k_walk_records(int64_t n_int, const uint32_t* __restrict__ qx, const uint32_t* __restrict__ qy,
+                               const uint32_t* __restrict__ qz, const float* __restrict__ massf,
+                               const uint8_t* __restrict__ leaf_depth, const uint4* __restrict__ walk,
+                               const uint8_t* __restrict__ o_depth, const uint8_t* __restrict__ kids,
+                               const uint32_t* __restrict__ child_first, const uint32_t* __restrict__ slots,
+                               WalkNode* __restrict__ recs) {
+  const int64_t P = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (P >= n_int) return;
+  auto internal = [&](uint32_t c) {
+    const uint4 w = walk[c];
+    const uint32_t k = kids[c];
+    WalkNode r;
+    r.cq[0] = w.x;
+    r.cq[1] = w.y;
+    r.cq[2] = w.z;
+    r.mass = __uint_as_float(w.w);
+    r.first = 1u + child_first[c];
+    r.info = (k & 15u) | ((uint32_t)o_depth[c] << 4) | ((k >> 4) << 12);
+    r.ref = c;
+    r.pad = 0;
+    return r;
+  };
+  if (P == 0) recs[0] = internal(0u);
+  WalkNode* out = recs + 1 + (int64_t)child_first[P];
+  uint32_t cs[8];
+#pragma unroll
+  for (int s = 0; s < 8; ++s) {
+    cs[s] = slots[P * 8 + s];
+    if (!(cs[s] & LEAF_BIT)) *out++ = internal(cs[s]);  // (EMPTY_SLOT has the leaf bit)
+  }
+#pragma unroll
+  for (int s = 0; s < 8; ++s) {
+    if (!(cs[s] & LEAF_BIT) || cs[s] == EMPTY_SLOT) continue;
+    const uint32_t j = cs[s] & ~LEAF_BIT;
+    WalkNode r;
     r.cq[0] = qx[j];
     r.cq[1] = qy[j];
     r.cq[2] = qz[j];
@@ -607,32 +612,9 @@ __device__ __forceinline__ WalkNode make_record(uint32_t c, const uint32_t* __re
     r.first = 0;
     r.info = ((uint32_t)leaf_depth[j] << 4) | WN_LEAF;
     r.ref = j;
-  } else {
-    const uint4 w = walk[c];
-    r.cq[0] = w.x;
-    r.cq[1] = w.y;
-    r.cq[2] = w.z;
-    r.mass = __uint_as_float(w.w);
-    r.first = 1u + child_first[c];
-    r.info = nchild[c] | ((uint32_t)o_depth[c] << 4) | ((uint32_t)ninner[c] << 12);
-    r.ref = c;
+    r.pad = 0;
+    *out++ = r;
   }
-  return r;
-}
-
-__global__ void k_walk_records(int64_t n_int, const uint32_t* __restrict__ qx, const uint32_t* __restrict__ qy,
-                               const uint32_t* __restrict__ qz, const float* __restrict__ massf,
-                               const uint8_t* __restrict__ leaf_depth, const uint4* __restrict__ walk,
-                               const uint8_t* __restrict__ o_depth, const uint32_t* __restrict__ nchild,
-                               const uint32_t* __restrict__ child_first, const uint32_t* __restrict__ child_ids,
-                               const uint8_t* __restrict__ ninner, WalkNode* __restrict__ recs) {
-  int64_t P = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (P >= n_int) return;
-  if (P == 0) recs[0] = make_record(0u, qx, qy, qz, massf, leaf_depth, walk, o_depth, nchild, child_first, ninner);
-  const uint32_t f = child_first[P], nc = nchild[P];
-  for (uint32_t r = 0; r < nc; ++r)
-    recs[1 + (int64_t)f + r] =
-        make_record(child_ids[f + r], qx, qy, qz, massf, leaf_depth, walk, o_depth, nchild, child_first, ninner);
 }
 
 // ---------------------------------------------------------------------------
@@ -648,49 +630,73 @@ __device__ __forceinline__ uint32_t child_first_particle(uint32_t c, const uint3
   return (c & LEAF_BIT) ? (c & ~LEAF_BIT) : o_first[c];
 }
 
-template <bool WRITE>
+// Two looks at the children of a node, the first to count its groups.  RESERVE:
+// a warp takes the slots of its nodes' groups at once, so the groups come nearly
+// in the order of the nodes.  COUNT and WRITE: the slots are a prefix sum in node
+// order, made between two launches; neighbouring groups then walk at the same
+// time, which is worth more in large boxes (walk of 256^3 40.7 -> 40.5 ms, accurate
+// 128^3 7.55 -> 7.47) than the four launches it costs (12 us).
+constexpr int64_t GROUPS_RESERVE_MAX = 262144;
+enum { GROUPS_RESERVE = 0, GROUPS_COUNT = 1, GROUPS_WRITE = 2 };
+template <int MODE>
 __global__ void k_groups(int64_t n_int, int group_max, int pack_depth, const uint8_t* __restrict__ o_depth,
                          const uint32_t* __restrict__ slots, const uint32_t* __restrict__ o_first,
-                         const uint32_t* __restrict__ o_last,
-                         uint32_t* __restrict__ counts, const uint32_t* __restrict__ base,
-                         uint32_t* __restrict__ gfirst, uint32_t* __restrict__ gsize) {
-  int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (id >= n_int) return;
-  const uint32_t mine = o_last[id] - o_first[id] + 1u;
-  uint32_t ng = 0, w = WRITE ? base[id] : 0u;
-  const int dep = o_depth[id];
-  if (mine > (uint32_t)group_max || dep < pack_depth) {
-    const uint32_t pack_max = dep < pack_depth ? 0u : (uint32_t)group_max;
-    uint32_t run_first = 0, run_n = 0;
-    for (int s = 0; s < 8; ++s) {
-      const uint32_t c = slots[id * 8 + s];
-      if (c == EMPTY_SLOT) continue;
-      const uint32_t k = child_count(c, o_first, o_last);
-      if (k > (uint32_t)group_max || (k > 1u && dep + 1 < pack_depth)) {
-        if (run_n) {
-          if (WRITE) { gfirst[w] = run_first; gsize[w] = run_n; ++w; }
-          ++ng;
+                         const uint32_t* __restrict__ o_last, uint32_t* __restrict__ count,
+                         uint32_t* __restrict__ per_node, uint32_t* __restrict__ gfirst,
+                         uint32_t* __restrict__ gsize) {
+  const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const bool live = id < n_int;
+  const uint32_t mine = live ? o_last[id] - o_first[id] + 1u : 0u;
+  const int dep = live ? o_depth[id] : 0;
+  const bool split = live && (mine > (uint32_t)group_max || dep < pack_depth);
+  const bool whole = live && !split && id == 0;  // the whole tree fits in one group
+  uint32_t w = MODE == GROUPS_WRITE && live ? per_node[id] : 0u;
+  for (int pass = MODE == GROUPS_WRITE ? 1 : 0; pass < 2; ++pass) {
+    uint32_t ng = 0;
+    auto emit = [&](uint32_t first, uint32_t n) {
+      if (pass) {
+        gfirst[w + ng] = first;
+        gsize[w + ng] = n;
+      }
+      ++ng;
+    };
+    if (split) {
+      const uint32_t pack_max = dep < pack_depth ? 0u : (uint32_t)group_max;
+      uint32_t run_first = 0, run_n = 0;
+      for (int s = 0; s < 8; ++s) {
+        const uint32_t c = slots[id * 8 + s];
+        if (c == EMPTY_SLOT) continue;
+        const uint32_t k = child_count(c, o_first, o_last);
+        const bool apart = k > (uint32_t)group_max || (k > 1u && dep + 1 < pack_depth);
+        if (run_n && (apart || run_n + k > pack_max)) {
+          emit(run_first, run_n);
           run_n = 0;
         }
-        continue;
+        if (apart) continue;
+        if (!run_n) run_first = child_first_particle(c, o_first);
+        run_n += k;
       }
-      if (run_n && run_n + k > pack_max) {
-        if (WRITE) { gfirst[w] = run_first; gsize[w] = run_n; ++w; }
-        ++ng;
-        run_n = 0;
+      if (run_n) emit(run_first, run_n);
+    } else if (whole) {
+      emit(o_first[0], mine);
+    }
+    if (MODE == GROUPS_COUNT) {
+      if (live) per_node[id] = ng;
+      return;
+    }
+    if (pass == 0) {
+      const int lane = threadIdx.x & 31;
+      uint32_t x = ng;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
       }
-      if (!run_n) run_first = child_first_particle(c, o_first);
-      run_n += k;
+      uint32_t base = 0;
+      if (lane == 31 && x) base = atomicAdd(count, x);
+      w = __shfl_sync(0xffffffffu, base, 31) + x - ng;
+      if (!__any_sync(0xffffffffu, ng != 0u)) return;
     }
-    if (run_n) {
-      if (WRITE) { gfirst[w] = run_first; gsize[w] = run_n; ++w; }
-      ++ng;
-    }
-  } else if (id == 0) {  // the whole tree fits in one group
-    if (WRITE) { gfirst[w] = o_first[0]; gsize[w] = mine; }
-    ng = 1;
   }
-  if (!WRITE) counts[id] = ng;
 }
 
 // ---------------------------------------------------------------------------
@@ -837,74 +843,50 @@ void launch_permute(const Particles& src, const Particles& dst, int64_t n, const
 
 void launch_levels(int64_t n, TreeBuffers& t, cudaStream_t s) {
   if (n < 2) return;
-  k_levels<<<grid_for(n, 256, 1ll << 30), 256, 0, s>>>(n, t.key_hi, t.key_lo, t.lev, t.oct_count);
+  TPM_CUDA(cudaMemsetAsync(t.depth_tab, 0, DEPTH_BINS * sizeof(uint32_t), s));
+  k_levels<<<grid_for(n, 256, 1ll << 30), 256, 0, s>>>(n, t.key_hi, t.key_lo, t.lev, t.oct_count, t.depth_tab);
+  TPM_LAUNCH_CHECK();
+  k_depth_offsets<<<1, 32, 0, s>>>(t.depth_tab);
   TPM_LAUNCH_CHECK();
 }
 
-void launch_octree_nodes(int64_t n, int64_t n_int, TreeBuffers& t, void* scan_scratch, cudaStream_t s) {
+void launch_octree_nodes(int64_t n, int64_t n_int, TreeBuffers& t, cudaStream_t s) {
   TPM_CUDA(cudaMemsetAsync(t.o_slots, 0xFF, (size_t)n_int * 8 * sizeof(uint32_t), s));
   k_oct_nodes<<<grid_for(n, 256, 1ll << 30), 256, 0, s>>>(n, n_int, t.lev, t.key_hi, t.key_lo, t.oct_base, t.o_parent,
                                                           t.o_depth, t.o_first, t.o_last, t.leaf_depth, t.o_slots,
-                                                          &t.scalars[2]);
-  TPM_LAUNCH_CHECK();
-  k_oct_nchild<<<grid_for(n_int, 256, 1ll << 30), 256, 0, s>>>(n_int, t.o_slots, t.o_nchild);
-  TPM_LAUNCH_CHECK();
-  exclusive_scan_u32(t.o_nchild, t.o_child_first, n_int, &t.scalars[3], scan_scratch, s);
-  k_oct_childlist<<<grid_for(n_int, 256, 1ll << 30), 256, 0, s>>>(n_int, t.o_slots, t.o_child_first, t.child_ids,
-                                                                  t.o_ninner);
+                                                          &t.scalars[2], t.depth_tab + 2 * DEPTH_BINS + 1, t.o_cnt);
   TPM_LAUNCH_CHECK();
 }
 
 // Level by level from the deepest internal nodes to the root: each launch
 // finishes one depth, so every node reads finished children without atomics
-// or fences.  One host synchronisation brings the per-depth counts back.
-void launch_aggregate(const Particles& p, int64_t n, int64_t n_int, double box, TreeBuffers& t, uint32_t* host_counts,
-                      cudaStream_t s, bool with_quad) {
+// or fences.
+void launch_aggregate(const Particles& p, int64_t n, int64_t n_int, double box, TreeBuffers& t, const uint32_t* counts,
+                      cudaStream_t s, bool with_quad, bool records) {
   (void)n;
   if (n_int <= 0) return;
+  const double scale = box / TWO32, inv_scale = TWO32 / box;
+  uint32_t* total = records ? &t.scalars[3] : nullptr;  // zero since the node count was made
   if (n_int <= AGG_SMALL_MAX) {
-    if (with_quad)
-      k_aggregate_small<true><<<1, AGG_SMALL_THREADS, 0, s>>>((int)n_int, t.o_depth, t.o_cnt, box / TWO32, p.qx, p.qy,
-                                                              p.qz, p.mass, t.o_slots, t.o_mass, t.o_com, t.o_quad);
-    else
-      k_aggregate_small<false><<<1, AGG_SMALL_THREADS, 0, s>>>((int)n_int, t.o_depth, t.o_cnt, box / TWO32, p.qx,
-                                                               p.qy, p.qz, p.mass, t.o_slots, t.o_mass, t.o_com,
-                                                               t.o_quad);
-    TPM_LAUNCH_CHECK();
-    k_walk_nodes<<<grid_for(n_int, 256, 1ll << 30), 256, 0, s>>>(n_int, TWO32 / box, t.o_mass, t.o_com, t.o_walk);
+    auto k = with_quad ? k_aggregate_small<true> : k_aggregate_small<false>;
+    k<<<1, AGG_SMALL_THREADS, 0, s>>>(t.depth_tab + DEPTH_BINS, t.o_cnt, scale, p.qx, p.qy, p.qz, p.mass, t.o_slots,
+                                      t.o_mass, t.o_com, t.o_quad, inv_scale, t.o_walk, t.o_kids, total,
+                                      t.o_child_first);
     TPM_LAUNCH_CHECK();
     return;
   }
-  uint32_t* hist = t.depth_tab;
-  TPM_CUDA(cudaMemsetAsync(hist, 0, DEPTH_BINS * sizeof(uint32_t), s));
-  k_depth_count<<<grid_for(n_int, 256, 1ll << 30), 256, 0, s>>>(n_int, t.o_depth, hist);
-  TPM_LAUNCH_CHECK();
-  k_depth_offsets<<<1, 32, 0, s>>>(t.depth_tab);
-  TPM_LAUNCH_CHECK();
-  const uint32_t* counts = host_counts;
-  TPM_CUDA(cudaMemcpyAsync(host_counts, hist, DEPTH_BINS * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  k_depth_scatter<<<grid_for(n_int, 256, 1ll << 30), 256, 0, s>>>(n_int, t.o_depth, t.depth_tab + 2 * DEPTH_BINS + 1,
-                                                                   t.o_cnt);
-  TPM_LAUNCH_CHECK();
-  TPM_CUDA(cudaStreamSynchronize(s));
   int64_t offset[DEPTH_BINS + 1];
   offset[0] = 0;
   for (int d = 0; d < DEPTH_BINS; ++d) offset[d + 1] = offset[d] + counts[d];
   if (offset[DEPTH_BINS] != n_int) throw Error(2, "octree depth buckets do not add up to the node count");
+  auto k = with_quad ? k_aggregate_level<true> : k_aggregate_level<false>;
   for (int d = DEPTH_BINS - 1; d >= 0; --d) {
     if (counts[d] == 0) continue;
-    if (with_quad)
-      k_aggregate_level<true><<<grid_for(counts[d], 128, 1ll << 30), 128, 0, s>>>(
-          t.o_cnt + offset[d], counts[d], box / TWO32, p.qx, p.qy, p.qz, p.mass, t.o_slots, t.o_mass, t.o_com,
-          t.o_quad);
-    else
-      k_aggregate_level<false><<<grid_for(counts[d], 128, 1ll << 30), 128, 0, s>>>(
-          t.o_cnt + offset[d], counts[d], box / TWO32, p.qx, p.qy, p.qz, p.mass, t.o_slots, t.o_mass, t.o_com,
-          t.o_quad);
+    k<<<grid_for(counts[d], 128, 1ll << 30), 128, 0, s>>>(t.o_cnt + offset[d], counts[d], scale, p.qx, p.qy, p.qz,
+                                                          p.mass, t.o_slots, t.o_mass, t.o_com, t.o_quad, inv_scale,
+                                                          t.o_walk, t.o_kids, total, t.o_child_first);
     TPM_LAUNCH_CHECK();
   }
-  k_walk_nodes<<<grid_for(n_int, 256, 1ll << 30), 256, 0, s>>>(n_int, TWO32 / box, t.o_mass, t.o_com, t.o_walk);
-  TPM_LAUNCH_CHECK();
 }
 
 void launch_cell_q(int64_t n_int, double box, TreeBuffers& t, cudaStream_t s) {
@@ -914,26 +896,29 @@ void launch_cell_q(int64_t n_int, double box, TreeBuffers& t, cudaStream_t s) {
   TPM_LAUNCH_CHECK();
 }
 
-void launch_walk_records(const Particles& p, int64_t n, int64_t n_int, TreeBuffers& t, cudaStream_t s) {
-  (void)n;
+void launch_walk_records(const Particles& p, int64_t n_int, TreeBuffers& t, cudaStream_t s) {
   k_walk_records<<<grid_for(n_int, 128, 1ll << 30), 128, 0, s>>>(n_int, p.qx, p.qy, p.qz, p.massf, t.leaf_depth,
-                                                                 t.o_walk, t.o_depth, t.o_nchild, t.o_child_first,
-                                                                 t.child_ids, t.o_ninner, t.recs);
+                                                                 t.o_walk, t.o_depth, t.o_kids, t.o_child_first,
+                                                                 t.o_slots, t.recs);
   TPM_LAUNCH_CHECK();
 }
 
-void launch_groups(int64_t n, int64_t n_int, int group_max, int pack_depth, TreeBuffers& t, void* scan_scratch,
-                   cudaStream_t s) {
-  (void)n;
-  k_groups<false><<<grid_for(n_int, 256, 1ll << 30), 256, 0, s>>>(
-      n_int, group_max, pack_depth, t.o_depth, t.o_slots, t.o_first, t.o_last, t.grp_count_per_node, nullptr, nullptr,
-      nullptr);
-  TPM_LAUNCH_CHECK();
-  exclusive_scan_u32(t.grp_count_per_node, t.grp_base, n_int, &t.scalars[1], scan_scratch, s);
-  k_groups<true><<<grid_for(n_int, 256, 1ll << 30), 256, 0, s>>>(
-      n_int, group_max, pack_depth, t.o_depth, t.o_slots, t.o_first, t.o_last, nullptr, t.grp_base, t.grp_first,
-      t.grp_size);
-  TPM_LAUNCH_CHECK();
+void launch_groups(int64_t n_int, int group_max, int pack_depth, TreeBuffers& t, void* scan_scratch, cudaStream_t s) {
+  const unsigned grid = grid_for(n_int, 256, 1ll << 30);
+  auto run = [&](auto k) {
+    k<<<grid, 256, 0, s>>>(n_int, group_max, pack_depth, t.o_depth, t.o_slots, t.o_first, t.o_last, &t.scalars[1],
+                           t.grp_base, t.grp_first, t.grp_size);
+    TPM_LAUNCH_CHECK();
+  };
+  // (the sum's scratch covers four entries per particle: a tree of chains, with
+  // more nodes than that, reserves too)
+  if (n_int <= GROUPS_RESERVE_MAX || n_int > 4 * (t.cap_groups - 1)) {
+    run(k_groups<GROUPS_RESERVE>);
+    return;
+  }
+  run(k_groups<GROUPS_COUNT>);
+  exclusive_scan_u32(t.grp_base, t.grp_base, n_int, &t.scalars[1], scan_scratch, s);
+  run(k_groups<GROUPS_WRITE>);
 }
 
 void launch_hilbert_keys(const Particles& p, int64_t n, double box, const TreeParams* prm, uint64_t* keys,

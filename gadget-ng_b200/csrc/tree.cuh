@@ -67,11 +67,9 @@ struct TreeBuffers {
   uint32_t* o_first;
   uint32_t* o_last;
   uint32_t* o_slots;  // 8 per node, EMPTY_SLOT or child id (LEAF_BIT | particle)
-  uint32_t* o_nchild;
-  uint32_t* o_child_first;
   uint32_t* o_cnt;      // internal node ids bucketed by depth (aggregation order)
-  uint8_t* o_ninner;    // internal children
-  uint32_t* child_ids;  // compacted (internal children, then leaves), same encoding as o_slots
+  uint32_t* o_child_first;  // start of the node's range of walk records
+  uint8_t* o_kids;      // children (low half byte), internal ones (high half byte)
   double* o_mass;
   double* o_com;   // 3 per node
   double* o_quad;  // 6 per node
@@ -81,7 +79,6 @@ struct TreeBuffers {
   // leaves
   uint8_t* leaf_depth;
   // walk groups
-  uint32_t* grp_count_per_node;
   uint32_t* grp_base;
   uint32_t* grp_first;
   uint32_t* grp_size;
@@ -100,16 +97,19 @@ void launch_bbox_root(const Particles& p, int64_t n, double box, TreeBuffers& t,
 void launch_tree_keys(const Particles& p, int64_t n, double box, TreeBuffers& t, cudaStream_t s);
 void launch_fix_ties(const Particles& p, int64_t n, double box, TreeBuffers& t, cudaStream_t s);
 void launch_permute(const Particles& src, const Particles& dst, int64_t n, const uint32_t* perm, cudaStream_t s);
-// Levels shared by neighbours and node counts per particle (oct_count, to be
-// summed into oct_base); then the nodes with their child lists.
+// Levels shared by neighbours, node counts per particle (oct_count, to be
+// summed into oct_base) and per depth (depth_tab); then the nodes, bucketed by
+// depth as well.
 void launch_levels(int64_t n, TreeBuffers& t, cudaStream_t s);
-void launch_octree_nodes(int64_t n, int64_t n_int, TreeBuffers& t, void* scan_scratch, cudaStream_t s);
+void launch_octree_nodes(int64_t n, int64_t n_int, TreeBuffers& t, cudaStream_t s);
 // Level-synchronous moments, deepest level first: mass and centre of mass, and
 // with_quad the quadrupole tensors too.
-// host_counts: DEPTH_BINS words of pinned host memory.
-void launch_aggregate(const Particles& p, int64_t n, int64_t n_int, double box, TreeBuffers& t, uint32_t* host_counts,
-                      cudaStream_t s, bool with_quad = false);
-void launch_walk_records(const Particles& p, int64_t n, int64_t n_int, TreeBuffers& t, cudaStream_t s);
+// counts: the nodes of each depth, on the host; also makes the walk's
+// fixed-point centres of mass and the child counts and (records) gives every
+// node its range of walk records.
+void launch_aggregate(const Particles& p, int64_t n, int64_t n_int, double box, TreeBuffers& t, const uint32_t* counts,
+                      cudaStream_t s, bool with_quad = false, bool records = true);
+void launch_walk_records(const Particles& p, int64_t n_int, TreeBuffers& t, cudaStream_t s);
 // Per internal node: the centre of its octree cell (child_center replayed
 // along the node's octant path, octree.rs:446-465) in fixed point and the
 // Frobenius norm of its six stored quadrupole components (the relative
@@ -117,8 +117,7 @@ void launch_walk_records(const Particles& p, int64_t n, int64_t n_int, TreeBuffe
 void launch_cell_q(int64_t n_int, double box, TreeBuffers& t, cudaStream_t s);
 // Walk groups of at most group_max particles, each inside one octree cell of
 // depth pack_depth or more.
-void launch_groups(int64_t n, int64_t n_int, int group_max, int pack_depth, TreeBuffers& t, void* scan_scratch,
-                   cudaStream_t s);
+void launch_groups(int64_t n_int, int group_max, int pack_depth, TreeBuffers& t, void* scan_scratch, cudaStream_t s);
 void launch_hilbert_keys(const Particles& p, int64_t n, double box, const TreeParams* prm, uint64_t* keys,
                          uint32_t* vals, cudaStream_t s);
 // Morton keys (particle_morton, sfc.rs:54-81) with the normalisation of prm's

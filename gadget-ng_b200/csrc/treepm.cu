@@ -457,18 +457,15 @@ void ensure_tree_capacity(tpm_handle* h, int64_t n_int) {
   T.o_first = h->alloc<uint32_t>(c, 2);
   T.o_last = h->alloc<uint32_t>(c, 2);
   T.o_slots = h->alloc<uint32_t>(8 * c, 2);
-  T.o_nchild = h->alloc<uint32_t>(c, 2);
-  T.o_child_first = h->alloc<uint32_t>(c, 2);
   T.o_cnt = h->alloc<uint32_t>(c, 2);
-  T.o_ninner = h->alloc<uint8_t>(c, 2);
-  T.child_ids = h->alloc<uint32_t>(c + h->cap + 8, 2);
+  T.o_kids = h->alloc<uint8_t>(c, 2);
+  T.o_child_first = h->alloc<uint32_t>(c, 2);
   T.o_mass = h->alloc<double>(c, 2);
   T.o_com = h->alloc<double>(3 * c, 2);
   T.o_quad = h->alloc<double>(6 * c, 2);
   T.o_walk = h->alloc<uint4>(c, 2);
   T.o_cell = h->alloc<uint4>(c, 2);
   T.recs = h->alloc<WalkNode>(c + h->cap + 8, 2);
-  T.grp_count_per_node = h->alloc<uint32_t>(c, 2);
   T.grp_base = h->alloc<uint32_t>(c, 2);
   T.grp_first = h->alloc<uint32_t>(h->cap + 1, 2);
   T.grp_size = h->alloc<uint32_t>(h->cap + 1, 2);
@@ -612,23 +609,25 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
       launch_levels(n, T, s);
       exclusive_scan_u32(T.oct_count, T.oct_base, n, &T.scalars[0], h->scan_scratch, s);
       TPM_CUDA(cudaMemcpyAsync(h->back->scalars, T.scalars, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+      TPM_CUDA(cudaMemcpyAsync(h->back->depth_counts, T.depth_tab, sizeof(h->back->depth_counts),
+                               cudaMemcpyDeviceToHost, s));
       TPM_CUDA(cudaMemcpyAsync(&h->back->params, T.params, sizeof(TreeParams), cudaMemcpyDeviceToHost, s));
       TPM_CUDA(cudaStreamSynchronize(s));
       h->params_host = h->back->params;
       h->n_int = h->back->scalars[0];
       ensure_tree_capacity(h, h->n_int);
-      launch_octree_nodes(n, h->n_int, T, h->scan_scratch, s);
+      launch_octree_nodes(n, h->n_int, T, s);
       // the accurate walk's relative opening criterion reads |Q|_F and the
       // cell centres: the quadrupole pass runs only for it
       const bool rel = relative_mac(h);
       launch_aggregate(h->P[h->cur], n, h->n_int, box, T, h->back->depth_counts, s, rel);
       h->quad_valid = rel;
       if (rel) launch_cell_q(h->n_int, box, T, s);
-      launch_walk_records(h->P[h->cur], n, h->n_int, T, s);
+      launch_walk_records(h->P[h->cur], h->n_int, T, s);
       int pack_depth = 0;  // the first depth whose cells are no wider than a walk group may be
       const double extent = max_extent(h);
       while (pack_depth < DEPTH_BINS && !(std::ldexp(2.0 * h->params_host.half, -pack_depth) <= extent)) ++pack_depth;
-      launch_groups(n, h->n_int, walk_group_size(n), pack_depth, T, h->scan_scratch, s);
+      launch_groups(h->n_int, walk_group_size(n), pack_depth, T, h->scan_scratch, s);
       // the group count and the tree depth stay on the device until the end of
       // the evaluation (the learned path sizes a launch by the group count)
       TPM_CUDA(cudaMemcpyAsync(h->back->scalars, T.scalars, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
@@ -672,8 +671,8 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
       const Particles& P = h->P[h->cur];
       a.qx = P.qx; a.qy = P.qy; a.qz = P.qz; a.massf = P.massf;
       a.recs = T.recs;
-      a.walk = T.o_walk; a.depth = T.o_depth; a.nchild = T.o_nchild; a.child_first = T.o_child_first;
-      a.child_ids = T.child_ids; a.o_com = T.o_com; a.leaf_depth = T.leaf_depth;
+      a.depth = T.o_depth; a.slots = T.o_slots;
+      a.o_com = T.o_com; a.leaf_depth = T.leaf_depth; a.walk = T.o_walk;
       a.gfirst = use_net ? h->lgrp_first : T.grp_first;
       a.gsize = use_net ? h->lgrp_size : T.grp_size;
       a.ngroups = use_net ? h->lgrp_count : &T.scalars[1];
@@ -2210,7 +2209,7 @@ int64_t tpm_export_tree(tpm_handle* h, int64_t cap, int32_t* depth, double* mass
       throw Error(TPM_ERR_INVALID_ARGUMENT, "null export array");
     cudaStream_t s = h->stream;
     if (!h->quad_valid && ni > 0) {  // the force evaluation made mass and centre of mass only
-      launch_aggregate(h->P[h->cur], n, ni, h->cfg.box_size, h->T, h->back->depth_counts, s, true);
+      launch_aggregate(h->P[h->cur], n, ni, h->cfg.box_size, h->T, h->back->depth_counts, s, true, false);
       h->quad_valid = true;
     }
     int32_t* dd;

@@ -883,12 +883,14 @@ __device__ void deferred_walk(const WalkArgs& a, uint2 job) {
   uint32_t stack[8 * 48];
   int sp = 0;
   float fx = 0.f, fy = 0.f, fz = 0.f;
-  // open `job.y`: push its children
-  {
-    const uint32_t nd = job.y;
-    const uint32_t f = a.child_first[nd], c = a.nchild[nd];
-    for (uint32_t k = 0; k < c; ++k) stack[sp++] = a.child_ids[f + k];
-  }
+  // push the children of a node
+  auto open = [&](uint32_t nd) {
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t c = a.slots[8 * (int64_t)nd + k];
+      if (c != EMPTY_SLOT) stack[sp++] = c;
+    }
+  };
+  open(job.y);
   int64_t guard = 0;
   while (sp > 0) {
     if (++guard > a.n_int + a.n + 2) {
@@ -920,14 +922,12 @@ __device__ void deferred_walk(const WalkArgs& a, uint2 job) {
       const int d = exact_terminal(a, p, node);
       if (d == 1) interact = true;
       else if (d == 2) {
-        const uint32_t f = a.child_first[node], cc = a.nchild[node];
-        if (sp + (int)cc > 8 * 48) { atomicOr(a.err, DEV_ERR_STACK); break; }
-        for (uint32_t k = 0; k < cc; ++k) stack[sp++] = a.child_ids[f + k];
+        if (sp + 8 > 8 * 48) { atomicOr(a.err, DEV_ERR_STACK); break; }
+        open(node);
       }
     } else {
-      const uint32_t f = a.child_first[node], cc = a.nchild[node];
-      if (sp + (int)cc > 8 * 48) { atomicOr(a.err, DEV_ERR_STACK); break; }
-      for (uint32_t k = 0; k < cc; ++k) stack[sp++] = a.child_ids[f + k];
+      if (sp + 8 > 8 * 48) { atomicOr(a.err, DEV_ERR_STACK); break; }
+      open(node);
     }
     if (interact) {
       atomicAdd(&a.pcounts[2 * (int64_t)p + ((node & LEAF_BIT) ? 0 : 1)], 1u);

@@ -23,9 +23,7 @@ struct WalkArgs {
   const WalkNode* recs;  // walk records, children contiguous
   const uint4* walk;  // internal nodes: fixed-point COM + float mass bits
   const uint8_t* depth;
-  const uint32_t* nchild;
-  const uint32_t* child_first;
-  const uint32_t* child_ids;
+  const uint32_t* slots;  // eight child slots per internal node
   const double* o_com;
   const uint8_t* leaf_depth;
   // groups
