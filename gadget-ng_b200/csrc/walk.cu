@@ -33,7 +33,7 @@
 // took two entries per iteration in f32x2 arithmetic (63 instructions for
 // two entries, ~106 before) and the traversal was split into open and item
 // steps; 5.93e9 take 7.1 ms at 73 % after (62.7 -> 40.3 ms on the clustered
-// 256^3 box).  Two thirds are the pair loop (60 per iteration), its FMA pipe
+// 256^3 box, 39.3 with 128-entry lists).  Two thirds are the pair loop (60 per iteration), its FMA pipe
 // 56 % busy.  The accurate mode took the same steps later: 10.3 -> 7.4 ms on the
 // clustered 128^3 box against its former traversal (32 children of a popped
 // batch per step, opening tests at pop time).
@@ -49,8 +49,14 @@ namespace {
 
 constexpr int WALK_WARPS = 4;
 constexpr int WALK_THREADS = WALK_WARPS * 32;
-constexpr int CHUNK_L = 64;  // leaf-list capacity (walk 72.9 -> 72.5 ms at 256^3 against 48; 32 is slower)
-constexpr int CHUNK_M = 64;  // monopole-list capacity
+// List capacities (leaves, monopoles).  Longer lists are flushed less often (30
+// times per group at 64 entries, each time a start of both pair loops and a
+// compensated add), but leave less L1 cache to the tree.  Parity, clustered
+// 256^3 / 128^3 / clustered 99^3, walk ms: 64 entries 40.6 / 7.17 / 4.05, 96 39.7 /
+// 7.02 / 3.97, 128 39.3 / 6.93 / 3.95, 192 leaves and 64 monopoles 39.1 / 6.93 /
+// 4.07, 256 and 64 39.2 / 6.92 / 4.07.  Accurate 128^3: 64 7.46, 96 7.53, 128 7.79.
+template <bool ACC> constexpr int chunk_l() { return ACC ? 64 : 128; }
+template <bool ACC> constexpr int chunk_m() { return ACC ? 64 : 128; }
 
 
 // An interaction list in shared memory, kept in pairs of entries so that the
@@ -78,12 +84,19 @@ template <int CAP, bool HALF> struct List {
   static_assert(CAP % 2 == 0, "entries are evaluated two at a time");
   EntryPair<HALF> pair[CAP / 2];
   // word w of entry e: members of a pair interleave its two entries
-  __device__ __forceinline__ float* word(int e) { return reinterpret_cast<float*>(&pair[e >> 1]) + (e & 1); }
+  __device__ __forceinline__ static float* word(EntryPair<HALF>* pair, int e) {
+    return reinterpret_cast<float*>(&pair[e >> 1]) + (e & 1);
+  }
+  __device__ __forceinline__ float* word(int e) { return word(pair, e); }
   __device__ __forceinline__ const float* word(int e) const {
     return reinterpret_cast<const float*>(&pair[e >> 1]) + (e & 1);
   }
   __device__ __forceinline__ void put(int e, float x, float y, float z, float m, float half, uint32_t see, uint32_t nd) {
-    float* w = word(e);
+    put(pair, e, x, y, z, m, half, see, nd);
+  }
+  __device__ __forceinline__ static void put(EntryPair<HALF>* pair, int e, float x, float y, float z, float m, float half,
+                                             uint32_t see, uint32_t nd) {
+    float* w = word(pair, e);
     w[0] = x;
     w[2] = y;
     w[4] = z;
@@ -434,8 +447,8 @@ __device__ __forceinline__ Sums eval(const WalkArgs& a, const L& list, int n, ui
 // registers across the traversal.
 template <bool PERIODIC, int KERNEL> struct Lists {
   static constexpr bool ACC = KERNEL == K_ACC;
-  List<CHUNK_L, !PERIODIC> leaf;
-  List<CHUNK_M, ACC || !PERIODIC> mono;
+  List<chunk_l<ACC>(), !PERIODIC> leaf;
+  List<chunk_m<ACC>(), ACC || !PERIODIC> mono;
 };
 template <bool PERIODIC, int KERNEL>
 __device__ __forceinline__ void flush(const WalkArgs& a, const Lists<PERIODIC, KERNEL>& lists, int nll, int nlm,
@@ -648,7 +661,7 @@ __device__ __forceinline__ void walk_group(const WalkArgs& a, uint32_t first, ui
     // a step adds up to 32 entries to either list (one call site of the list
     // evaluation, the last flush included)
     const bool done = sp == 0 && nq == 0;
-    if (done || nll > CHUNK_L - 32 || nlm > CHUNK_M - 32) {
+    if (done || nll > chunk_l<ACC>() - 32 || nlm > chunk_m<ACC>() - 32) {
       if (lane == 0) {
         mem.lists.leaf.close(nll);
         mem.lists.mono.close(nlm);
@@ -695,9 +708,10 @@ __device__ __forceinline__ void walk_group(const WalkArgs& a, uint32_t first, ui
         if constexpr (ACC) {
           mem.lists.leaf.put(nll + __popc(el & below), sx, sy, sz, __uint_as_float(r0.w), h, see, r1.z | LEAF_BIT);
         } else {
-          auto& list = leaf ? mem.lists.leaf : mem.lists.mono;  // the same layout
-          list.put(leaf ? nll + __popc(el & below) : nlm + __popc(em & below), sx, sy, sz, __uint_as_float(r0.w), h,
-                   see, leaf ? r1.z | LEAF_BIT : r1.z);
+          // both lists have the same layout of pairs
+          List<2, !PERIODIC>::put(leaf ? mem.lists.leaf.pair : mem.lists.mono.pair,
+                                  leaf ? nll + __popc(el & below) : nlm + __popc(em & below), sx, sy, sz,
+                                  __uint_as_float(r0.w), h, see, leaf ? r1.z | LEAF_BIT : r1.z);
         }
       }
       nll += __popc(el);
