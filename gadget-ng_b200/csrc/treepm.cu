@@ -248,7 +248,7 @@ struct tpm_handle {
   void* scan_scratch = nullptr;
   uint32_t* stack = nullptr;
   int walk_grid = 0;
-  bool poly = false;  // the walk's erfc polynomial covers r_cut
+  ErfcPoly poly{};  // the walk's erfc polynomial, and how far it holds
   uint2* deferred = nullptr;
   uint32_t* ndeferred = nullptr;
   unsigned long long* stats_dev = nullptr;
@@ -488,6 +488,12 @@ double max_extent(const tpm_handle* h) {
   return std::max(0.0, std::min(fits, std::max(box / 16.0, std::min(0.25 * box, 2.8 * rc))));
 }
 
+// The longest distance (softening aside) at which the parity walk evaluates a
+// pair.  Periodic: leaves end at r_cut, and the box of a monopole, of half side
+// below 0.1 r_cut, reaches sqrt(3) times that farther.  Aperiodic: a leaf is cut
+// on the gap to its cell, which may be a large part of the box.
+double pair_reach(const tpm_handle* h) { return h->periodic ? 1.18 * h->r_cut : std::sqrt(3.0) * h->cfg.box_size; }
+
 // A float in both halves of a packed pair.
 unsigned long long twice(float v) {
   uint32_t b;
@@ -709,11 +715,15 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
       a.eps2_2 = twice(std::max(a.eps2_u, 1e-30f));
       const double cx = u / (std::sqrt(2.0) * h->r_s);
       a.pcx = (float)(0.3275911 * cx);
-      a.poly = h->poly ? 1 : 0;
-      if (h->poly) {
-        float c[POLY_DEGREE + 1];
-        erfc_poly(h->r_cut / (std::sqrt(2.0) * h->r_s), cx, c);
-        for (int k = 0; k <= POLY_DEGREE; ++k) a.poly2[k] = twice(c[k]);
+      // erfc by the polynomial where it holds out to the farthest pair
+      const double reach = pair_reach(h);
+      a.poly = std::sqrt(reach * reach + eps2) <= h->poly.end * std::sqrt(2.0) * h->r_s ? 1 : 0;
+      if (a.poly) {
+        double power = 1.0;
+        for (int k = 0; k <= POLY_DEGREE; ++k) {
+          a.poly2[k] = twice((float)(h->poly.coef[k] * power));
+          power *= cx;
+        }
       }
       a.ex2k = (float)(-(cx * cx) / std::log(2.0));
       const double tq = std::ldexp(4.0, -U);
@@ -1062,11 +1072,8 @@ int tpm_create(const tpm_config* cfg, tpm_handle** out) {
     h->learned_count = h->alloc<unsigned long long>(1, 0);
     h->deferred = h->alloc<uint2>(DEFERRED_CAP, 0);
     int sms = prop.multiProcessorCount;
-    {
-      float unused[POLY_DEGREE + 1];
-      h->poly = erfc_poly(h->r_cut / (std::sqrt(2.0) * h->r_s), 1.0, unused);
-    }
-    h->walk_grid = sms * walk_blocks_per_sm(h->periodic, (cfg->flags & TPM_FLAG_ACCURATE) != 0, h->poly);
+    h->poly = erfc_poly(h->r_cut / (std::sqrt(2.0) * h->r_s), 2.0 * pair_reach(h) / (std::sqrt(2.0) * h->r_s));
+    h->walk_grid = sms * walk_blocks_per_sm(h->periodic, (cfg->flags & TPM_FLAG_ACCURATE) != 0);
     h->stack = h->alloc<uint32_t>(walk_stack_words(h->walk_grid, STACK_CAP), 0);
     TPM_CUDA(cudaMemset(h->T.err, 0, sizeof(uint32_t)));
     pm_plan_init(h->pm, nm, cfg->box_size, h->pm_only ? 0.0 : h->r_s, cfg->flags, cfg->device);

@@ -37,6 +37,7 @@
 // 56 % busy.  The accurate mode took the same steps later: 10.3 -> 7.4 ms on the
 // clustered 128^3 box against its former traversal (32 children of a popped
 // batch per step, opening tests at pop time).
+#include <algorithm>
 #include <cmath>
 #include <type_traits>
 
@@ -991,7 +992,7 @@ static void launch_t(const WalkArgs& a, int grid, cudaStream_t s) {
   k_walk<walk_blocks<PERIODIC, KERNEL>(), PERIODIC, KERNEL><<<grid, WALK_THREADS, smem, s>>>(a);
 }
 
-// The kernel of a handle, by its walk and pair term; also sizes its grid.
+// The kernel of a walk, by its mode and pair term; also sizes its grid.
 template <class F>
 static void with_kernel(bool periodic, bool accurate, bool poly, F&& f) {
   using P = std::true_type;
@@ -1014,44 +1015,64 @@ int walk_group_size(int64_t n) {
   return size;
 }
 
-int walk_blocks_per_sm(bool periodic, bool accurate, bool poly) {
+// (a handle of the parity walk may take either pair term, call by call)
+int walk_blocks_per_sm(bool periodic, bool accurate) {
   int nb = 1;
-  with_kernel(periodic, accurate, poly,
-              [&](auto p, auto k) { nb = blocks_for<decltype(p)::value, decltype(k)::value>(); });
+  for (const bool poly : {false, true})
+    with_kernel(periodic, accurate, poly, [&](auto p, auto k) {
+      nb = std::max(nb, blocks_for<decltype(p)::value, decltype(k)::value>());
+    });
   return nb;
 }
 
 // Interpolation at the Chebyshev nodes of [0, x_max] of log2 of the A&S
-// 7.1.26 erfc, as coefficients of powers of r = x / cx.  On x_max <= 3.6 (a cut
-// of 5 r_s is x = 3.54) the polynomial stays within 2e-8 of that function,
-// relative, and its FP32 evaluation within 7e-8 absolute (the A&S form itself
-// in FP32: 3.9e-7), so the walk takes one reciprocal less per pair; longer
-// cuts keep the A&S form.
-bool erfc_poly(double x_max, double cx, float* coef) {
-  if (!(x_max <= 3.6)) return false;
+// 7.1.26 erfc.  On x_max <= 3.6 (a cut of 5 r_s is x = 3.54) the polynomial stays
+// within 2e-8 of that function, absolute, and its FP32 evaluation within 8e-8
+// (the A&S form itself in FP32: 3.9e-7), so the walk takes one reciprocal less per
+// pair; longer cuts keep the A&S form.
+//
+// Some pairs lie beyond the cut: monopoles by their half side, leaves of the
+// aperiodic walk by that of their cell, all of them when the softening is long.
+// Out there 2^P keeps falling to 0 for cuts from 3.65 r_s on, but for shorter ones
+// P turns and rises without bound (at 2 r_s from 1.57 r_cut on).  `end` is the
+// distance up to which its FP32 evaluation was found within 1e-7 of the function
+// (at 65 points of the fit, then in steps of 1 %); beyond it the A&S form serves.
+ErfcPoly erfc_poly(double x_max, double x_far) {
+  ErfcPoly out{};
+  if (!(x_max <= 3.6)) return out;
+  const auto tail = [](double x) {  // the A&S form times exp(x^2)
+    const double t = 1.0 / (1.0 + 0.3275911 * x);
+    return t * (0.254829592 + t * (-0.284496736 + t * (1.421413741 + t * (-1.453152027 + t * 1.061405429))));
+  };
   constexpr int N = POLY_DEGREE + 1;
   double node[N], div[N];
   for (int i = 0; i < N; ++i) {
     const double x = 0.5 * x_max * (1.0 - std::cos(M_PI * (i + 0.5) / N));
-    const double t = 1.0 / (1.0 + 0.3275911 * x);
-    const double p = t * (0.254829592 + t * (-0.284496736 + t * (1.421413741 + t * (-1.453152027 + t * 1.061405429))));
     node[i] = x;
-    div[i] = std::log2(p) - x * x / std::log(2.0);
+    div[i] = std::log2(tail(x)) - x * x / std::log(2.0);
   }
   for (int k = 1; k < N; ++k)  // Newton's divided differences
     for (int i = N - 1; i >= k; --i) div[i] = (div[i] - div[i - 1]) / (node[i] - node[i - k]);
-  double c[N] = {0.0};
+  double* c = out.coef;
   c[0] = div[N - 1];
   for (int k = N - 2; k >= 0; --k) {  // c <- c (x - node[k]) + div[k]
     for (int i = N - 1; i > 0; --i) c[i] = c[i - 1] - node[k] * c[i];
     c[0] = div[k] - node[k] * c[0];
   }
-  double scale = 1.0;
-  for (int i = 0; i < N; ++i) {
-    coef[i] = (float)(c[i] * scale);
-    scale *= cx;
+  const auto holds = [&](double x) {
+    float p = (float)c[N - 1];
+    for (int k = N - 2; k >= 0; --k) p = std::fma(p, (float)x, (float)c[k]);
+    return std::fabs(std::exp2((double)p) - tail(x) * std::exp(-x * x)) <= 1e-7;  // (false for a NaN)
+  };
+  for (int i = 0; i <= 64; ++i)
+    if (!holds(x_max * i / 64.0)) return out;
+  out.end = x_max;
+  for (double x = x_max; out.end < x_far && holds(x);) {
+    out.end = x;
+    x = std::min(1.01 * x, x_far);
+    if (x == x_far && holds(x)) out.end = x;
   }
-  return true;
+  return out;
 }
 
 size_t walk_stack_words(int grid, int stack_cap) {

@@ -8,9 +8,14 @@
 namespace tpm {
 
 constexpr int POLY_DEGREE = 10;
-// Coefficients (powers of r in walk units, x = cx r) of P with erfc(x) =
-// 2^P(r) on [0, x_max]; false when x_max is beyond the fitted range.
-bool erfc_poly(double x_max, double cx, float* coef);
+// P with erfc(x) = 2^P(x) on [0, x_max]: coefficients of powers of x, and the
+// end of the range on which it may be used: at most x_far, and 0 when x_max
+// itself is beyond what a polynomial of this degree fits.
+struct ErfcPoly {
+  double coef[POLY_DEGREE + 1];
+  double end;
+};
+ErfcPoly erfc_poly(double x_max, double x_far);
 
 struct WalkArgs {
   int64_t n, n_int;
@@ -76,7 +81,7 @@ struct WalkArgs {
 
 constexpr int WALK_TARGETS = 32;  // targets per warp at most
 int walk_group_size(int64_t n);   // targets per walk group in a box of n particles
-int walk_blocks_per_sm(bool periodic, bool accurate, bool poly);
+int walk_blocks_per_sm(bool periodic, bool accurate);
 size_t walk_stack_words(int grid, int stack_cap);
 void launch_walk(const WalkArgs& a, int grid, cudaStream_t s);
 void launch_deferred(const WalkArgs& a, cudaStream_t s);

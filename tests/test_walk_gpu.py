@@ -27,6 +27,9 @@ def _positions(kind, n, box, seed):
         x = g[:n] + rng.normal(0.0, 0.3 * box / side, (n, 3))
     elif kind == "clump":  # everything inside one terminal cell, across the corner of the box
         x = rng.normal(0.0, 2e-4 * box, (n, 3))
+    elif kind == "middle":  # half of the particles in a clump, the others far apart: leaves in wide cells
+        x = rng.uniform(0.0, box, (n, 3))
+        x[: n // 2] = 0.5 * box + rng.normal(0.0, 5e-3 * box, (n // 2, 3))
     else:  # two dense clumps on a sparse background
         x = rng.uniform(0.0, box, (n, 3))
         k = n // 3
@@ -82,6 +85,62 @@ def test_interactions_and_forces_match_the_oracle(kind, n, mesh, cells, factor, 
         assert np.sqrt(np.mean(np.sum((sr - ref) ** 2, axis=1))) < 1e-5 * scale
     else:
         assert not sr.any()
+
+
+# Pairs far beyond the range that the erfc polynomial is fitted on: leaves of the
+# aperiodic walk in wide cells (cut on the gap to the cell), and a softening that
+# is longer than r_cut.
+FAR = [
+    # kind, n, mesh, r_split cells, r_cut factor, periodic, softening / r_cut
+    ("uniform", 10, 64, 2.5, 1.0, False, 0.0),
+    ("uniform", 10, 64, 2.5, 2.0, False, 0.0),
+    ("uniform", 10, 64, 2.5, 3.0, False, 0.0),
+    ("middle", 1000, 128, 1.25, 1.0, False, 0.05),
+    ("middle", 1000, 128, 1.25, 2.0, False, 0.05),
+    ("middle", 1000, 128, 1.25, 3.0, False, 0.05),
+    ("middle", 1000, 128, 1.25, 3.5, False, 0.05),
+    ("middle", 1000, 128, 1.25, 3.6, False, 0.05),
+    ("middle", 1000, 128, 1.25, 3.65, False, 0.05),
+    ("middle", 1000, 128, 1.25, 5.0, False, 0.05),
+    ("middle", 1000, 32, 1.25, 1.0, True, 0.05),
+    ("middle", 1000, 32, 1.25, 2.0, True, 0.0),
+    ("middle", 1000, 32, 1.25, 2.0, True, 1.5),
+    ("middle", 1000, 32, 1.25, 3.0, True, 4.0),
+    ("middle", 1000, 32, 1.25, 4.5, True, 4.0),
+    ("middle", 1000, 64, 1.25, 2.0, False, 4.0),
+]
+
+
+@pytest.mark.parametrize("kind,n,mesh,cells,factor,periodic,soft", FAR)
+def test_each_particle_matches_the_oracle_beyond_the_fitted_range(kind, n, mesh, cells, factor, periodic, soft):
+    """Per particle: 1e-6 of erfc (the A&S form in FP32 is off by 4e-7, the
+    polynomial by 1e-7) times the sum of m / r^2, and 1e-5 of the sum of the
+    pair forces (distances are rounded relative to a group, as above)."""
+    import treepm
+    from scipy.special import erfc
+    box, g = 50.0, 1.7
+    pos = _positions(kind, n, box, n + mesh)
+    mass = np.random.default_rng(n).uniform(0.5, 1.5, n) / n
+    r_split = cells * box / mesh
+    eps2 = (soft * factor * r_split) ** 2
+    s = treepm.TreePmSolver(mesh, box, r_split, r_cut_factor=factor, periodic_walk=periodic)
+    s.set_particles(pos, mass)
+    s.compute_forces(eps2, g)
+    _, sr = s.force_parts(n)
+    counts = s.interaction_counts(n)
+    s.close()
+    ref, ref_counts = oracle().short_range(pos, mass, eps2, g, r_split, factor * r_split, box, periodic=periodic,
+                                           counts=True)
+    assert np.array_equal(counts, ref_counts)
+    d = pos[None] - pos[:, None]
+    if periodic:
+        d -= box * np.round(d / box)
+    r2 = np.sum(d * d, axis=2) + eps2
+    np.fill_diagonal(r2, np.inf)
+    w = erfc(np.sqrt(r2) / (np.sqrt(2.0) * r_split))
+    allowed = g * np.sum(mass[None] / r2 * (1e-6 + 1e-5 * w), axis=1)
+    assert np.isfinite(sr).all()
+    assert (np.linalg.norm(sr - ref, axis=1) <= allowed).all()
 
 
 @pytest.mark.parametrize("n,periodic", [(31, True), (700, True), (2100, True), (700, False)])
