@@ -146,11 +146,11 @@ __device__ __forceinline__ float min3_abs(float a, float b, float c) {
   return r;
 }
 
-__device__ __forceinline__ int32_t rel32(uint32_t a, uint32_t b, int periodic) {
-  if (periodic) return (int32_t)(a - b);  // minimum image modulo 2^32
-  int64_t d = (int64_t)a - (int64_t)b;
-  d = d > 0x7FFFFFFFll ? 0x7FFFFFFFll : (d < -0x7FFFFFFFll ? -0x7FFFFFFFll : d);
-  return (int32_t)d;
+// a - b in quanta: the minimum image (modulo 2^32), or in the aperiodic walk the
+// difference itself, up to a whole box.
+__device__ __forceinline__ float rel(uint32_t a, uint32_t b, int periodic) {
+  if (periodic) return (float)(int32_t)(a - b);
+  return a >= b ? (float)(a - b) : -(float)(b - a);
 }
 
 
@@ -630,7 +630,8 @@ __device__ __forceinline__ void walk_group(const WalkArgs& a, uint32_t first, ui
       // positions relative to the middle of the group's box: half the extent
       // bounds them, and with them the rounding of the pair distances
       const uint32_t q0 = __shfl_sync(0xffffffffu, tq[d], 0);
-      const int32_t tr = rel32(tq[d], q0, PERIODIC);
+      // (a group lies in a cell far smaller than half the box)
+      const int32_t tr = (int32_t)(tq[d] - q0);
       const int32_t lo = __reduce_min_sync(0xffffffffu, has ? tr : 0x7FFFFFFF);
       const int32_t hi = __reduce_max_sync(0xffffffffu, has ? tr : -0x7FFFFFFF);
       const int32_t mid = lo + ((hi - lo) >> 1);
@@ -694,8 +695,8 @@ __device__ __forceinline__ void walk_group(const WalkArgs& a, uint32_t first, ui
       }
       const bool leaf = ACC || (r1.y & WN_LEAF) != 0u;
       const float h = !leaf ? a.h_term : (PERIODIC ? 0.f : half_side(a.h0_u, wn_depth(r1.y)));
-      const float sx = (float)rel32(r0.x, GO.x, PERIODIC) * a.u_inv, sy = (float)rel32(r0.y, GO.y, PERIODIC) * a.u_inv;
-      const float sz = (float)rel32(r0.z, GO.z, PERIODIC) * a.u_inv;
+      const float sx = rel(r0.x, GO.x, PERIODIC) * a.u_inv, sy = rel(r0.y, GO.y, PERIODIC) * a.u_inv;
+      const float sz = rel(r0.z, GO.z, PERIODIC) * a.u_inv;
       // the gap between the group box and the node's box
       const float gx = fmaxf(fabsf(sx) - (GW.x + h), 0.f), gy = fmaxf(fabsf(sy) - (GW.y + h), 0.f);
       const float gz = fmaxf(fabsf(sz) - (GW.z + h), 0.f);
@@ -737,8 +738,8 @@ __device__ __forceinline__ void walk_group(const WalkArgs& a, uint32_t first, ui
     // cull half side: the COM-centred AABB's, or (accurate) twice that, which
     // holds the whole cell
     const float h = ACC ? 2.f * hnode : hnode;
-    const float sx = (float)rel32(r0.x, GO.x, PERIODIC) * a.u_inv, sy = (float)rel32(r0.y, GO.y, PERIODIC) * a.u_inv;
-    const float sz = (float)rel32(r0.z, GO.z, PERIODIC) * a.u_inv;
+    const float sx = rel(r0.x, GO.x, PERIODIC) * a.u_inv, sy = rel(r0.y, GO.y, PERIODIC) * a.u_inv;
+    const float sz = rel(r0.z, GO.z, PERIODIC) * a.u_inv;
     const float ux = fabsf(sx), uy = fabsf(sy), uz = fabsf(sz);
     // the nearest and the farthest a target can be from the node's box
     const float gx = fmaxf(ux - (GW.x + h), 0.f), gy = fmaxf(uy - (GW.y + h), 0.f), gz = fmaxf(uz - (GW.z + h), 0.f);
@@ -765,8 +766,8 @@ __device__ __forceinline__ void walk_group(const WalkArgs& a, uint32_t first, ui
         // the target must be outside the node's cell: a group box touching the
         // cell leaves the node to the per-target test
         const uint4 cc = __ldg(&a.cellq[r1.z]);
-        cell = make_float4((float)rel32(cc.x, GO.x, PERIODIC) * a.u_inv, (float)rel32(cc.y, GO.y, PERIODIC) * a.u_inv,
-                           (float)rel32(cc.z, GO.z, PERIODIC) * a.u_inv, __uint_as_float(cc.w) / __uint_as_float(r0.w));
+        cell = make_float4(rel(cc.x, GO.x, PERIODIC) * a.u_inv, rel(cc.y, GO.y, PERIODIC) * a.u_inv,
+                           rel(cc.z, GO.z, PERIODIC) * a.u_inv, __uint_as_float(cc.w) / __uint_as_float(r0.w));
         const float hc = hnode * 1.0001f;
         const bool touch = fabsf(cell.x) <= GW.x + hc && fabsf(cell.y) <= GW.y + hc && fabsf(cell.z) <= GW.z + hc;
         const bool inside = fabsf(cell.x) + GW.x <= hc && fabsf(cell.y) + GW.y <= hc && fabsf(cell.z) + GW.z <= hc;
@@ -946,9 +947,9 @@ __device__ void deferred_walk(const WalkArgs& a, uint2 job) {
     }
     if (interact) {
       atomicAdd(&a.pcounts[2 * (int64_t)p + ((node & LEAF_BIT) ? 0 : 1)], 1u);
-      const float dx = (float)rel32(cq[0], tq[0], a.periodic) * a.u_inv;
-      const float dy = (float)rel32(cq[1], tq[1], a.periodic) * a.u_inv;
-      const float dz = (float)rel32(cq[2], tq[2], a.periodic) * a.u_inv;
+      const float dx = rel(cq[0], tq[0], a.periodic) * a.u_inv;
+      const float dy = rel(cq[1], tq[1], a.periodic) * a.u_inv;
+      const float dz = rel(cq[2], tq[2], a.periodic) * a.u_inv;
       const float r2b = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
       const float f = a.poly ? pair_factor<K_POLY>(a, r2b, m) : pair_factor<K_AS>(a, r2b, m);
       fx = fmaf(dx, f, fx);

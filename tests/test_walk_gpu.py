@@ -30,6 +30,9 @@ def _positions(kind, n, box, seed):
     elif kind == "middle":  # half of the particles in a clump, the others far apart: leaves in wide cells
         x = rng.uniform(0.0, box, (n, 3))
         x[: n // 2] = 0.5 * box + rng.normal(0.0, 5e-3 * box, (n // 2, 3))
+    elif kind == "corner":  # half of the particles in a clump near a corner: nodes more than half a box away
+        x = rng.uniform(0.0, box, (n, 3))
+        x[: n // 2] = 0.95 * box + rng.normal(0.0, 1e-2 * box, (n // 2, 3))
     else:  # two dense clumps on a sparse background
         x = rng.uniform(0.0, box, (n, 3))
         k = n // 3
@@ -58,6 +61,11 @@ CASES = [
     ("lattice", 13824, 32, 1.25, 4.5, False),
     ("lattice", 29791, 32, 1.25, 6.0, False),
     ("lattice", 59319, 64, 2.5, 5.0, False),
+    ("corner", 600, 32, 1.25, 5.0, False),  # boxes that corner targets do not open at all
+    ("corner", 1500, 32, 1.25, 5.0, False),
+    ("corner", 8000, 32, 1.25, 4.5, False),
+    ("corner", 40000, 64, 2.5, 5.0, False),
+    ("clumps", 30000, 64, 1.25, 4.5, False),
 ]
 
 
