@@ -62,10 +62,11 @@ template <bool ACC> constexpr int chunk_m() { return ACC ? 64 : 128; }
 
 // An interaction list in shared memory, kept in pairs of entries so that the
 // pair loop reads both entries of a packed (f32x2) operand with one load:
-// source positions relative to the group's origin in walk units (one
-// rounding of the exact int32 difference; the group is compact, so the
-// rounding stays far below the softening length and the float64 band settles
-// every borderline cut), masses, the masks of targets that see them, the nodes
+// source positions relative to the middle of the group's box in walk units (the
+// exact difference of the coordinates, rounded once: the float64 band settles
+// every borderline cut, and CLOSE walks take the exact difference of the target
+// and the source where the two are near), masses, the masks of targets that see
+// them, the nodes
 // (LEAF_BIT | particle for leaves) and, where a list needs them, cull half
 // sides.
 template <bool HALF> struct __align__(16) EntryPair {
@@ -326,12 +327,13 @@ __device__ __forceinline__ float cut_s(float dx, float dy, float dz, float r2b, 
 // One lane's share of a list, two entries per iteration in packed arithmetic
 // (issue slots bound the walk, and the f32x2 instructions halve those of the
 // distance, the polynomial and the sums).  Returns true when the lane met a
-// pair that FP32 cannot decide: one inside the band around r_cut^2 or (NEAR) a
-// centre of mass within a few quanta of the target.  Its result is then void,
-// and redo_lane evaluates the lane's share again.  So the loop itself keeps only the
+// pair that the loop cannot settle: one inside the band around r_cut^2 or (NEAR)
+// one at a distance^2 below near.  Its result is then void, and redo_lane
+// evaluates the lane's share again.  So the loop itself keeps only the
 // sign of s - r_cut^2 and two running minima per pair of entries.
-template <int CUT, bool BAND, bool NEAR, int KERNEL, class L>
-__device__ __forceinline__ bool eval_list(const WalkArgs& a, const L& list, int n, uint32_t lanes, float tx, float ty, float tz, Sums& out) {
+template <int CUT, bool BAND, bool NEAR, bool OWN, int KERNEL, class L>
+__device__ __forceinline__ bool eval_list(const WalkArgs& a, const L& list, int n, uint32_t lanes, float tx, float ty,
+                                          float tz, float near, Sums& out) {
   const uint32_t tbit = 1u << (lanes & 0xffu);
   const uint32_t stride = lanes >> 16;
   auto* e = &list.pair[(lanes >> 8) & 0xffu];
@@ -359,11 +361,12 @@ __device__ __forceinline__ bool eval_list(const WalkArgs& a, const L& list, int 
     }
     const float2 q = unpack2(add2(s, nmid));
     if (BAND) edge = min3_abs(edge, q.x, q.y);
-    if (NEAR) {
+    const bool in0 = M.x & tbit, in1 = M.y & tbit;
+    if (NEAR) {  // (OWN: the target's own leaf, at no distance, is not for it to see)
       const float2 c = unpack2(r2b);
-      close = min3_abs(close, c.x, c.y);
+      close = OWN ? min3_abs(close, in0 ? c.x : 1e30f, in1 ? c.y : 1e30f) : min3_abs(close, c.x, c.y);
     }
-    const bool ok0 = (M.x & tbit) && q.x <= 0.f, ok1 = (M.y & tbit) && q.y <= 0.f;
+    const bool ok0 = in0 && q.x <= 0.f, ok1 = in1 && q.y <= 0.f;
     const float2 f = unpack2(pair_factor2<KERNEL>(a, r2b, pack2(B.z, B.w)));
     const f32x2 g = pack2(ok0 ? f.x : 0.f, ok1 ? f.y : 0.f);
     fx = fma2(dx, g, fx);
@@ -377,15 +380,31 @@ __device__ __forceinline__ bool eval_list(const WalkArgs& a, const L& list, int 
   out.y = Y.x + Y.y;
   out.z = Z.x + Z.y;
   out.n = cnt;
-  return (BAND && edge <= a.pband) || (NEAR && close < a.tiny_u);
+  return (BAND && edge <= a.pband) || (NEAR && close < near);
+}
+
+// Position of a list entry's source, in quanta.
+__device__ __forceinline__ void source_quanta(const WalkArgs& a, uint32_t node, uint32_t q[3]) {
+  if (node & LEAF_BIT) {
+    const uint32_t j = node & ~LEAF_BIT;
+    q[0] = a.qx[j];
+    q[1] = a.qy[j];
+    q[2] = a.qz[j];
+  } else {
+    const uint4 w = a.walk[node];
+    q[0] = w.x;
+    q[1] = w.y;
+    q[2] = w.z;
+  }
 }
 
 // The share of lane `src` again (rare), all 32 lanes taking entry pairs of it,
-// with the reference's float64 decisions for the undecided entries.  Every
-// lane returns the sums.
-template <int CUT, bool NEAR, int KERNEL, class L>
+// with the reference's float64 decisions for the undecided entries (MONO: also
+// for a centre of mass within a few quanta of the target) and, CLOSE, the exact
+// coordinate differences for the near ones.  Every lane returns the sums.
+template <int CUT, bool BAND, bool MONO, bool CLOSE, bool PERIODIC, int KERNEL, class L>
 __device__ __noinline__ Sums redo_lane(const WalkArgs& a, const L& list, int n, uint32_t lanes, uint32_t p, float tx,
-                                       float ty, float tz, uint32_t* nexact) {
+                                       float ty, float tz, float near, uint32_t* nexact) {
   const int t = lanes & 0xffu, stride = lanes >> 16, lane = threadIdx.x & 31;
   Sums o = {0.f, 0.f, 0.f, 0u};
   for (int e = 2 * (int)(((lanes >> 8) & 0xffu) + (uint32_t)(lane * stride)); e < n; e += 64 * stride) {
@@ -393,11 +412,19 @@ __device__ __noinline__ Sums redo_lane(const WalkArgs& a, const L& list, int n, 
       const float* w = list.word(k);
       const uint32_t node = __float_as_uint(w[10]);
       if (!((__float_as_uint(w[8]) >> t) & 1u)) continue;
-      const float dx = w[0] - tx, dy = w[2] - ty, dz = w[4] - tz;
-      const float r2b = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+      float dx = w[0] - tx, dy = w[2] - ty, dz = w[4] - tz;
+      float r2b = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+      if (CLOSE && r2b < near) {
+        uint32_t q[3];
+        source_quanta(a, node, q);
+        dx = rel(q[0], a.qx[p], PERIODIC) * a.u_inv;
+        dy = rel(q[1], a.qy[p], PERIODIC) * a.u_inv;
+        dz = rel(q[2], a.qz[p], PERIODIC) * a.u_inv;
+        r2b = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+      }
       const float s = cut_s<CUT>(dx, dy, dz, r2b, CUT == CUT_OWN_HALF ? w[12] : a.h_term);
       bool take = s <= a.prc2_lo;
-      if ((s > a.prc2_lo && s <= a.prc2_hi) || (NEAR && r2b < a.tiny_u)) {
+      if (BAND && ((s > a.prc2_lo && s <= a.prc2_hi) || (MONO && r2b < a.tiny_u))) {
         ++*nexact;
         const int d = exact_terminal(a, p, node);
         if (d == 2) defer(a, p, node);
@@ -423,11 +450,13 @@ __device__ __noinline__ Sums redo_lane(const WalkArgs& a, const L& list, int n, 
 
 // A list against this lane's pair-phase target (its position comes from the
 // lane that holds it, its particle is first + target).
-template <int CUT, bool BAND, bool NEAR, int KERNEL, class L>
+template <int CUT, bool MONO, bool CLOSE, bool PERIODIC, int KERNEL, class L>
 __device__ __forceinline__ Sums eval(const WalkArgs& a, const L& list, int n, uint32_t lanes, uint32_t first,
-                                     const float4* tfs, const float4& T, uint32_t& nexact) {
+                                     const float4* tfs, const float4& T, float near, uint32_t& nexact) {
+  // (the accurate mode reproduces no float64 decisions)
+  constexpr bool BAND = KERNEL != K_ACC, NEAR = CLOSE || (MONO && BAND);
   Sums o;
-  const bool flag = eval_list<CUT, BAND, NEAR, KERNEL>(a, list, n, lanes, T.x, T.y, T.z, o);
+  const bool flag = eval_list<CUT, BAND, NEAR, !MONO, KERNEL>(a, list, n, lanes, T.x, T.y, T.z, near, o);
   if (BAND || NEAR) {
     uint32_t again = __ballot_sync(0xffffffffu, flag);
     while (again) {
@@ -435,7 +464,8 @@ __device__ __forceinline__ Sums eval(const WalkArgs& a, const L& list, int n, ui
       again &= again - 1;
       const uint32_t sl = __shfl_sync(0xffffffffu, lanes, src);
       const float4 S = tfs[sl & 0xffu];
-      const Sums r = redo_lane<CUT, NEAR, KERNEL>(a, list, n, sl, first + (sl & 0xffu), S.x, S.y, S.z, &nexact);
+      const Sums r = redo_lane<CUT, BAND, MONO, CLOSE, PERIODIC, KERNEL>(a, list, n, sl, first + (sl & 0xffu), S.x, S.y,
+                                                                         S.z, near, &nexact);
       if ((threadIdx.x & 31) == src) o = r;
     }
   }
@@ -451,17 +481,17 @@ template <bool PERIODIC, int KERNEL> struct Lists {
   List<chunk_l<ACC>(), !PERIODIC> leaf;
   List<chunk_m<ACC>(), ACC || !PERIODIC> mono;
 };
-template <bool PERIODIC, int KERNEL>
+template <bool PERIODIC, int KERNEL, bool CLOSE>
 __device__ __forceinline__ void flush(const WalkArgs& a, const Lists<PERIODIC, KERNEL>& lists, int nll, int nlm,
-                                      int lane, uint32_t lanes, uint32_t first, const float4* tfs, float4* s0,
-                                      float4* s1, uint32_t& nexact, uint32_t& neval) {
+                                      int lane, uint32_t lanes, uint32_t first, const float4* tfs, float near,
+                                      float4* s0, float4* s1, uint32_t& nexact, uint32_t& neval) {
   constexpr bool ACC = KERNEL == K_ACC;
   neval += (uint32_t)(nll + nlm);
   const float4 T = tfs[lanes & 0xffu];
-  const Sums l = eval<PERIODIC ? CUT_BARE : CUT_OWN_HALF, !ACC, false, KERNEL>(a, lists.leaf, nll, lanes, first,
-                                                                               tfs, T, nexact);
-  const Sums m = eval<ACC ? CUT_OWN_HALF : CUT_ONE_HALF, !ACC, !ACC, KERNEL>(a, lists.mono, nlm, lanes, first, tfs,
-                                                                             T, nexact);
+  const Sums l = eval<PERIODIC ? CUT_BARE : CUT_OWN_HALF, false, CLOSE, PERIODIC, KERNEL>(a, lists.leaf, nll, lanes,
+                                                                                          first, tfs, T, near, nexact);
+  const Sums m = eval<ACC ? CUT_OWN_HALF : CUT_ONE_HALF, true, CLOSE, PERIODIC, KERNEL>(a, lists.mono, nlm, lanes,
+                                                                                        first, tfs, T, near, nexact);
   __syncwarp();
   const float4 A = s0[lane], B = s1[lane];
   Acc acc = {A.x, A.y, A.z, A.w, B.x, B.y};
@@ -470,6 +500,15 @@ __device__ __forceinline__ void flush(const WalkArgs& a, const Lists<PERIODIC, K
   s1[lane] = make_float4(acc.cy, acc.cz, __uint_as_float(__float_as_uint(B.z) + l.n),
                          __uint_as_float(__float_as_uint(B.w) + m.n));
 }
+
+// CLOSE: pairs nearer than a sixteenth of the group's extent take their exact
+// coordinate differences (in distance^2, over the square of half the extent).  A
+// relative position is off by up to 2^-25 of half the extent, so a pair beyond
+// that keeps its distance to 5e-7 per coordinate, and the nearer ones are few:
+// walk of 32^3 particles .203 -> .208 ms, 48^3 .410 -> .418 (at an eighth .210
+// and .440), error of the short range against float64 in four boxes of 32^3
+// 4.3 .. 5.5e-7 -> 2.2 .. 2.5e-7 (1.9 .. 2.4e-7), of 48^3 3.5 .. 6.8e-7 -> 2.6 .. 2.8e-7.
+constexpr float NEAR_SHARE = 1.f / 64.f;
 
 constexpr int STACK_ENTRIES = 1024;  // global, per warp
 
@@ -531,7 +570,7 @@ template <bool PERIODIC, int KERNEL> struct __align__(16) WarpMem {
   float4 cells[ACC ? 32 : 1];  // relative criterion: cell centre, |Q|_F / M of the undecided nodes
   float4 s0[32], s1[32];       // the lanes' running sums
   float4 tfs[32];              // target positions
-  float4 gbox[2];              // half widths of the group box, the origin
+  float4 gbox[2];              // half widths of the group box and the near distance^2, the origin
   uint4 queue[40];             // nodes whose terminal children wait {first record, count, mask}
 };
 
@@ -609,7 +648,7 @@ __device__ __noinline__ uint32_t refine_slow(const WalkArgs& a, WarpMem<PERIODIC
 // terminal children against the group box and appends them to the lists.  The
 // item step, which meets most of the nodes, needs neither the periodic images
 // nor the opening test.
-template <bool PERIODIC, int KERNEL>
+template <bool PERIODIC, int KERNEL, bool CLOSE>
 __device__ __forceinline__ void walk_group(const WalkArgs& a, uint32_t first, uint32_t count,
                                            WarpMem<PERIODIC, KERNEL>& mem, uint4* stk) {
   constexpr bool ACC = KERNEL == K_ACC;
@@ -641,7 +680,8 @@ __device__ __forceinline__ void walk_group(const WalkArgs& a, uint32_t first, ui
     }
     mem.tfs[lane] = make_float4(tf[0], tf[1], tf[2], 0.f);
     if (lane == 0) {
-      mem.gbox[0] = make_float4(w[0], w[1], w[2], 0.f);
+      const float wide = fmaxf(w[0], fmaxf(w[1], w[2]));  // half the group's extent
+      mem.gbox[0] = make_float4(w[0], w[1], w[2], CLOSE ? fmaxf(a.tiny_u, NEAR_SHARE * wide * wide) : a.tiny_u);
       reinterpret_cast<uint4*>(mem.gbox)[1] = make_uint4(oq[0], oq[1], oq[2], 0u);
       // the root: a terminal node by itself, or an open one
       if (term_depth == 0) mem.queue[0] = make_uint4(0u, 1u, mask0, 0u);
@@ -669,7 +709,8 @@ __device__ __forceinline__ void walk_group(const WalkArgs& a, uint32_t first, ui
         mem.lists.mono.close(nlm);
       }
       __syncwarp();
-      flush<PERIODIC, KERNEL>(a, mem.lists, nll, nlm, lane, lanes, first, mem.tfs, mem.s0, mem.s1, nexact, neval);
+      flush<PERIODIC, KERNEL, CLOSE>(a, mem.lists, nll, nlm, lane, lanes, first, mem.tfs, mem.gbox[0].w, mem.s0, mem.s1,
+                                     nexact, neval);
       __syncwarp();
       nll = 0;
       nlm = 0;
@@ -866,7 +907,7 @@ __device__ __forceinline__ void walk_group(const WalkArgs& a, uint32_t first, ui
   store_sums(a, p, has, count, mem.s0[lane], mem.s1[lane], nexact, neval);
 }
 
-template <int MIN_BLOCKS, bool PERIODIC, int KERNEL>
+template <int MIN_BLOCKS, bool PERIODIC, int KERNEL, bool CLOSE>
 __global__ void __launch_bounds__(WALK_THREADS, MIN_BLOCKS) k_walk(const __grid_constant__ WalkArgs a) {
   extern __shared__ __align__(16) unsigned char s_walk[];
   using Mem = WarpMem<PERIODIC, KERNEL>;
@@ -885,7 +926,7 @@ __global__ void __launch_bounds__(WALK_THREADS, MIN_BLOCKS) k_walk(const __grid_
     g = __shfl_sync(0xffffffffu, g, 0);
     if (g >= ngroups) break;
     const uint32_t first = a.gfirst[g], count = a.gsize[g];
-    walk_group<PERIODIC, KERNEL>(a, first, count, mem, stk);
+    walk_group<PERIODIC, KERNEL, CLOSE>(a, first, count, mem, stk);
   }
 }
 
@@ -975,11 +1016,11 @@ __global__ void k_deferred(const __grid_constant__ WalkArgs a) {
 // walk takes 96 registers (clustered 256^3: 44.0 ms at 4 blocks, 40.3 at 5, 41.0
 // at 6 with 72 bytes of spills), the accurate one 64 (clustered 128^3: 7.46 at 5,
 // 7.40 at 6, 7.51 at 7, where shared memory leaves the L1 cache 16 KB).
-template <bool PERIODIC, int KERNEL> constexpr int walk_blocks() { return KERNEL == K_ACC ? 6 : 5; }
+template <int KERNEL> constexpr int walk_blocks() { return KERNEL == K_ACC ? 6 : 5; }
 
-template <bool PERIODIC, int KERNEL>
+template <bool PERIODIC, int KERNEL, bool CLOSE>
 static int blocks_for() {
-  auto k = k_walk<walk_blocks<PERIODIC, KERNEL>(), PERIODIC, KERNEL>;
+  auto k = k_walk<walk_blocks<KERNEL>(), PERIODIC, KERNEL, CLOSE>;
   const size_t smem = sizeof(WarpMem<PERIODIC, KERNEL>) * WALK_WARPS;
   TPM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int nb = 0;
@@ -987,20 +1028,23 @@ static int blocks_for() {
   return nb < 1 ? 1 : nb;
 }
 
-template <bool PERIODIC, int KERNEL>
+template <bool PERIODIC, int KERNEL, bool CLOSE>
 static void launch_t(const WalkArgs& a, int grid, cudaStream_t s) {
   const size_t smem = sizeof(WarpMem<PERIODIC, KERNEL>) * WALK_WARPS;
-  k_walk<walk_blocks<PERIODIC, KERNEL>(), PERIODIC, KERNEL><<<grid, WALK_THREADS, smem, s>>>(a);
+  k_walk<walk_blocks<KERNEL>(), PERIODIC, KERNEL, CLOSE><<<grid, WALK_THREADS, smem, s>>>(a);
 }
 
-// The kernel of a walk, by its mode and pair term; also sizes its grid.
+// The kernel of a walk, by its mode, pair term and near pairs; also sizes its grid.
 template <class F>
-static void with_kernel(bool periodic, bool accurate, bool poly, F&& f) {
-  using P = std::true_type;
-  using A = std::false_type;
-  if (accurate) periodic ? f(P{}, std::integral_constant<int, K_ACC>{}) : f(A{}, std::integral_constant<int, K_ACC>{});
-  else if (poly) periodic ? f(P{}, std::integral_constant<int, K_POLY>{}) : f(A{}, std::integral_constant<int, K_POLY>{});
-  else periodic ? f(P{}, std::integral_constant<int, K_AS>{}) : f(A{}, std::integral_constant<int, K_AS>{});
+static void with_kernel(bool periodic, bool accurate, bool poly, bool close, F&& f) {
+  const auto flag = [](bool v, auto&& g) { v ? g(std::true_type{}) : g(std::false_type{}); };
+  flag(periodic, [&](auto p) {
+    flag(close, [&](auto c) {
+      if (accurate) f(p, std::integral_constant<int, K_ACC>{}, c);
+      else if (poly) f(p, std::integral_constant<int, K_POLY>{}, c);
+      else f(p, std::integral_constant<int, K_AS>{}, c);
+    });
+  });
 }
 
 // Targets per walk group: 32 fill a warp, but a small box then leaves most of
@@ -1016,13 +1060,14 @@ int walk_group_size(int64_t n) {
   return size;
 }
 
-// (a handle of the parity walk may take either pair term, call by call)
+// (a handle may take several of the kernels, call by call)
 int walk_blocks_per_sm(bool periodic, bool accurate) {
   int nb = 1;
   for (const bool poly : {false, true})
-    with_kernel(periodic, accurate, poly, [&](auto p, auto k) {
-      nb = std::max(nb, blocks_for<decltype(p)::value, decltype(k)::value>());
-    });
+    for (const bool close : {false, true})
+      with_kernel(periodic, accurate, poly, close, [&](auto p, auto k, auto c) {
+        nb = std::max(nb, blocks_for<decltype(p)::value, decltype(k)::value, decltype(c)::value>());
+      });
   return nb;
 }
 
@@ -1082,8 +1127,9 @@ size_t walk_stack_words(int grid, int stack_cap) {
 }
 
 void launch_walk(const WalkArgs& a, int grid, cudaStream_t s) {
-  with_kernel(a.periodic != 0, a.accurate != 0, a.poly != 0,
-              [&](auto p, auto k) { launch_t<decltype(p)::value, decltype(k)::value>(a, grid, s); });
+  with_kernel(a.periodic != 0, a.accurate != 0, a.poly != 0, a.close != 0, [&](auto p, auto k, auto c) {
+    launch_t<decltype(p)::value, decltype(k)::value, decltype(c)::value>(a, grid, s);
+  });
   TPM_LAUNCH_CHECK();
 }
 

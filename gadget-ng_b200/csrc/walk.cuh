@@ -51,6 +51,7 @@ struct WalkArgs {
   unsigned long long eps2_2;  // two floats: max(eps^2, 1e-30) in u^2 (no quantum squared is as small)
   int poly;       // erfc as 2^P(r): P's coefficients, each as two floats
   unsigned long long poly2[POLY_DEGREE + 1];
+  int close;      // exact coordinate differences for pairs near against the group's extent
   float h_term;   // parity: cull half side of the monopoles (all at the terminal depth)
   int term_depth; // the first depth whose half side is below 0.1 r_cut
   float pcx;      // 0.3275911 * scale*2^U / (sqrt(2) r_s)

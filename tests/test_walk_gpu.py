@@ -61,6 +61,8 @@ CASES = [
     ("lattice", 13824, 32, 1.25, 4.5, False),
     ("lattice", 29791, 32, 1.25, 6.0, False),
     ("lattice", 59319, 64, 2.5, 5.0, False),
+    ("lattice", 131071, 64, 1.25, 4.5, True),  # the last with exact near pairs, in groups wider than L/16
+    ("lattice", 131072, 64, 1.25, 4.5, True),
     ("corner", 600, 32, 1.25, 5.0, False),  # boxes that corner targets do not open at all
     ("corner", 1500, 32, 1.25, 5.0, False),
     ("corner", 8000, 32, 1.25, 4.5, False),
@@ -149,6 +151,57 @@ def test_each_particle_matches_the_oracle_beyond_the_fitted_range(kind, n, mesh,
     allowed = g * np.sum(mass[None] / r2 * (1e-6 + 1e-5 * w), axis=1)
     assert np.isfinite(sr).all()
     assert (np.linalg.norm(sr - ref, axis=1) <= allowed).all()
+
+
+@pytest.mark.parametrize("n,mesh,periodic,accurate", [(13600, 16, True, False), (20000, 32, True, False),
+                                                      (30000, 32, True, False), (30000, 32, False, False),
+                                                      (60000, 32, True, False), (20000, 32, True, True),
+                                                      (60000, 32, True, True)])
+def test_tight_pairs_in_wide_groups_keep_their_bits(n, mesh, periodic, accurate):
+    """Pairs far closer than their group is wide, nearly unsoftened: a position
+    relative to a group of up to L/4 is off by 2^-25 L/8, a pair at L/64 (a
+    sixteenth of the extent) then by 5e-7 per coordinate, 3.3e-6 in its force;
+    nearer ones take exact differences.  erfc as in the test above.  The parity
+    walk meets a pair alone in its cell as a centre of mass: twice the mass at half
+    the distance (8 times the force), rounded to quanta (2e-10 L of the 5e-5 L or
+    more between it and a particle: 8e-6 in the force)."""
+    import treepm
+    from scipy.special import erfc
+    box, g = 50.0, 1.7
+    pos = _positions("lattice", n, box, n)
+    rng = np.random.default_rng(n + 1)
+    k = 60  # the first particle of each pair stays, the second goes beside it
+    which = rng.choice(n, 2 * k, replace=False)
+    step = rng.normal(0.0, 1.0, (k, 3))
+    step *= (box * 10.0 ** rng.uniform(-4.0, -3.0, k) / np.linalg.norm(step, axis=1))[:, None]
+    q = np.floor(np.mod((pos[which[:k]] + step) / box, 1.0) * 2.0 ** 32)
+    pos[which[k:]] = q * (box / 2.0 ** 32)
+    mass = np.full(n, 1.0 / n)
+    r_split, factor, eps2 = 1.25 * box / mesh, 4.5, (3e-6 * box) ** 2
+    s = treepm.TreePmSolver(mesh, box, r_split, r_cut_factor=factor, periodic_walk=periodic, accurate=accurate,
+                            theta=0.01 if accurate else 0.5)
+    s.set_particles(pos, mass)
+    s.compute_forces(eps2, g)
+    _, sr = s.force_parts(n)
+    s.close()
+    d = pos[None] - pos[which][:, None]
+    if periodic:
+        d -= box * np.round(d / box)
+    r2 = np.sum(d * d, axis=2)
+    cut = r2 > (factor * r_split) ** 2
+    r2 += eps2
+    r2[np.arange(2 * k), which] = np.inf
+    x = np.sqrt(r2) / (np.sqrt(2.0) * r_split)
+    w = erfc(x)
+    if accurate:
+        w += np.where(np.isinf(x), 0.0, 2.0 / np.sqrt(np.pi) * x) * np.exp(-x * x)
+        f = np.where(cut, 0.0, w) * mass[None] / r2 ** 1.5
+        f[np.isinf(r2)] = 0.0
+        ref = g * np.einsum("ijk,ij->ik", d, f)
+    else:
+        ref = oracle().short_range(pos, mass, eps2, g, r_split, factor * r_split, box, periodic=periodic)[which]
+    allowed = g * np.sum(mass[None] / r2 * (1e-6 + (3.3e-6 if accurate else 8 * 1.13e-5) * w), axis=1)
+    assert (np.linalg.norm(sr[which] - ref, axis=1) <= allowed).all()
 
 
 @pytest.mark.parametrize("n,periodic", [(31, True), (700, True), (2100, True), (700, False)])
