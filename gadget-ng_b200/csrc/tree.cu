@@ -130,7 +130,8 @@ __global__ void k_tie_low(const uint32_t* __restrict__ qx, const uint32_t* __res
 }
 
 // Runs of equal high keys (particles sharing the first 21 octant levels) are
-// ordered by the low key.  Equal full keys mean coincident positions.
+// ordered by the low key.  Equal full keys mean coincident positions.  A run that
+// is too long is left as it is, and the host makes no tree of such keys.
 constexpr int MAX_TIE_RUN = 1 << 14;
 
 __global__ void k_fix_ties(int64_t n, const uint64_t* __restrict__ hi, uint32_t* __restrict__ perm,
@@ -308,8 +309,7 @@ __global__ void k_oct_nodes(int64_t n, int64_t n_int, const int8_t* __restrict__
         }
         j = in;
       }
-      // (in range by construction; a run of ties that was refused leaves low
-      // keys in no order, and must not write outside the nodes)
+      // (in range for keys in order, the only ones that come here)
       const int64_t u = (int64_t)base[j] + (before - lev[j] - 1);
       up = u >= 0 && u < n_int ? (int32_t)u : -1;
     }

@@ -615,19 +615,27 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
   const bool need_tree = !h->pm_only;
   const bool use_net = h->fe.use_net;
   h->fe.eps2 = eps2;
+  bool tree = n >= 2;
   if (need_tree) {
     // ---- tree
     h->n_int = 0;
-    if (n >= 2) {
+    if (tree) {
       TPM_CUDA(cudaMemsetAsync(T.scalars, 0, 4 * sizeof(uint32_t), s));
       launch_levels(n, T, s);
       exclusive_scan_u32(T.oct_count, T.oct_base, n, &T.scalars[0], h->scan_scratch, s);
       TPM_CUDA(cudaMemcpyAsync(h->back->scalars, T.scalars, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
       TPM_CUDA(cudaMemcpyAsync(h->back->depth_counts, T.depth_tab, sizeof(h->back->depth_counts),
                                cudaMemcpyDeviceToHost, s));
-      TPM_CUDA(cudaMemcpyAsync(&h->back->params, T.params, sizeof(TreeParams), cudaMemcpyDeviceToHost, s));
-      TPM_CUDA(cudaStreamSynchronize(s));
-      h->params_host = h->back->params;
+      TPM_CUDA(cudaMemcpyAsync(&h->back->err, T.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    }
+    TPM_CUDA(cudaMemcpyAsync(&h->back->params, T.params, sizeof(TreeParams), cudaMemcpyDeviceToHost, s));
+    TPM_CUDA(cudaStreamSynchronize(s));
+    h->params_host = h->back->params;
+    // The low keys of a run of ties that was refused are in no order, and no
+    // tree comes of them: none is built or walked, and the end of the evaluation
+    // raises the error.
+    if (tree && (h->back->err & DEV_ERR_TIE_RUN)) tree = false;
+    if (tree) {
       h->n_int = h->back->scalars[0];
       ensure_tree_capacity(h, h->n_int);
       launch_octree_nodes(n, h->n_int, T, s);
@@ -647,12 +655,9 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
       TPM_CUDA(cudaMemcpyAsync(h->back->scalars, T.scalars, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
       if (use_net) TPM_CUDA(cudaStreamSynchronize(s));
     } else {
-      TPM_CUDA(cudaMemcpyAsync(&h->back->params, T.params, sizeof(TreeParams), cudaMemcpyDeviceToHost, s));
-      TPM_CUDA(cudaStreamSynchronize(s));
-      h->params_host = h->back->params;
       std::memset(h->back->scalars, 0, sizeof(h->back->scalars));
     }
-    h->tree_valid = true;
+    h->tree_valid = tree || n < 2;
     TPM_CUDA(cudaEventRecord(h->ev[3], s));
     if (use_net) {
       // the network and the dense-cell mask read the mesh: long range first
@@ -668,13 +673,13 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
       if (h->net.near_cells > 0.f) {  // exact pairs below the mesh scale for the network's particles
         near_of(h, eps2, h->fallback, h->srx, h->sry, h->srz);
       }
-      learned_groups(T.grp_first, T.grp_size, n >= 2 ? h->back->scalars[1] : 0, h->fallback, h->lgrp_first, h->lgrp_size, h->lgrp_count,
-                     s);
+      learned_groups(T.grp_first, T.grp_size, h->back->scalars[1], h->fallback, h->lgrp_first, h->lgrp_size,
+                     h->lgrp_count, s);
       TPM_CUDA(cudaMemcpyAsync(&h->back->learned_groups, h->lgrp_count, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
       TPM_CUDA(cudaEventRecord(h->ev[8], s));
     }
     // ---- short-range walk
-    if (n >= 2) {
+    if (tree) {
       const double scale = box / TWO32;
       const double h0 = h->params_host.half;
       const int U = (int)std::lround(std::log2(h->r_cut / scale));

@@ -43,3 +43,31 @@ def test_tree_of_a_small_box_matches_the_insertion_octree(n):
     assert np.array_equal(got["com"][a], rc[b])
     _, ref_counts = oracle().short_range(pos, mass, 1e-3, 1.0, 5.0, 25.0, 64.0, counts=True)
     assert np.array_equal(counts, ref_counts)
+
+
+@pytest.mark.parametrize("accurate", [False, True])
+def test_a_refused_run_of_ties_makes_no_tree(accurate):
+    """More than 16,384 particles in one cell of level 21 are refused, and neither a
+    tree nor a walk is made of their keys, which are in no order.  The handle goes on."""
+    import treepm
+    rng = np.random.default_rng(9)
+    # corners first, so the root cube is known: its level-21 cells are 2048.002
+    # quanta wide, with a face at its centre
+    q = 2 ** 31 + 21504 + np.unique(rng.integers(-256, 256, (20000, 3)), axis=0)
+    q = np.concatenate([[[0, 0, 0], [2 ** 32 - 1] * 3], q])
+    n = len(q)
+    assert n > 17000
+    pos = q.astype(np.float64) * (64.0 / 2.0 ** 32)
+    s = treepm.TreePmSolver(16, 64.0, 5.0, accurate=accurate)
+    s.set_particles(pos, np.full(n, 1.0 / n))
+    for _ in range(2):
+        with pytest.raises(treepm.TreePmError) as e:
+            s.compute_forces(1e-3, 1.0)
+        assert e.value.code == 4
+        with pytest.raises(treepm.TreePmError):
+            s.export_tree()
+    pos = _box(5000, 3)
+    s.set_particles(pos, np.full(len(pos), 1.0 / len(pos)))
+    s.compute_forces(1e-3, 1.0)
+    assert len(s.export_tree()["mass"]) > len(pos) and np.isfinite(s.get_state(len(pos))[2]).all()
+    s.close()
