@@ -61,8 +61,8 @@ __global__ void k_scan_sums(uint32_t* __restrict__ sums, int64_t nb, uint32_t* _
   if (threadIdx.x == 0 && total_out) *total_out = carry;
 }
 
-__global__ void k_apply(const uint32_t* __restrict__ in, int64_t n, const uint32_t* __restrict__ sums,
-                        uint32_t* __restrict__ out) {
+// (in and out may be the same array: a thread reads its items before it writes them)
+__global__ void k_apply(const uint32_t* in, int64_t n, const uint32_t* __restrict__ sums, uint32_t* out) {
   __shared__ uint32_t sh[32];
   int64_t base = (int64_t)blockIdx.x * SCAN_TILE;
   // thread-contiguous items keep the scan order exact
@@ -84,8 +84,7 @@ __global__ void k_apply(const uint32_t* __restrict__ in, int64_t n, const uint32
 
 // Short arrays in one block: the three launches above cost more than the
 // passes of a single block (1,000-particle box: three scans, 9 -> 3 launches).
-__global__ void k_scan_one(const uint32_t* __restrict__ in, int64_t n, uint32_t* __restrict__ out,
-                           uint32_t* __restrict__ total_out) {
+__global__ void k_scan_one(const uint32_t* in, int64_t n, uint32_t* out, uint32_t* __restrict__ total_out) {
   __shared__ uint32_t sh[32];
   uint32_t carry = 0;
   for (int64_t c0 = 0; c0 < n; c0 += SCAN_TILE) {
