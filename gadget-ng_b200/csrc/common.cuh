@@ -39,7 +39,6 @@ enum : uint32_t {
   DEV_ERR_STACK = 1u << 0,
   DEV_ERR_DEFERRED = 1u << 1,
   DEV_ERR_COINCIDENT = 1u << 2,
-  DEV_ERR_LIST = 1u << 3,
   DEV_ERR_TIE_RUN = 1u << 4,
   DEV_ERR_NONFINITE = 1u << 5,
   DEV_ERR_MMA_TIMEOUT = 1u << 6,  // a tensor-core wait ran past its time limit

@@ -3,7 +3,7 @@
 // One handle = one solver (TreePmSolver / PmSolver of the reference) on one
 // device and one stream, with device-resident particle state.  A force
 // evaluation runs: bounding box -> octant-path keys -> radix sort -> particle
-// permutation -> radix tree -> octree -> bit-exact moments -> walk groups ->
+// permutation -> octree -> bit-exact moments -> walk groups ->
 // short-range walk -> CIC deposit -> FFT Poisson -> gather (+ kick).  A
 // domain-decomposed step runs the same stages in three calls around the
 // caller's density all-reduce, with halo copies of other ranks' particles
@@ -36,7 +36,6 @@ using namespace tpm;
 
 namespace {
 
-constexpr int STACK_CAP = 2048;
 constexpr uint32_t DEFERRED_CAP = 1u << 16;
 
 __global__ void k_encode(const double* __restrict__ pos, const double* __restrict__ vel,
@@ -591,8 +590,10 @@ void fe_sort(tpm_handle* h) {
     launch_bbox_root(h->P[h->cur], n, box, T, s);
     launch_tree_keys(h->P[h->cur], n, box, T, s);
     TPM_CUDA(cudaEventRecord(h->ev[1], s));
-    // every digit of an octant path varies in a box that is not a clump of
-    // lattice points, so all eight passes run without asking the host
+    // All eight passes, without asking the host for constant digits: along the
+    // longest axis of the root cube the first particle lies as far above the lower
+    // face as the last one below the upper face, so their octant bits differ on
+    // every level, and each digit holds two levels at least
     radix_sort_u64_all_passes(T.key_hi, T.perm, n, h->sort_scratch, h->sort_bytes, s);
     launch_fix_ties(h->P[h->cur], n, box, T, s);
     launch_permute(h->P[h->cur], h->P[1 - h->cur], n, T.perm, s);
@@ -767,7 +768,7 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
       a.ax = h->srx; a.ay = h->sry; a.az = h->srz;
       a.stats = h->stats_dev; a.err = T.err;
       a.deferred = h->deferred; a.ndeferred = h->ndeferred; a.cap_deferred = DEFERRED_CAP;
-      a.stack = h->stack; a.stack_cap = STACK_CAP;
+      a.stack = h->stack;
       a.pcounts = h->pcounts;
       a.only = use_net ? h->fallback : only;
       {
@@ -1088,7 +1089,7 @@ int tpm_create(const tpm_config* cfg, tpm_handle** out) {
     int sms = prop.multiProcessorCount;
     h->poly = erfc_poly(h->r_cut / (std::sqrt(2.0) * h->r_s), 2.0 * pair_reach(h) / (std::sqrt(2.0) * h->r_s));
     h->walk_grid = sms * walk_blocks_per_sm(h->periodic, (cfg->flags & TPM_FLAG_ACCURATE) != 0);
-    h->stack = h->alloc<uint32_t>(walk_stack_words(h->walk_grid, STACK_CAP), 0);
+    h->stack = h->alloc<uint32_t>(walk_stack_words(h->walk_grid), 0);
     TPM_CUDA(cudaMemset(h->T.err, 0, sizeof(uint32_t)));
     pm_plan_init(h->pm, nm, cfg->box_size, h->pm_only ? 0.0 : h->r_s, cfg->flags, cfg->device);
     h->mem_used += (size_t)nm * nm * nm * 4 * 4 + (size_t)nm * nm * (nm / 2 + 1) * 8 * 4;  // PM meshes

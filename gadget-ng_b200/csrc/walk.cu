@@ -1121,8 +1121,7 @@ ErfcPoly erfc_poly(double x_max, double x_far) {
   return out;
 }
 
-size_t walk_stack_words(int grid, int stack_cap) {
-  (void)stack_cap;
+size_t walk_stack_words(int grid) {
   return (size_t)grid * WALK_WARPS * STACK_ENTRIES * 4;  // one 16-byte entry = 4 words
 }
 

@@ -74,7 +74,6 @@ struct WalkArgs {
   uint32_t* ndeferred;
   uint32_t cap_deferred;
   uint32_t* stack;
-  int stack_cap;
   uint32_t* pcounts;     // per target (sorted order): leaf pairs, monopoles
   const uint8_t* only;   // nullptr, or: walk only the targets p with only[p] != 0
   int img_depth;         // periodic: nodes shallower than this need the +-L images in the group cull
@@ -83,7 +82,7 @@ struct WalkArgs {
 constexpr int WALK_TARGETS = 32;  // targets per warp at most
 int walk_group_size(int64_t n);   // targets per walk group in a box of n particles
 int walk_blocks_per_sm(bool periodic, bool accurate);
-size_t walk_stack_words(int grid, int stack_cap);
+size_t walk_stack_words(int grid);  // the walk's stacks, in 32-bit words
 void launch_walk(const WalkArgs& a, int grid, cudaStream_t s);
 void launch_deferred(const WalkArgs& a, cudaStream_t s);
 
