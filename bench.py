@@ -161,7 +161,7 @@ def measured_peaks():
 # DRAM bytes (read + write) of one k_walk launch on these workloads, from
 # single-pass ncu captures of dram__bytes_read.sum + dram__bytes_write.sum made
 # outside the bench (ncu cannot run inside a timed bench); reported with that label.
-WALK_DRAM_BYTES = {"clustered256_L200": 963312384 + 368289792, "treepm128_L100": 144405760 + 69206272}
+WALK_DRAM_BYTES = {"clustered256_L200": 840081920 + 321728256, "treepm128_L100": 112343808 + 26762240}
 
 
 def profile_traffic(workload):

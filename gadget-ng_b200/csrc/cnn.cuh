@@ -1,8 +1,9 @@
 // Learned short-range network: three valid 3x3x3 convolutions (16 channels,
 // GELU) and a linear head 16 -> 3 read at the particles by trilinear (CIC)
 // interpolation.  The convolutions run on the tcgen05 tensor cores in BF16
-// with FP32 accumulation in tensor memory; the weight gradients, the head,
-// the loss and Adam run on the CUDA cores in FP32.
+// with FP32 accumulation in tensor memory, the weight gradients on mma.sync
+// (BF16 in, FP32 accumulate); the head, the loss and Adam run on the CUDA cores
+// in FP32.
 //
 // Tensors are channel-last BF16 volumes [B][Z][Y][X][16] (32 bytes a node);
 // input channels beyond the network's c_in are zero.  No counterpart exists in

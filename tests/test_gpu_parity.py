@@ -312,7 +312,7 @@ def test_nonfinite_rejected():
 
 def test_memory_cap_refuses_cleanly():
     t = treepm()
-    # the handle's fixed buffers (the walk's per-warp stacks: 66 MB at 7
+    # the handle's fixed buffers (the walk's per-warp stacks: 48 MB at 5
     # resident blocks of 4 warps on 148 SMs) fit under the cap; the particle
     # buffers of 128^3 particles do not
     s = t.TreePmSolver(16, 100.0, memory_cap_bytes=128 << 20)
