@@ -10,6 +10,7 @@
 // resident for one evaluation.
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <string>
 #include <thread>
@@ -208,22 +209,24 @@ struct Cosmo {
 
 }  // namespace
 
-// What the host reads back from the device during a force evaluation, in pinned
-// memory: the copies queue behind the kernels and one synchronisation serves
-// them all.
-struct Readback {
-  uint32_t err, pm_err;
-  uint32_t scalars[4];
-  uint32_t depth_counts[DEPTH_BINS];
-  uint32_t learned_groups;
-  unsigned long long learned_count;
+// What a force evaluation leaves on the device for the host, in one block: one
+// copy into ordinary memory of the handle brings all of it.  (With the words apart
+// and copied to a pinned block behind one wait, page-locking that block took
+// 1 to 2.5 ms of the 5 to 7 ms that a handle's creation takes.)
+struct Status {
   unsigned long long stats[8];
+  uint32_t work, ndeferred;  // the walk's, cleared with the statistics
+  unsigned long long learned_count;
   TreeParams params;
+  uint32_t err, pm_err, learned_groups;
+  uint32_t scalars[8];
+  uint32_t depth_tab[3 * DEPTH_BINS + 1];
 };
 
 struct tpm_handle {
   tpm_config cfg{};
-  Readback* back = nullptr;
+  Status* status = nullptr;  // on the device
+  Status back{};             // its last copy
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   double r_s = 0, r_cut = 0, rc2 = 0, thr = 0;
@@ -249,9 +252,6 @@ struct tpm_handle {
   int walk_grid = 0;
   ErfcPoly poly{};  // the walk's erfc polynomial, and how far it holds
   uint2* deferred = nullptr;
-  uint32_t* ndeferred = nullptr;
-  unsigned long long* stats_dev = nullptr;
-  uint32_t* work = nullptr;
   double* staging = nullptr;  // float64 host-exchange buffer (n x 3 + n)
   size_t staging_elems = 0;
   bool forces_valid = false;
@@ -358,16 +358,18 @@ int fail(tpm_handle* h, const Error& e) {
   return e.code ? e.code : TPM_ERR_CUDA;
 }
 
-// Wait for the stream (and for any other readback queued on it) and raise
-// what the device flagged.
-void check_dev_err(tpm_handle* h) {
-  h->back->pm_err = 0;
-  if (h->pm.err)
-    TPM_CUDA(cudaMemcpyAsync(&h->back->pm_err, h->pm.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
-  TPM_CUDA(cudaMemcpyAsync(&h->back->err, h->T.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
+void read_status(tpm_handle* h) {
+  TPM_CUDA(cudaMemcpyAsync(&h->back, h->status, sizeof(Status), cudaMemcpyDeviceToHost, h->stream));
   TPM_CUDA(cudaStreamSynchronize(h->stream));
-  if (h->back->pm_err) pm_check(h->pm, h->stream);
-  const uint32_t e = h->back->err;
+}
+
+// Wait for the stream and raise what the device flagged.
+void check_dev_err(tpm_handle* h) {
+  if (h->pm.err)
+    TPM_CUDA(cudaMemcpyAsync(&h->status->pm_err, h->pm.err, sizeof(uint32_t), cudaMemcpyDeviceToDevice, h->stream));
+  read_status(h);
+  if (h->back.pm_err) pm_check(h->pm, h->stream);
+  const uint32_t e = h->back.err;
   if (!e) return;
   TPM_CUDA(cudaMemsetAsync(h->T.err, 0, sizeof(uint32_t), h->stream));
   if (e & DEV_ERR_NONFINITE) throw Error(TPM_ERR_NONFINITE, "non-finite position or mass");
@@ -582,7 +584,7 @@ void fe_sort(tpm_handle* h) {
   h->fe.launches0 = g_kernel_launches;
   TPM_CUDA(cudaEventRecord(h->ev[0], s));
   // the statistics, the walk's work counter and its deferred count: one block
-  TPM_CUDA(cudaMemsetAsync(h->stats_dev, 0, 10 * sizeof(unsigned long long), s));
+  TPM_CUDA(cudaMemsetAsync(h->status, 0, offsetof(Status, learned_count), s));
   const bool need_tree = !h->pm_only;
   h->fe.use_net = need_tree && h->learned && h->net_attached;
   h->tree_valid = false;
@@ -620,30 +622,25 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
   if (need_tree) {
     // ---- tree
     h->n_int = 0;
+    TPM_CUDA(cudaMemsetAsync(T.scalars, 0, 4 * sizeof(uint32_t), s));
     if (tree) {
-      TPM_CUDA(cudaMemsetAsync(T.scalars, 0, 4 * sizeof(uint32_t), s));
       launch_levels(n, T, s);
       exclusive_scan_u32(T.oct_count, T.oct_base, n, &T.scalars[0], h->scan_scratch, s);
-      TPM_CUDA(cudaMemcpyAsync(h->back->scalars, T.scalars, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-      TPM_CUDA(cudaMemcpyAsync(h->back->depth_counts, T.depth_tab, sizeof(h->back->depth_counts),
-                               cudaMemcpyDeviceToHost, s));
-      TPM_CUDA(cudaMemcpyAsync(&h->back->err, T.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     }
-    TPM_CUDA(cudaMemcpyAsync(&h->back->params, T.params, sizeof(TreeParams), cudaMemcpyDeviceToHost, s));
-    TPM_CUDA(cudaStreamSynchronize(s));
-    h->params_host = h->back->params;
+    read_status(h);
+    h->params_host = h->back.params;
     // The low keys of a run of ties that was refused are in no order, and no
     // tree comes of them: none is built or walked, and the end of the evaluation
     // raises the error.
-    if (tree && (h->back->err & DEV_ERR_TIE_RUN)) tree = false;
+    if (tree && (h->back.err & DEV_ERR_TIE_RUN)) tree = false;
     if (tree) {
-      h->n_int = h->back->scalars[0];
+      h->n_int = h->back.scalars[0];
       ensure_tree_capacity(h, h->n_int);
       launch_octree_nodes(n, h->n_int, T, s);
       // the accurate walk's relative opening criterion reads |Q|_F and the
       // cell centres: the quadrupole pass runs only for it
       const bool rel = relative_mac(h);
-      launch_aggregate(h->P[h->cur], n, h->n_int, box, T, h->back->depth_counts, s, rel);
+      launch_aggregate(h->P[h->cur], n, h->n_int, box, T, h->back.depth_tab, s, rel);
       h->quad_valid = rel;
       if (rel) launch_cell_q(h->n_int, box, T, s);
       launch_walk_records(h->P[h->cur], h->n_int, T, s);
@@ -653,10 +650,7 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
       launch_groups(h->n_int, walk_group_size(n), pack_depth, T, h->scan_scratch, s);
       // the group count and the tree depth stay on the device until the end of
       // the evaluation (the learned path sizes a launch by the group count)
-      TPM_CUDA(cudaMemcpyAsync(h->back->scalars, T.scalars, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-      if (use_net) TPM_CUDA(cudaStreamSynchronize(s));
-    } else {
-      std::memset(h->back->scalars, 0, sizeof(h->back->scalars));
+      if (use_net) read_status(h);
     }
     h->tree_valid = tree || n < 2;
     TPM_CUDA(cudaEventRecord(h->ev[3], s));
@@ -674,9 +668,8 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
       if (h->net.near_cells > 0.f) {  // exact pairs below the mesh scale for the network's particles
         near_of(h, eps2, h->fallback, h->srx, h->sry, h->srz);
       }
-      learned_groups(T.grp_first, T.grp_size, h->back->scalars[1], h->fallback, h->lgrp_first, h->lgrp_size,
+      learned_groups(T.grp_first, T.grp_size, tree ? h->back.scalars[1] : 0, h->fallback, h->lgrp_first, h->lgrp_size,
                      h->lgrp_count, s);
-      TPM_CUDA(cudaMemcpyAsync(&h->back->learned_groups, h->lgrp_count, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
       TPM_CUDA(cudaEventRecord(h->ev[8], s));
     }
     // ---- short-range walk
@@ -696,7 +689,7 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
       a.gfirst = use_net ? h->lgrp_first : T.grp_first;
       a.gsize = use_net ? h->lgrp_size : T.grp_size;
       a.ngroups = use_net ? h->lgrp_count : &T.scalars[1];
-      a.work = h->work;
+      a.work = &h->status->work;
       a.scale = scale; a.box = box; a.rc2 = h->rc2; a.thr = h->thr; a.h0 = h0;
       a.periodic = h->periodic ? 1 : 0;
       a.u_inv = (float)std::ldexp(1.0, -U);
@@ -766,8 +759,8 @@ void fe_tree_walk(tpm_handle* h, double eps2, const uint8_t* only) {
         a.tiny_u = -1.f;
       }
       a.ax = h->srx; a.ay = h->sry; a.az = h->srz;
-      a.stats = h->stats_dev; a.err = T.err;
-      a.deferred = h->deferred; a.ndeferred = h->ndeferred; a.cap_deferred = DEFERRED_CAP;
+      a.stats = h->status->stats; a.err = T.err;
+      a.deferred = h->deferred; a.ndeferred = &h->status->ndeferred; a.cap_deferred = DEFERRED_CAP;
       a.stack = h->stack;
       a.pcounts = h->pcounts;
       a.only = use_net ? h->fallback : only;
@@ -836,11 +829,8 @@ void fe_long_range(tpm_handle* h, double g, double kick, bool deposit, bool solv
   ga.kick = kick;
   pm_gather_kick(h->pm, ga, s);
   TPM_CUDA(cudaEventRecord(h->ev[6], s));
-  Readback& rb = *h->back;
-  TPM_CUDA(cudaMemcpyAsync(rb.stats, h->stats_dev, sizeof(rb.stats), cudaMemcpyDeviceToHost, s));
-  if (use_net)
-    TPM_CUDA(cudaMemcpyAsync(&rb.learned_count, h->learned_count, sizeof(rb.learned_count), cudaMemcpyDeviceToHost, s));
   check_dev_err(h);
+  const Status& rb = h->back;
   const unsigned long long* st = rb.stats;
   h->n_groups = h->pm_only ? 0 : rb.scalars[1];
   if (!h->pm_only && n >= 2) h->stats.max_tree_depth = (int32_t)rb.scalars[2];
@@ -1066,31 +1056,27 @@ int tpm_create(const tpm_config* cfg, tpm_handle** out) {
     TPM_CUDA(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     h->own_stream = true;
     for (auto& e : h->ev) TPM_CUDA(cudaEventCreate(&e));
-    h->T.params = h->alloc<TreeParams>(1, 0);
+    h->status = h->alloc<Status>(1, 0);
+    h->T.params = &h->status->params;
     h->T.bbox = h->alloc<uint32_t>(6, 0);
-    h->T.scalars = h->alloc<uint32_t>(8, 0);
-    h->T.depth_tab = h->alloc<uint32_t>(3 * DEPTH_BINS + 1, 0);
-    h->T.err = h->alloc<uint32_t>(1, 0);
-    h->stats_dev = h->alloc<unsigned long long>(10, 0);
-    h->work = reinterpret_cast<uint32_t*>(h->stats_dev + 8);
-    h->ndeferred = reinterpret_cast<uint32_t*>(h->stats_dev + 9);
-    TPM_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&h->back), sizeof(Readback), cudaHostAllocDefault));
-    std::memset(h->back, 0, sizeof(Readback));
+    h->T.scalars = h->status->scalars;
+    h->T.depth_tab = h->status->depth_tab;
+    h->T.err = &h->status->err;
+    h->learned_count = &h->status->learned_count;
+    h->lgrp_count = &h->status->learned_groups;
     h->dom_counts = h->alloc<unsigned long long>(MAX_RANKS + 8, 0);
-    h->lgrp_count = h->alloc<uint32_t>(1, 0);
     if (h->learned) {
       const int64_t nm3 = (int64_t)nm * nm * nm;
       h->cell_start = h->alloc<uint32_t>(nm3 + 1, 0);
       h->cell_cursor = h->alloc<uint32_t>(nm3 + 1, 0);
       h->cell_scan = h->alloc<char>(scan_scratch_bytes(nm3 + 1), 0);
     }
-    h->learned_count = h->alloc<unsigned long long>(1, 0);
     h->deferred = h->alloc<uint2>(DEFERRED_CAP, 0);
     int sms = prop.multiProcessorCount;
     h->poly = erfc_poly(h->r_cut / (std::sqrt(2.0) * h->r_s), 2.0 * pair_reach(h) / (std::sqrt(2.0) * h->r_s));
     h->walk_grid = sms * walk_blocks_per_sm(h->periodic, (cfg->flags & TPM_FLAG_ACCURATE) != 0);
     h->stack = h->alloc<uint32_t>(walk_stack_words(h->walk_grid), 0);
-    TPM_CUDA(cudaMemset(h->T.err, 0, sizeof(uint32_t)));
+    TPM_CUDA(cudaMemset(h->status, 0, sizeof(Status)));
     pm_plan_init(h->pm, nm, cfg->box_size, h->pm_only ? 0.0 : h->r_s, cfg->flags, cfg->device);
     h->mem_used += (size_t)nm * nm * nm * 4 * 4 + (size_t)nm * nm * (nm / 2 + 1) * 8 * 4;  // PM meshes
   } catch (const Error& e) {
@@ -1108,7 +1094,6 @@ void tpm_destroy(tpm_handle* h) {
   cudaSetDevice(h->cfg.device);
   if (h->stream) cudaStreamSynchronize(h->stream);
   for (const auto& a : h->allocs) cudaFree(a.p);
-  if (h->back) cudaFreeHost(h->back);
   pm_slab_free(h->slab);
   pm_plan_free(h->pm);
   for (auto& e : h->ev)
@@ -2231,7 +2216,7 @@ int64_t tpm_export_tree(tpm_handle* h, int64_t cap, int32_t* depth, double* mass
       throw Error(TPM_ERR_INVALID_ARGUMENT, "null export array");
     cudaStream_t s = h->stream;
     if (!h->quad_valid && ni > 0) {  // the force evaluation made mass and centre of mass only
-      launch_aggregate(h->P[h->cur], n, ni, h->cfg.box_size, h->T, h->back->depth_counts, s, true, false);
+      launch_aggregate(h->P[h->cur], n, ni, h->cfg.box_size, h->T, h->back.depth_tab, s, true, false);
       h->quad_valid = true;
     }
     int32_t* dd;
