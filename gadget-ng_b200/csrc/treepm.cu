@@ -979,6 +979,7 @@ void take_upload(tpm_handle* h, bool vel, int64_t n) {
   h->cur = 0;
   ++h->version;
   h->forces_valid = false;
+  h->tree_valid = false;
   h->m_total_valid = false;
   if (n == 0) return;
   cudaStream_t s = h->stream;
@@ -1508,6 +1509,7 @@ int tpm_set_particles_fixed(tpm_handle* h, const uint32_t* q, const float* vel, 
     h->cur = 0;
     ++h->version;
     h->forces_valid = false;
+    h->tree_valid = false;
     h->m_total_valid = false;
     cudaStream_t s = h->stream;
     std::vector<uint32_t> tmp((size_t)n);
@@ -1746,6 +1748,7 @@ int tpm_kdk_step_host(tpm_handle* h, double* pos, double* vel, const double* mas
     h->n_owned = n;
     h->cur = 0;
     h->forces_valid = false;
+    h->tree_valid = false;
     h->m_total_valid = false;
     ++h->version;
     k_encode<<<grid_for(n, 256, 1ll << 30), 256, 0, s>>>(din, din + 3 * n, din + 6 * n, n, h->cfg.box_size, h->P[0],
@@ -1775,6 +1778,7 @@ int tpm_set_particles_zeldovich(tpm_handle* h, const tpm_zeldovich* cfg) {
     h->cur = 0;
     ++h->version;
     h->forces_valid = false;
+    h->tree_valid = false;
     h->m_total_valid = false;
     zeldovich_fill(cfg, h->cfg.box_size, h->P[0], h->stream, &h->pm);
   } catch (const Error& e) {

@@ -71,3 +71,17 @@ def test_a_refused_run_of_ties_makes_no_tree(accurate):
     s.compute_forces(1e-3, 1.0)
     assert len(s.export_tree()["mass"]) > len(pos) and np.isfinite(s.get_state(len(pos))[2]).all()
     s.close()
+
+
+def test_new_particles_have_no_tree():
+    """The tree of an evaluation goes with its particles: its arrays are sized for them."""
+    import treepm
+    s = treepm.TreePmSolver(16, 64.0, 5.0)
+    for seed, n in ((1, 500), (2, 300), (3, 5000)):  # fewer, then more than the capacity
+        pos = _box(n, seed)
+        s.set_particles(pos, np.full(len(pos), 1.0 / len(pos)))
+        with pytest.raises(treepm.TreePmError):
+            s.export_tree()
+        s.compute_forces(1e-3, 1.0)
+        assert np.sort(s.export_tree()["particle"])[-len(pos):].tolist() == list(range(len(pos)))
+    s.close()
