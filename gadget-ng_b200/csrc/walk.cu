@@ -25,15 +25,16 @@
 // in shared memory.  Any decision that falls inside a narrow band around r_cut
 // is re-evaluated in float64 with the reference's exact expression, so the
 // interaction set equals the reference's.  Pair arithmetic is FP32: exact
-// fixed-point differences rounded once, rsqrt / ex2 hardware approximations,
-// a polynomial for the A&S 7.1.26 erfc, Kahan-compensated per-target sums.
+// fixed-point differences rounded once, rsqrt / ex2 hardware approximations, the
+// A&S 7.1.26 erfc as a polynomial where that holds out to the farthest pair,
+// Kahan-compensated per-target sums.
 //
 // What bounds it (lattice of 128^3, 84 k groups, B200 at 1965 MHz): issue slots.
 // 11.28e9 warp instructions took 11.3 ms at 88 % issue before the pair loop
 // took two entries per iteration in f32x2 arithmetic (63 instructions for
 // two entries, ~106 before) and the traversal was split into open and item
-// steps; 5.93e9 take 7.1 ms at 73 % after (62.7 -> 40.3 ms on the clustered
-// 256^3 box, 39.3 with 128-entry lists).  Two thirds are the pair loop (60 per iteration), its FMA pipe
+// steps; 5.74e9 take 6.93 ms at 73 % now (62.7 -> 39.3 ms on the clustered
+// 256^3 box).  Two thirds are the pair loop (60 per iteration), its FMA pipe
 // 56 % busy.  The accurate mode took the same steps later: 10.3 -> 7.4 ms on the
 // clustered 128^3 box against its former traversal (32 children of a popped
 // batch per step, opening tests at pop time).
